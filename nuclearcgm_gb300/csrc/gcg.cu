@@ -144,10 +144,7 @@ double msSince(std::chrono::steady_clock::time_point t0) {
 
 } // namespace
 
-// Orthonormalise the k columns of V (N x k, ld N) into Q with MGS-equivalent
-// dropping (pivot <= 1e-24). Returns kept column count; Q gets them compacted.
-// reads and clears the error word of the exact-digit tensor-core kernels
-static int takeExactErr() {
+int takeExactErr() {
   int flag = 0, zero = 0;
   if (cudaMemcpy(&flag, exactGramErrWord(), sizeof(int),
                  cudaMemcpyDeviceToHost) != cudaSuccess)
@@ -157,12 +154,12 @@ static int takeExactErr() {
   return flag;
 }
 
+// Orthonormalise the k columns of V (N x k, ld N) into Q with MGS-equivalent
+// dropping (pivot <= 1e-24). Returns kept column count; Q gets them compacted.
 static int cholQR2(ncgm_ctx *ctx, const double2 *V, int k, double2 *Q,
-                   double2 *Q1, double2 *small, double2 *partials,
-                   int maxChunks, int *dKeep, int *dIdx, cudaStream_t s,
-                   std::vector<int> *keptOrig = nullptr,
-                   float *tcPart = nullptr, void *vcPart = nullptr,
-                   bool fast = false) {
+                   double2 *Q1, double2 *small, const BlockProducts &prod,
+                   int *dKeep, int *dIdx, cudaStream_t s,
+                   std::vector<int> *keptOrig = nullptr, bool fast = false) {
   const size_t N = ctx->N;
   double2 *G = small, *R = small + (size_t)k * k, *T = small + 2 * (size_t)k * k,
           *Tk = small + 3 * (size_t)k * k;
@@ -173,14 +170,7 @@ static int cholQR2(ncgm_ctx *ctx, const double2 *V, int k, double2 *Q,
   std::vector<int> orig(k);
   std::iota(orig.begin(), orig.end(), 0);
   for (int pass = 0; pass < 2; ++pass) {
-    // tensor-core form: both passes' Grams on the tensor cores with exact
-    // digit products (~1e-12 relative; the basis is orthonormal to that
-    // level); otherwise FP64
-    if (tcPart)
-      gramTCExact(src, N, cols, src, N, cols, N, G, cols,
-                  reinterpret_cast<double *>(tcPart), s);
-    else
-      gram(src, N, cols, src, N, cols, N, G, cols, partials, maxChunks, s);
+    prod.gram(src, N, cols, src, N, cols, N, G, cols, s);
     cholDrop(G, cols, cols, 1e-24, R, T, dKeep, s, fast);
     cudaError_t e = cudaMemcpyAsync(keep.data(), dKeep, sizeof(int) * cols,
                                     cudaMemcpyDeviceToHost, s);
@@ -204,10 +194,7 @@ static int cholQR2(ncgm_ctx *ctx, const double2 *V, int k, double2 *Q,
     gatherSmall<<<(cols * kept + 255) / 256, 256, 0, s>>>(T, cols, cols, dIdx,
                                                           kept, Tk, cols);
     double2 *out = (pass == 0) ? dst : Q;
-    if (vcPart)
-      gemmVCExact(src, N, cols, Tk, cols, kept, out, N, N, vcPart, s);
-    else
-      gemmVC(src, N, cols, Tk, cols, kept, out, N, N, 0.0, s);
+    prod.vc(src, N, cols, Tk, cols, kept, out, N, N, s);
     src = out;
     cols = kept;
   }
@@ -238,8 +225,9 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   const bool fp32 =
       prm.precision == NCGM_FP32 || prm.precision == NCGM_FP32_TC;
   const bool learned = prm.precond == NCGM_PRECOND_LEARNED;
-  // tensor-core Gram products of the search space (FP32-level accuracy)
-  const bool tc = prm.precision == NCGM_FP32_TC;
+  // products of the search space: 6 digits in the tensor-core form (~1e-12
+  // relative), FP64 accuracy otherwise
+  const int digits = prm.precision == NCGM_FP32_TC ? 6 : 8;
   if (learned && !ctx->lp) {
     setError("ncgm_gcg: learned preconditioner requested but no network set "
              "(ncgm_set_lp)");
@@ -257,13 +245,19 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   need += ctx->ns * sizeof(float) + 256; // FP32 inverse Jacobi diagonal
   char *base = static_cast<char *>(ctx->buf(10, need + 64 * 4096));
   if (!base) return NCGM_ERR_NOMEM;
-  float *tcPart = nullptr;
-  void *vcPart = nullptr;
-  if (tc) {
-    tcPart = static_cast<float *>(ctx->buf(
-        11, sizeof(double) * exactGramScratchDoubles(N, vmax, vmax) + 256));
-    vcPart = ctx->buf(31, exactVCScratchBytes(N, vmax, vmax));
-    if (!tcPart || !vcPart) return NCGM_ERR_NOMEM;
+  BlockProducts prod;
+  prod.digits = digits;
+  if (digits == 6 || digitsPayGram(N, vmax, vmax)) {
+    prod.gramScr = static_cast<double *>(ctx->buf(
+        11, sizeof(double) * exactGramScratchDoubles(N, vmax, vmax, digits) +
+                256));
+    prod.vcScr = ctx->buf(31, exactVCScratchBytes(N, vmax, vmax, digits));
+    if (!prod.gramScr || !prod.vcScr) {
+      if (digits == 6) return NCGM_ERR_NOMEM;
+      // no room for the digit images: the plain FP64 kernels
+      prod.gramScr = nullptr;
+      prod.vcScr = nullptr;
+    }
   }
   // the projected eigensolver's workspace (Householder methods)
   const size_t heigScrB = heigScratchBytes(mx);
@@ -294,6 +288,8 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   int *dLive = ar.take<int>(1), *dNdone = ar.take<int>(1);
   unsigned *dArrive = ar.take<unsigned>(2 * (size_t)nev);
   float *dInv32 = ar.take<float>(ctx->ns);
+  prod.partials = partials;
+  prod.maxChunks = (int)maxChunks;
   double2 *Gs = small, *Cw = small + 4 * (size_t)mx * mx,
           *Ev = small + 5 * (size_t)mx * mx, *Ap = small + 6 * (size_t)mx * mx;
 
@@ -312,8 +308,8 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   NCGM_CUDA(cudaMemcpyAsync(V, Xinit, N * (size_t)nev * sizeof(double2),
                             cudaMemcpyDeviceToDevice, s));
   std::vector<int> keptInit;
-  int nkept = cholQR2(ctx, V, nev, Q, Q1, Gs, partials, (int)maxChunks, dKeep,
-                      dIdx, s, &keptInit, tcPart, vcPart, fp32);
+  int nkept = cholQR2(ctx, V, nev, Q, Q1, Gs, prod, dKeep, dIdx, s, &keptInit,
+                      fp32);
   if (nkept < 0) return NCGM_ERR_CUDA;
   if (nkept == 0) {
     setError("ncgm_gcg: initial block has no independent columns");
@@ -334,23 +330,13 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   // initial Rayleigh-Ritz (rayleighRitz_complex_no_B, solver.cpp:418-463)
   {
     applyA(Xa, AV, nx, shift);
-    if (tc)
-      gramTCExact(Xa, N, nx, AV, N, nx, N, Ap, nx,
-                  reinterpret_cast<double *>(tcPart), s);
-    else
-      gram(Xa, N, nx, AV, N, nx, N, Ap, nx, partials, (int)maxChunks, s);
+    prod.gram(Xa, N, nx, AV, N, nx, N, Ap, nx, s);
     heig(Ap, nx, nx, Cw, Ev, dW, dPerm, dStat, s, fp32, heigScr, heigScrB);
-    if (tc)
-      gemmVCExact(Xa, N, nx, Ev, nx, nx, Xn, N, N, vcPart, s);
-    else
-      gemmVC(Xa, N, nx, Ev, nx, nx, Xn, N, N, 0.0, s);
+    prod.vc(Xa, N, nx, Ev, nx, nx, Xn, N, N, s);
     NCGM_CUDA(cudaMemcpyAsync(Xa, Xn, N * (size_t)nx * sizeof(double2),
                               cudaMemcpyDeviceToDevice, s));
     // A X of the rotated block (shift removed), kept for the FP32 correction
-    if (tc)
-      gemmVCExact(AV, N, nx, Ev, nx, nx, AXa, N, N, vcPart, s);
-    else
-      gemmVC(AV, N, nx, Ev, nx, nx, AXa, N, N, 0.0, s);
+    prod.vc(AV, N, nx, Ev, nx, nx, AXa, N, N, s);
     if (shift != 0.0)
       axpyCols<<<gridN(nx), 256, 0, s>>>(AXa, Xa, N, nx, -shift);
     NCGM_CUDA(cudaMemcpyAsync(hw.data(), dW, sizeof(double) * nx,
@@ -525,8 +511,8 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
       msPcg += msSince(tp);
     }
     const int vcols = nconv + nact + pc + nact;
-    int m = cholQR2(ctx, V, vcols, Q, Q1, Gs, partials, (int)maxChunks, dKeep,
-                    dIdx, s, nullptr, tcPart, vcPart, fp32);
+    int m = cholQR2(ctx, V, vcols, Q, Q1, Gs, prod, dKeep, dIdx, s, nullptr,
+                    fp32);
     if (m < 0) return NCGM_ERR_CUDA;
     if (m == 0) {
       setError("ncgm_gcg: search space collapsed");
@@ -535,20 +521,11 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
     lastBasis = m;
     // Rayleigh-Ritz on A_shifted
     applyA(Q, AV, m, shift);
-    if (tc)
-      gramTCExact(Q, N, m, AV, N, m, N, Ap, m,
-                  reinterpret_cast<double *>(tcPart), s);
-    else
-      gram(Q, N, m, AV, N, m, N, Ap, m, partials, (int)maxChunks, s);
+    prod.gram(Q, N, m, AV, N, m, N, Ap, m, s);
     heig(Ap, m, m, Cw, Ev, dW, dPerm, dStat, s, fp32, heigScr, heigScrB);
     const int rr = std::min(nev, m);
-    if (tc) {
-      gemmVCExact(Q, N, m, Ev, m, rr, Xn, N, N, vcPart, s);
-      gemmVCExact(AV, N, m, Ev, m, rr, AXn, N, N, vcPart, s);
-    } else {
-      gemmVC(Q, N, m, Ev, m, rr, Xn, N, N, 0.0, s);
-      gemmVC(AV, N, m, Ev, m, rr, AXn, N, N, 0.0, s);
-    }
+    prod.vc(Q, N, m, Ev, m, rr, Xn, N, N, s);
+    prod.vc(AV, N, m, Ev, m, rr, AXn, N, N, s);
     axpyCols<<<gridN(rr), 256, 0, s>>>(AXn, Xn, N, rr, -shift); // = A Xn
     NCGM_CUDA(cudaMemcpyAsync(hw.data(), dW, sizeof(double) * m,
                               cudaMemcpyDeviceToHost, s));
@@ -644,7 +621,7 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   for (int k = 0; k < nev; ++k) lamOut[k] = finalL[order[k]];
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
-  if (tc && takeExactErr()) {
+  if (prod.gramScr && takeExactErr()) {
     setError("ncgm_gcg: tensor-core kernel wait timed out");
     return NCGM_ERR_TIMEOUT;
   }
@@ -760,22 +737,29 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
                        : static_cast<double2 *>(
                              ctx->buf(28, (size_t)p * q * sizeof(double2)));
   if (!dC) return NCGM_ERR_NOMEM;
+  bool digits = false;
   if (precision == NCGM_FP32) {
     float *part = static_cast<float *>(
         ctx->buf(29, sizeof(float) * tcGramPartialFloats(N, p, q) + 256));
     if (!part) return NCGM_ERR_NOMEM;
     gramTC(dA, N, p, dB, N, q, N, dC, p, part, s);
-  } else if (precision == NCGM_FP32_TC) {
-    double *part = static_cast<double *>(
-        ctx->buf(29, sizeof(double) * exactGramScratchDoubles(N, p, q) + 256));
-    if (!part) return NCGM_ERR_NOMEM;
-    gramTCExact(dA, N, p, dB, N, q, N, dC, p, part, s);
   } else {
-    const int chunks = gramMaxChunks();
-    auto *part = static_cast<double2 *>(
-        ctx->buf(29, sizeof(double2) * (size_t)chunks * p * q));
-    if (!part) return NCGM_ERR_NOMEM;
-    gram(dA, N, p, dB, N, q, N, dC, p, part, chunks, s);
+    BlockProducts prod;
+    prod.digits = precision == NCGM_FP32_TC ? 6 : 8;
+    if (prod.digits == 6 || digitsPayGram(N, p, q))
+      prod.gramScr = static_cast<double *>(ctx->buf(
+          29, sizeof(double) * exactGramScratchDoubles(N, p, q, prod.digits) +
+                  256));
+    if (!prod.gramScr) {
+      // FP64 on small blocks, or no room for the digit images
+      if (prod.digits == 6) return NCGM_ERR_NOMEM;
+      prod.maxChunks = gramMaxChunks();
+      prod.partials = static_cast<double2 *>(
+          ctx->buf(29, sizeof(double2) * (size_t)prod.maxChunks * p * q));
+      if (!prod.partials) return NCGM_ERR_NOMEM;
+    }
+    digits = prod.gramScr != nullptr;
+    prod.gram(dA, N, p, dB, N, q, N, dC, p, s);
   }
   if (!devOut)
     NCGM_CUDA(cudaMemcpyAsync(C, dC, (size_t)p * q * sizeof(double2),
@@ -783,15 +767,13 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
   int flag = 0;
-  if (precision == NCGM_FP32_TC) flag = takeExactErr();
+  if (digits) flag = takeExactErr();
   if (precision == NCGM_FP32)
     NCGM_CUDA(cudaMemcpy(&flag, tcGramErrWord(), sizeof(int),
                          cudaMemcpyDeviceToHost));
-  if (precision != NCGM_FP64) {
-    if (flag) {
-      setError("ncgm_gram: tensor-core kernel wait timed out");
-      return NCGM_ERR_TIMEOUT;
-    }
+  if (flag) {
+    setError("ncgm_gram: tensor-core kernel wait timed out");
+    return NCGM_ERR_TIMEOUT;
   }
   return NCGM_OK;
 }
@@ -822,19 +804,19 @@ extern "C" int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C,
                        : static_cast<double2 *>(
                              ctx->buf(28, N * (size_t)k * sizeof(double2)));
   if (!dY) return NCGM_ERR_NOMEM;
-  if (precision == NCGM_FP32_TC) {
-    void *part = ctx->buf(29, exactVCScratchBytes(N, m, k));
-    if (!part) return NCGM_ERR_NOMEM;
-    gemmVCExact(dV, N, m, dC, m, k, dY, N, N, part, s);
-  } else {
-    gemmVC(dV, N, m, dC, m, k, dY, N, N, 0.0, s);
+  BlockProducts prod;
+  prod.digits = precision == NCGM_FP32_TC ? 6 : 8;
+  if (prod.digits == 6 || digitsPayVC(N, m, k)) {
+    prod.vcScr = ctx->buf(29, exactVCScratchBytes(N, m, k, prod.digits));
+    if (!prod.vcScr && prod.digits == 6) return NCGM_ERR_NOMEM;
   }
+  prod.vc(dV, N, m, dC, m, k, dY, N, N, s);
   if (!devOut)
     NCGM_CUDA(cudaMemcpyAsync(Y, dY, N * (size_t)k * sizeof(double2),
                               cudaMemcpyDeviceToHost, s));
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
-  if (precision == NCGM_FP32_TC && takeExactErr()) {
+  if (prod.vcScr && takeExactErr()) {
     setError("ncgm_vc: tensor-core kernel wait timed out");
     return NCGM_ERR_TIMEOUT;
   }

@@ -261,18 +261,32 @@ struct Run {
   double tPair = 0, tFields = 0, tPoisson = 0, tGcg = 0;
   double constraintEnergy = 0; // of the last energy evaluation
   std::vector<void *> allocs;
-  // tensor-core form: scratch of the exact-digit Gram / V C products of the
-  // driver's own overlaps and rotations (allocated on first use)
-  void *tcScr = nullptr;
-  bool tc() const { return cfg.hf_gcg.precision == NCGM_FP32_TC; }
-  void *tcScratch() {
-    if (!tcScr) {
-      int M = std::max(sp[0].orb, sp[1].orb);
-      size_t b = std::max(exactGramScratchDoubles(N, M, M) * sizeof(double),
-                          exactVCScratchBytes(N, M, M));
-      tcScr = alloc<char>(b + 1024);
+  // scratch of the digit Gram / V C products of the driver's own overlaps and
+  // rotations (allocated on first use; without room the plain FP64 kernels)
+  void *digitScr = nullptr;
+  bool digitTried = false;
+  int digits() const {
+    return cfg.hf_gcg.precision == NCGM_FP32_TC ? 6 : 8;
+  }
+  size_t digitBytes(size_t gramRows) const {
+    const int M = std::max(sp[0].orb, sp[1].orb);
+    return std::max(exactGramScratchDoubles(gramRows, M, M, digits()) *
+                        sizeof(double),
+                    exactVCScratchBytes(N, M, M, digits())) +
+           1024;
+  }
+  BlockProducts products() {
+    const int M = std::max(sp[0].orb, sp[1].orb);
+    if (!digitTried && (digits() == 6 || digitsPayGram(N, M, M))) {
+      digitScr = alloc<char>(digitBytes(N));
+      if (!digitScr) cudaGetLastError();
     }
-    return tcScr;
+    digitTried = true;
+    BlockProducts p;
+    p.digits = digits();
+    p.gramScr = static_cast<double *>(digitScr);
+    p.vcScr = digitScr;
+    return p;
   }
 
   // HFB workspace and both species' amplitude matrices (first use)
@@ -284,13 +298,13 @@ struct Run {
     HfbWork w;
     w.M = M;
     w.gemmParts = alloc<double2>(HfbWork::kChunks * MM);
-    if (tc()) {
+    if (digits() == 6 || digitsPayGram(ns, M, M)) {
       // both bounds hold for every window size nS <= M
-      const size_t b =
-          std::max(exactGramScratchDoubles(ns, M, M) * sizeof(double),
-                   exactVCScratchBytes(N, M, M));
-      w.gemmExact = alloc<char>(b + 1024);
-      if (!w.gemmExact) return nullptr;
+      w.gemmExact = alloc<char>(digitBytes(ns));
+      if (!w.gemmExact) {
+        if (digits() == 6) return nullptr;
+        cudaGetLastError();
+      }
     }
     double *d = alloc<double>(4 * (size_t)M + 4 * MM + 2 * (size_t)M + 16);
     double2 *c = alloc<double2>(2 * MM + 3 * 4 * MM + 3 * MM);
@@ -331,7 +345,9 @@ struct Run {
   }
   PairingGemm pairingGemm() const {
     PairingGemm g;
-    if (tc()) g.exactScratch = hw.gemmExact;
+    g.digits = digits();
+    g.gramScr = static_cast<double *>(hw.gemmExact);
+    g.vcScr = hw.gemmExact;
     g.partials = hw.gemmParts;
     g.maxChunks = HfbWork::kChunks;
     return g;
@@ -402,11 +418,10 @@ int hostGram(Run &R, const double2 *A, int p, const double2 *B, int q,
     }
     cap = need;
   }
-  if (R.tc() && R.tcScratch())
-    gramTCExact(A, R.N, p, B, R.N, q, R.N, R.cplx, p,
-                static_cast<double *>(R.tcScratch()), R.s);
-  else
-    gram(A, R.N, p, B, R.N, q, R.N, R.cplx, p, parts, maxChunks, R.s);
+  BlockProducts prod = R.products();
+  prod.partials = parts;
+  prod.maxChunks = maxChunks;
+  prod.gram(A, R.N, p, B, R.N, q, R.N, R.cplx, p, R.s);
   C.resize((size_t)p * q);
   cudaMemcpyAsync(C.data(), R.cplx, sizeof(double2) * p * q,
                   cudaMemcpyDeviceToHost, R.s);
@@ -697,10 +712,7 @@ int hfbSpecies(Run &R, Species &S, int target, HFBRes &out) {
 // Phi = phi * T (occupation transform), T on the device (M x M, col-major)
 int occupyDev(Run &R, Species &S, const double2 *T) {
   const int M = S.orb;
-  if (R.tc() && R.tcScratch())
-    gemmVCExact(S.X, R.N, M, T, M, M, S.Phi, R.N, R.N, R.tcScratch(), R.s);
-  else
-    gemmVC(S.X, R.N, M, T, M, M, S.Phi, R.N, R.N, 0.0, R.s);
+  R.products().vc(S.X, R.N, M, T, M, M, S.Phi, R.N, R.N, R.s);
   return NCGM_OK;
 }
 
@@ -1161,11 +1173,7 @@ int conjDir(Run &R, Species &S) {
                   cudaMemcpyHostToDevice, R.s);
   cudaMemcpyAsync(S.CD, S.Xn, sizeof(double2) * R.N * M,
                   cudaMemcpyDeviceToDevice, R.s);
-  if (R.tc() && R.tcScratch())
-    gemmVCExact(S.X, R.N, M, R.cplx, M, M, S.CD, R.N, R.N, R.tcScratch(),
-                R.s, true);
-  else
-    gemmVC(S.X, R.N, M, R.cplx, M, M, S.CD, R.N, R.N, 1.0, R.s);
+  R.products().vc(S.X, R.N, M, R.cplx, M, M, S.CD, R.N, R.N, R.s, true);
   normalizeEuclid(S.CD, R.N, R.N, M, R.small, R.s);
   S.cdCols = M;
   return sync(R);
@@ -1862,7 +1870,12 @@ extern "C" int ncgm_state_update(ncgm_state *st, const double *Xn,
       st->multipolesAdded = true;
     }
     NCGM_TRY(updateQuantities(R, iter));
-    return sync(R);
+    NCGM_TRY(sync(R));
+    if ((R.digitScr || R.hw.gemmExact) && takeExactErr()) {
+      setError("ncgm_state_update: tensor-core kernel wait timed out");
+      return NCGM_ERR_TIMEOUT;
+    }
+    return NCGM_OK;
   } catch (const std::exception &e) {
     setError(e.what());
     return NCGM_ERR_ARG;

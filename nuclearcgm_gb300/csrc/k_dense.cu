@@ -594,6 +594,40 @@ void gemmVC(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
   }
 }
 
+// Measured per call (self-Gram / Y = V C, m = k columns, plain -> digits):
+// n = 36: m = 60 4250 -> 275 us / 3660 -> 454 us; m = 8 370 -> 181 / 81 ->
+// 122. n = 16: m = 24 132 -> 75 / 94 -> 81. The plain Gram never falls below
+// ~130 us (its chunk reduction is a serial chain), so the digits win on every
+// lattice a run uses; on smaller ones (N = 2 n^3 < 6000) both are launches
+// and latency, and the plain kernels keep the small-lattice fixed points on
+// the rounding path they are compared on. The plain V C is FP64-pipe bound
+// from a few million products on (13 us per million) and otherwise one short
+// launch against six.
+bool digitsPayGram(size_t N, int p, int q) {
+  return N >= 6000 && p > 0 && q > 0;
+}
+bool digitsPayVC(size_t N, int m, int k) {
+  return N >= 6000 && (double)N * m * k >= 9e6;
+}
+
+void BlockProducts::gram(const double2 *A, size_t lda, int p, const double2 *B,
+                         size_t ldb, int q, size_t N, double2 *C, int ldc,
+                         cudaStream_t s) const {
+  if (gramScr && (digits == 6 || digitsPayGram(N, p, q)))
+    gramTCExact(A, lda, p, B, ldb, q, N, C, ldc, gramScr, s, digits);
+  else
+    ncgm::gram(A, lda, p, B, ldb, q, N, C, ldc, partials, maxChunks, s);
+}
+
+void BlockProducts::vc(const double2 *V, size_t ldv, int m, const double2 *Cm,
+                       int ldc, int k, double2 *Y, size_t ldy, size_t N,
+                       cudaStream_t s, bool accum) const {
+  if (vcScr && (digits == 6 || digitsPayVC(N, m, k)))
+    gemmVCExact(V, ldv, m, Cm, ldc, k, Y, ldy, N, vcScr, s, accum, digits);
+  else
+    gemmVC(V, ldv, m, Cm, ldc, k, Y, ldy, N, accum ? 1.0 : 0.0, s);
+}
+
 // Same factorisation in shared memory, right-looking: at step j the pivot is
 // the updated diagonal A_jj = G_jj - sum_{k<j} |R_kj|^2, row j of R is
 // A_j. / R_jj, and the trailing upper triangle takes the rank-1 update

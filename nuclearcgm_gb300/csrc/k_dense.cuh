@@ -19,27 +19,55 @@ void gramTC(const double2 *A, size_t lda, int p, const double2 *B, size_t ldb,
             cudaStream_t s);
 size_t tcGramPartialFloats(size_t N, int p, int q);
 int *tcGramErrWord();
-// C = A^H B on the tensor cores to ~1e-13 relative: error-free splitting into
-// BF16 integer digits (digitised once per operand), exact FP32 level sums,
-// exact 64-bit combination (k_tcgram_exact.cu). scratch:
-// exactGramScratchDoubles(N, p, q) doubles, 16-byte aligned.
+// C = A^H B on the tensor cores: error-free splitting into 6 (~1e-13 relative)
+// or 8 (FP64 accuracy) BF16 integer digits (digitised once per operand),
+// exact FP32 level sums, exact integer combination (k_tcgram_exact.cu).
+// scratch: exactGramScratchDoubles(N, p, q, digits) doubles, 16-byte aligned.
+// 8 digits: operands with infinities, NaNs or extreme magnitudes take a plain
+// FP64 sum on the device.
 void gramTCExact(const double2 *A, size_t lda, int p, const double2 *B,
                  size_t ldb, int q, size_t N, double2 *C, int ldc,
-                 double *scratch, cudaStream_t s);
-size_t exactGramScratchDoubles(size_t N, int p, int q);
+                 double *scratch, cudaStream_t s, int digits = 6);
+size_t exactGramScratchDoubles(size_t N, int p, int q, int digits = 6);
 int *exactGramErrWord();
+// reads and clears the error word of the exact-digit kernels (non-zero: a
+// bounded wait of one of them gave up)
+int takeExactErr();
 // Y = V C on the tensor cores with the exact digit products of gramTCExact
-// (~1e-12 relative of the column maxima; k_tcgram_exact.cu). scratch:
-// exactVCScratchBytes(N, m, k) bytes, 16-byte aligned.
+// (6 digits: ~1e-12 relative of the column maxima; 8: FP64 accuracy;
+// k_tcgram_exact.cu). scratch: exactVCScratchBytes(N, m, k, digits) bytes,
+// 16-byte aligned.
 void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *C,
                  int ldc, int k, double2 *Y, size_t ldy, size_t N,
-                 void *scratch, cudaStream_t s, bool accum = false);
-size_t exactVCScratchBytes(size_t N, int m, int k);
+                 void *scratch, cudaStream_t s, bool accum = false,
+                 int digits = 6);
+size_t exactVCScratchBytes(size_t N, int m, int k, int digits = 6);
 // Y = V C + beta Y (V: N x m with m <= 1600, C: m x k; C is staged in
 // shared memory in blocks of columns).
 void gemmVC(const double2 *V, size_t ldv, int m, const double2 *C, int ldc,
             int k, double2 *Y, size_t ldy, size_t N, double beta,
             cudaStream_t s);
+// Whether the 8-digit tensor-core products beat the plain FP64 kernels for
+// C (p x q) = A^H B and Y (N x k) = V (N x m) C.
+bool digitsPayGram(size_t N, int p, int q);
+bool digitsPayVC(size_t N, int m, int k);
+// The products of tall blocks in one of three forms: 6 digits (tensor-core
+// precision form), 8 digits (FP64 accuracy on the tensor cores, where
+// digitsPay) or the plain FP64 kernels (no scratch, or small blocks).
+struct BlockProducts {
+  int digits = 8;
+  double *gramScr = nullptr; // exactGramScratchDoubles
+  void *vcScr = nullptr;     // exactVCScratchBytes (may be the same memory)
+  double2 *partials = nullptr; // plain Gram: maxChunks p q
+  int maxChunks = 1;
+  // C = A^H B
+  void gram(const double2 *A, size_t lda, int p, const double2 *B, size_t ldb,
+            int q, size_t N, double2 *C, int ldc, cudaStream_t s) const;
+  // Y = V C (accum: Y += V C)
+  void vc(const double2 *V, size_t ldv, int m, const double2 *C, int ldc,
+          int k, double2 *Y, size_t ldy, size_t N, cudaStream_t s,
+          bool accum = false) const;
+};
 // Cholesky of Gram G with MGS-equivalent drop; T = R^{-1}; keep flags.
 // fast: the FP32 forms' variant (double-float pivot roots and reciprocals).
 void cholDrop(const double2 *G, int ldg, int m, double dropTol, double2 *R,

@@ -528,10 +528,7 @@ void kappaFieldGemm(const double2 *Phi, size_t ld, int nS, const double *Kff,
   if (nS <= 0) return;
   const size_t N = 2 * ns;
   kffTransposeKernel<<<(nS * nS + 255) / 256, 256, 0, s>>>(Kff, nS, C);
-  if (g.exactScratch)
-    gemmVCExact(Phi, ld, nS, C, nS, nS, Q, N, N, g.exactScratch, s);
-  else
-    gemmVC(Phi, ld, nS, C, nS, nS, Q, N, N, 0.0, s);
+  g.vc(Phi, ld, nS, C, nS, nS, Q, N, N, s);
   kappaReduceKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(
       Phi, ld, Q, N, nS, ns, kappa);
 }
@@ -545,11 +542,7 @@ void deltaMatrixGemm(const double2 *Phi, size_t ld, int nS, const double *ff,
   double2 *A0 = work, *B1 = work + ns * nS;
   dim3 grid((unsigned)((ns + 255) / 256), nS);
   deltaOperandsKernel<<<grid, 256, 0, s>>>(Phi, ld, nS, kappa, n, h, A0, B1);
-  if (g.exactScratch)
-    gramTCExact(A0, ns, nS, B1, ns, nS, ns, G, nS,
-                static_cast<double *>(g.exactScratch), s);
-  else
-    gram(A0, ns, nS, B1, ns, nS, ns, G, nS, g.partials, g.maxChunks, s);
+  g.gram(A0, ns, nS, B1, ns, nS, ns, G, nS, s);
   deltaFromGramKernel<<<(nS * nS + 255) / 256, 256, 0, s>>>(G, nS, ff, V0,
                                                            Delta);
 }

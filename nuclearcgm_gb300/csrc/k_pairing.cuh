@@ -1,5 +1,7 @@
 // Pairing and guess kernels (see k_pairing.cu).
 #pragma once
+#include "k_dense.cuh"
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -18,15 +20,9 @@ void bcsSolve(const double *eps, const double *Gp, int np, int A,
               double window, int windowBoth, const double *oldDelta,
               bool useOld, double oldLambda, double *u2, double *v2,
               double *Delta, double *scal, double *work, cudaStream_t s);
-// Dense-product back ends of the two HFB pairing-field routines: the
-// exact-digit tensor-core kernels when exactScratch is set (gemmVCExact and
-// gramTCExact scratch sized for nS columns), otherwise the FP64 kernels with
-// `partials` (>= maxChunks nS^2 double2) for the Gram.
-struct PairingGemm {
-  void *exactScratch = nullptr;
-  double2 *partials = nullptr;
-  int maxChunks = 1;
-};
+// The two HFB pairing-field routines take the run's block products, with
+// scratch (or `partials`) sized for nS columns.
+using PairingGemm = BlockProducts;
 // kappa(r) from Kff (K_ab f_a f_b, nS x nS col-major) over the nS columns of
 // Phi (ld): Q = Phi Kff^T (one N x nS by nS x nS product), then one pass over
 // the points. Q: N x nS scratch, C: nS x nS complex scratch.

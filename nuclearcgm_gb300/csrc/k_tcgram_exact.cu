@@ -13,10 +13,21 @@
 // 2^(-7l)) accumulate in FP32 tensor memory over 256 rows, so every partial
 // sum is an integer below 2^24 and the FP32 accumulation is exact. After each
 // 256-row block the levels are combined exactly in 64-bit integers (held in
-// registers over at most 16 blocks), converted to FP64 once per CTA, and the
-// CTA's FP64 partial is summed with the other row chunks in a fixed order.
+// registers over at most 16 blocks); the chunks' integers are added in 128
+// bits and rounded to FP64 once.
 // Levels above kDig + 1 are dropped: the truncation error is ~2^(-7 kDig) of
-// the column max per element (kDig = 6: ~2e-13 relative).
+// the column max per element. 6 digits (the tensor-core precision form) give
+// ~2e-13 relative; 8 digits hold all 53 bits of every entry above 2^-4 of its
+// column's maximum, and the product is then as accurate as an FP64 sum or
+// better: against 113-bit sums, 2 36^3 rows, 60 columns of orbitals and
+// corrections 1000 times smaller, the Gram is off by 2.4e-17 rms (1.3e-16 at
+// most) of |a||b| where the FP64 kernel is off by 1.5e-16 (9.8e-16), and V C
+// by 1.2e-16 of |y| where it is off by 3.0e-16.
+//
+// What bounds it: GB300's FP64 pipe retires two operations per clock per SM,
+// so the FP64 kernels take 4.25 ms (Gram) and 3.66 ms (V C) at 2 36^3 x 60,
+// m = k = 60; the 36 digit products run on the tensor cores in 0.28 and
+// 0.45 ms. The digit images (16 bytes per real value) go through L2.
 //
 // Two passes per product:
 //  1. A digitising kernel writes each operand's digits once, as the exact
@@ -39,10 +50,10 @@
 namespace ncgm {
 
 int smCount();
+int *exactGramErrWord();
 
 namespace {
 
-constexpr int kDig = 6;                  // digits per value
 constexpr int kM = 128, kN = 64;         // D tile
 constexpr int kSlab = 32;                // K rows per stage (2 MMAs of K 16)
 constexpr int kFold = 8;                 // slabs per exact accumulation block
@@ -50,12 +61,21 @@ constexpr int kMaxFolds = 16;            // fold blocks per 64-bit sum
 constexpr int kThr = 256;
 constexpr int kABytes = kM * kSlab * 2;  // one digit plane of A: 8 KB
 constexpr int kBBytes = kN * kSlab * 2;  // one digit plane of B: 4 KB
-constexpr int kTile = kDig * kABytes;    // a digitised 128 x 32 tile: 48 KB
-constexpr int kBuf = kDig * (kABytes + kBBytes); // one stage: 72 KB
-constexpr int kStages = 3;
-constexpr int kSmem = kStages * kBuf + 128; // + barriers, TMEM slot
 constexpr uint32_t kLBO = 128, kSBO = 512;       // 8 rows x 16 B cores; K 32
-constexpr uint32_t kTmemCols = 512; // kDig levels x kN = 384 -> 512
+constexpr uint32_t kTmemCols = 512; // kDig levels x kN = 384 or 512
+
+// sizes of a digit format of kDig digits per value: 6 (42 bits, the
+// tensor-core precision form) or 8 (56 bits, the FP64 form)
+template <int kDig> struct Fmt {
+  static_assert(kDig == 6 || kDig == 8, "digit formats");
+  static constexpr int kBits = 7 * kDig;
+  // a digitised 128 x 32 tile: 48 / 64 KB; one stage (A tile and the 64
+  // columns of B): 72 / 96 KB, so 3 / 2 stages fit the 227 KB of an SM
+  static constexpr int kTile = kDig * kABytes;
+  static constexpr int kBuf = kDig * (kABytes + kBBytes);
+  static constexpr int kStages = kDig == 6 ? 3 : 2;
+  static constexpr int kSmem = kStages * kBuf + 128; // + barriers, TMEM slot
+};
 
 __device__ __forceinline__ uint32_t sAddr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -106,58 +126,69 @@ __device__ __forceinline__ bool waitSpin(uint64_t *bar, uint32_t phase) {
   }
 }
 
-// digits of a scaled value: w = round(x 2^(42-e)), |w| < 2^42, written as
-// sum_t a_t 2^(42-7t) with |a_1| <= 128 and |a_t| <= 64, by integer rounding
-// divisions (exact; the digits are integers, exact in BF16). One 64-bit
-// rounding split w = h 2^21 + l (|l| <= 2^20) leaves 32-bit work: three
-// digits from each half, and 32-bit integer-to-float conversions (the
-// 64-bit conversion runs on the slow FP64 pipe).
-static_assert(kDig == 6, "digits() splits 42 bits as 3 + 3 digits");
-__device__ __forceinline__ void digits(long long w, float d[kDig]) {
-  const long long hh = (w + (1ll << 20)) >> 21;
-  int l = (int)(w - (hh << 21));
+// digits of a scaled value: w = round(x 2^(kBits-e)), |w| <= 2^kBits, written
+// as sum_t a_t 2^(kBits-7t) with |a_1| <= 128 and |a_t| <= 64, by integer
+// rounding divisions (exact; the digits are integers, exact in BF16). One
+// 64-bit rounding split w = h 2^S + l (S = kBits / 2, |l| <= 2^(S-1)) leaves
+// 32-bit work: half of the digits from each part, and 32-bit
+// integer-to-float conversions (the 64-bit conversion runs on the slow FP64
+// pipe).
+template <int kDig>
+__device__ __forceinline__ void digits(long long w, float (&d)[kDig]) {
+  constexpr int H = kDig / 2, S = 7 * H;
+  const long long hh = (w + (1ll << (S - 1))) >> S;
+  int l = (int)(w - (hh << S));
   int h = (int)hh;
 #pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int sh = 14 - 7 * t;
+  for (int t = 0; t < H - 1; ++t) {
+    const int sh = 7 * (H - 1 - t);
     const int a = (h + (1 << (sh - 1))) >> sh;
     d[t] = (float)a;
     h -= a << sh;
     const int b = (l + (1 << (sh - 1))) >> sh;
-    d[3 + t] = (float)b;
+    d[H + t] = (float)b;
     l -= b << sh;
   }
-  d[2] = (float)h;
-  d[5] = (float)l;
+  d[H - 1] = (float)h;
+  d[kDig - 1] = (float)l;
 }
 
-// w = round(x 2^(42 - e)) for |x| < 2^e, from the bits of x with integer
+// w = round(x 2^(kBits - e)) for |x| < 2^e, from the bits of x with integer
 // operations only (round half away from zero; the FP64 pipe is slow)
+template <int kBits>
 __device__ __forceinline__ long long scaledInt(double x, int e) {
   const long long bits = __double_as_longlong(x);
   const int ex = (int)((bits >> 52) & 0x7FF);
   if (ex == 0) return 0; // zero or subnormal: below 2^-1022
   const long long mant = (bits & 0xFFFFFFFFFFFFFll) | (1ll << 52);
-  // x = mant 2^(ex - 1075); the result is mant 2^(ex - 1033 - e), where the
-  // shift is <= -11 since |x| < 2^e
-  const int sh = 1033 + e - ex;
+  // x = mant 2^(ex - 1075); the result is mant 2^(ex - 1075 + kBits - e),
+  // where the right shift is >= 53 - kBits since |x| < 2^e
+  const int sh = 1075 - kBits + e - ex;
   if (sh >= 63) return 0;
-  const long long w = (mant + (1ll << (sh - 1))) >> sh;
+  const long long w =
+      sh > 0 ? (mant + (1ll << (sh - 1))) >> sh : mant << (kBits > 53 ? -sh : 0);
   return bits < 0 ? -w : w;
 }
 
 // per column c of the interleaved block X (N x 2p): the power of two
 // sc[c] = 2^e above its max-abs, and e = ex[c]. Pass 1: blocks (complex
 // column, row chunk) fold |Re| and |Im| maxima into sc as IEEE bit patterns
-// (for non-negative doubles the integer order is the numeric order); pass
-// 2 turns them into exponents.
+// (for non-negative doubles the integer order is the numeric order, and a
+// NaN or an infinity stays the largest); pass 2 turns them into exponents.
+// flag (may be null): set when a column holds a NaN or an infinity, or its
+// maximum is outside [2^-900, 2^900], where the scaled products could leave
+// the normal range: the caller's plain FP64 kernel then computes the product.
 __global__ void colMaxKernel(const double2 *X, size_t ld, int p, size_t N,
                              size_t rowsPerBlock, double *sc) {
-  __shared__ double sh[2][256];
+  using u64 = unsigned long long;
+  __shared__ u64 sh[2][256];
   const int c = blockIdx.x;
   const size_t r0 = (size_t)blockIdx.y * rowsPerBlock;
   const size_t r1 = r0 + rowsPerBlock < N ? r0 + rowsPerBlock : N;
-  double mr = 0, mi = 0;
+  u64 mr = 0, mi = 0;
+  auto mag = [](double x) {
+    return (u64)(__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll);
+  };
   const double2 *col = X + (size_t)c * ld;
   size_t r = r0 + threadIdx.x;
   for (; r + 3 * blockDim.x < r1; r += 4 * blockDim.x) {
@@ -166,33 +197,40 @@ __global__ void colMaxKernel(const double2 *X, size_t ld, int p, size_t N,
     for (int i = 0; i < 4; ++i) v[i] = col[r + i * blockDim.x];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      mr = fmax(mr, fabs(v[i].x));
-      mi = fmax(mi, fabs(v[i].y));
+      mr = max(mr, mag(v[i].x));
+      mi = max(mi, mag(v[i].y));
     }
   }
   for (; r < r1; r += blockDim.x) {
     const double2 v = col[r];
-    mr = fmax(mr, fabs(v.x));
-    mi = fmax(mi, fabs(v.y));
+    mr = max(mr, mag(v.x));
+    mi = max(mi, mag(v.y));
   }
   sh[0][threadIdx.x] = mr;
   sh[1][threadIdx.x] = mi;
   __syncthreads();
   for (int s = blockDim.x / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
-      sh[0][threadIdx.x] = fmax(sh[0][threadIdx.x], sh[0][threadIdx.x + s]);
-      sh[1][threadIdx.x] = fmax(sh[1][threadIdx.x], sh[1][threadIdx.x + s]);
+      sh[0][threadIdx.x] = max(sh[0][threadIdx.x], sh[0][threadIdx.x + s]);
+      sh[1][threadIdx.x] = max(sh[1][threadIdx.x], sh[1][threadIdx.x + s]);
     }
     __syncthreads();
   }
   if (threadIdx.x < 2)
-    atomicMax(reinterpret_cast<unsigned long long *>(sc) + 2 * c + threadIdx.x,
-              (unsigned long long)__double_as_longlong(sh[threadIdx.x][0]));
+    atomicMax(reinterpret_cast<u64 *>(sc) + 2 * c + threadIdx.x,
+              sh[threadIdx.x][0]);
 }
-__global__ void colExpKernel(int cols, double *sc, int *exq) {
+// exponent field of 2^900 and 2^-900 (bias 1023)
+constexpr int kExpHi = 1023 + 900, kExpLo = 1023 - 900;
+__device__ __forceinline__ bool expOutside(double x) {
+  const int f = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
+  return f > kExpHi || (f < kExpLo && x != 0.0);
+}
+__global__ void colExpKernel(int cols, double *sc, int *exq, int *flag) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   const double m = sc[c]; // the bit pattern written by colMaxKernel
+  if (flag && expOutside(m)) *flag = 1;
   int e = 0;
   if (m > 0) frexp(m, &e); // m < 2^e
   sc[c] = ldexp(1.0, e);   // column scale: entries / sc in (-1, 1)
@@ -200,18 +238,19 @@ __global__ void colExpKernel(int cols, double *sc, int *exq) {
 }
 // column maxima of the p complex columns of X (2p interleaved real columns)
 void colMax(const double2 *X, size_t ld, int p, size_t N, double *sc, int *ex,
-            cudaStream_t s) {
+            int *flag, cudaStream_t s) {
   const int chunks = (int)std::min<size_t>(
       std::max<size_t>(1, (size_t)(4 * smCount()) / (size_t)std::max(p, 1)),
       (N + 4095) / 4096);
   const size_t rows = (N + chunks - 1) / chunks;
   cudaMemsetAsync(sc, 0, 2 * (size_t)p * sizeof(double), s);
   colMaxKernel<<<dim3(p, chunks), 256, 0, s>>>(X, ld, p, N, rows, sc);
-  colExpKernel<<<(2 * p + 127) / 128, 128, 0, s>>>(2 * p, sc, ex);
+  colExpKernel<<<(2 * p + 127) / 128, 128, 0, s>>>(2 * p, sc, ex, flag);
 }
 
 // packs the BF16 digits t of 8 consecutive values into one 16-byte row of a
 // core matrix (element k at byte 2k)
+template <int kDig>
 __device__ __forceinline__ uint4 packRow(const float (*d)[kDig], int t) {
   uint4 w;
   __nv_bfloat162 b;
@@ -232,11 +271,19 @@ __device__ __forceinline__ uint4 packRow(const float (*d)[kDig], int t) {
 // Thread (complex column cc of the tile, 8-row group kq) loads 8 consecutive
 // entries (4 lanes read 512 contiguous bytes) and writes one 16-byte core
 // row per digit for Re (tile row 2 cc) and Im (2 cc + 1). Rows past N and
-// columns past p are zero digits.
+// columns past p are zero digits. sq (8 digits, the Gram of a block with
+// itself): the products of level 8, the first one that the MMAs leave out,
+// of every real column with itself. Between different columns those products
+// have random signs; in a column's square the term a_4^2 does not, and left
+// out it would put 2e-15 on the diagonal of a block of narrow peaks.
+template <int kDig>
 __global__ void __launch_bounds__(256)
     digitizeGramKernel(const double2 *__restrict__ X, size_t ld, int p,
                        size_t N, const int *__restrict__ ex, int nslab,
-                       unsigned char *__restrict__ img) {
+                       unsigned char *__restrict__ img, const int *flag,
+                       unsigned long long *__restrict__ sq) {
+  constexpr int kTile = Fmt<kDig>::kTile;
+  if (flag && *flag) return;
   const int s = blockIdx.x, mt = blockIdx.y;
   const int kq = threadIdx.x & 3, cc = threadIdx.x >> 2;
   const int c = mt * (kM / 2) + cc;
@@ -253,12 +300,27 @@ __global__ void __launch_bounds__(256)
     float d[8][kDig];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      digits(scaledInt(part ? v[i].y : v[i].x, e), d[i]);
+      digits<kDig>(scaledInt<Fmt<kDig>::kBits>(part ? v[i].y : v[i].x, e),
+                   d[i]);
     const uint32_t o = off16(2 * cc + part, 8 * kq);
 #pragma unroll
     for (int t = 0; t < kDig; ++t)
       *reinterpret_cast<uint4 *>(base + (size_t)t * kABytes + o) =
-          packRow(d, t);
+          packRow<kDig>(d, t);
+    if (kDig == 8 && sq) {
+      // level 8 of the column's square, in integers below 2^18
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        m += d[i][4] * d[i][4] +
+             2.f * (d[i][1] * d[i][7] + d[i][2] * d[i][6] +
+                    d[i][3] * d[i][5]);
+      int k = __float2int_rn(m);
+      k += __shfl_xor_sync(0xffffffffu, k, 1);
+      k += __shfl_xor_sync(0xffffffffu, k, 2);
+      if (kq == 0 && c < p)
+        atomicAdd(sq + 2 * c + part, (unsigned long long)(long long)k);
+    }
   }
 }
 
@@ -272,6 +334,7 @@ __global__ void __launch_bounds__(256)
     digitizeVCKernel(const double2 *__restrict__ V, size_t ld, int m,
                      size_t N, const int *__restrict__ ex, int nslab,
                      unsigned char *__restrict__ img) {
+  constexpr int kDig = 6, kTile = Fmt<kDig>::kTile;
   const int mt = blockIdx.x, s = blockIdx.y;
   unsigned char *base = img + ((size_t)mt * nslab + s) * (size_t)kTile;
   for (int task = threadIdx.x; task < kM * (kSlab / 8); task += 256) {
@@ -287,14 +350,90 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool in = c0 + i < m;
-      digits(scaledInt(v[i].x, in ? ex[2 * (c0 + i)] : 0), d[2 * i]);
-      digits(scaledInt(v[i].y, in ? ex[2 * (c0 + i) + 1] : 0), d[2 * i + 1]);
+      digits<kDig>(scaledInt<42>(v[i].x, in ? ex[2 * (c0 + i)] : 0), d[2 * i]);
+      digits<kDig>(scaledInt<42>(v[i].y, in ? ex[2 * (c0 + i) + 1] : 0),
+                   d[2 * i + 1]);
     }
     const uint32_t o = off16(row, 8 * kq);
 #pragma unroll
     for (int t = 0; t < kDig; ++t)
       *reinterpret_cast<uint4 *>(base + (size_t)t * kABytes + o) =
-          packRow(d, t);
+          packRow<kDig>(d, t);
+  }
+}
+
+// The same image with 8 digits and a power-of-two scale per lattice row on
+// top of the column scales (eR[r]: the row's entries, column-scaled, lie
+// below 2^eR), so that a row far from the nucleus, where every orbital is
+// small, keeps its own 56 bits as FP64 would. One block per 128-row tile:
+// the threads first take the row maxima over all columns (reading the tile
+// from memory), then digitise slab by slab (reading it from L1 / L2).
+__global__ void __launch_bounds__(256)
+    digitizeVCRowKernel(const double2 *__restrict__ V, size_t ld, int m,
+                        size_t N, const int *__restrict__ ex, int nslab,
+                        unsigned char *__restrict__ img,
+                        int *__restrict__ eR, const int *flag) {
+  constexpr int kDig = 8, kTile = Fmt<kDig>::kTile;
+  __shared__ int emax[2][kM];
+  if (*flag) return;
+  const int mt = blockIdx.x;
+  const int row = threadIdx.x & (kM - 1), half = threadIdx.x / kM;
+  const size_t r = (size_t)mt * kM + row;
+  // exponent e of a normal |x| < 2^e; none for zeros and subnormals
+  auto expOf = [](double x, int e) {
+    const int f = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
+    return f ? f - 1022 - e : -100000;
+  };
+  int em = -100000;
+  if (r < N) {
+    int c = half;
+    for (; c + 6 < m; c += 8) {
+      double2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = V[(size_t)(c + 2 * i) * ld + r];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        em = max(em, max(expOf(v[i].x, ex[2 * (c + 2 * i)]),
+                         expOf(v[i].y, ex[2 * (c + 2 * i) + 1])));
+    }
+    for (; c < m; c += 2) {
+      const double2 v = V[(size_t)c * ld + r];
+      em = max(em, max(expOf(v.x, ex[2 * c]), expOf(v.y, ex[2 * c + 1])));
+    }
+  }
+  emax[half][row] = em;
+  __syncthreads();
+  em = max(emax[0][row], emax[1][row]);
+  if (em == -100000) em = 0; // an all-zero row
+  if (half == 0 && r < N) eR[r] = em;
+  for (int s = 0; s < nslab; ++s) {
+    unsigned char *base = img + ((size_t)mt * nslab + s) * (size_t)kTile;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) { // 4 groups of 8 real columns, two a thread
+      const int kq = 2 * u + half;
+      const int c0 = s * (kSlab / 2) + 4 * kq;
+      double2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = (c0 + i < m && r < N) ? V[(size_t)(c0 + i) * ld + r]
+                                     : make_double2(0.0, 0.0);
+      float d[8][kDig];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool in = c0 + i < m;
+        digits<kDig>(
+            scaledInt<56>(v[i].x, em + (in ? ex[2 * (c0 + i)] : 0)),
+            d[2 * i]);
+        digits<kDig>(
+            scaledInt<56>(v[i].y, em + (in ? ex[2 * (c0 + i) + 1] : 0)),
+            d[2 * i + 1]);
+      }
+      const uint32_t o = off16(row, 8 * kq);
+#pragma unroll
+      for (int t = 0; t < kDig; ++t)
+        *reinterpret_cast<uint4 *>(base + (size_t)t * kABytes + o) =
+            packRow<kDig>(d, t);
+    }
   }
 }
 
@@ -318,16 +457,17 @@ __device__ __forceinline__ void mmaIssue(uint32_t td, uint64_t ad,
 // digit t and B digit u. B's digit planes lie 4 KB (8 row groups) apart, so
 // planes u0 .. u1 read as one B operand of N = 64 (u1 - u0 + 1) rows, and
 // one MMA with A digit t writes the levels t + u0 .. t + u1 into their
-// adjacent 64-column blocks of tensor memory: per 16 K, A digit 0 takes B
-// digits 0-3 and 4-5, digit 1 takes 0-3 and 4, digits 2 .. 5 take 0 ..
-// 5 - t (8 MMAs instead of 21). aBase / bBase: shared addresses of digit
+// adjacent 64-column blocks of tensor memory: per 16 K and with 6 digits, A
+// digit 0 takes B digits 0-3 and 4-5, digit 1 takes 0-3 and 4, digits 2 .. 5
+// take 0 .. 5 - t (8 MMAs instead of 21; with 8 digits 12 instead of 36). aBase / bBase: shared addresses of digit
 // plane 0 of A and B. first: the slab opens a fold block (A digit 0 writes
 // every level first and overwrites). Descriptors are the plane-0
 // descriptor plus a constant: the start-address field holds address / 16
 // and shared addresses stay below 256 KB, so the addition never carries.
+template <int kDig>
 __device__ __forceinline__ void issueSlab(uint32_t taddr, uint32_t aBase,
                                           uint32_t bBase, bool first) {
-  static_assert(kDig == 6 && kBBytes == 8 * kSBO, "stacked B planes");
+  static_assert(kBBytes == 8 * kSBO, "stacked B planes");
   const uint64_t a0 = smemDesc(aBase), b0 = smemDesc(bBase);
 #pragma unroll
   for (int ks = 0; ks < kSlab / 16; ++ks) {
@@ -353,7 +493,6 @@ __device__ __forceinline__ void issueSlab(uint32_t taddr, uint32_t aBase,
 // sum_l L_l 2^(7 (kDig-1-l)) = (L0 2^7 + L1) 2^28 + (L2 2^7 + L3) 2^14 +
 // (L4 2^7 + L5), each pair in 32 bits (|L_l| < 2^23), the sum below 2^58.1,
 // so kMaxFolds = 16 blocks stay below 2^63. Two levels per load wait.
-static_assert(kDig == 6, "foldLevels combines three level pairs");
 __device__ __forceinline__ void tmemLoad16(uint32_t ta, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, "
@@ -364,8 +503,48 @@ __device__ __forceinline__ void tmemLoad16(uint32_t ta, uint32_t (&v)[16]) {
         "=r"(v[15])
       : "r"(ta));
 }
-__device__ __forceinline__ void foldLevels(uint32_t taddr, int lw, int cBeg,
-                                           long long acc[32]) {
+__device__ __forceinline__ void tmemLoad8(uint32_t ta, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, "
+               "%5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]),
+                 "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(ta));
+}
+// The sums of one thread's 32 outputs. 6 digits: one 64-bit integer each.
+template <int kDig> struct Sums {
+  long long hi[32];
+  __device__ void clear() {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) hi[j] = 0;
+  }
+  __device__ void fold(uint32_t taddr, int lw, int cBeg);
+  // (sum) 2^e as a double
+  __device__ double value(int j, int e) const;
+  __device__ void storeLo(int *, int) const {}
+};
+// 8 digits: hi 2^14 + lo with |lo| <= 2^13. A fold adds (L0 2^7 + L1) 2^28 +
+// (L2 2^7 + L3) 2^14 + (L4 2^7 + L5) to hi and L6 2^7 + L7 to lo, whose
+// multiples of 2^14 carry into hi: every level is kept, exactly. |L_l| <=
+// 256 (2 2^13 + 6 2^12) < 2^23.4, so a pair stays below 2^30.5 in 32 bits and
+// hi below 2^58.1 per fold.
+template <> struct Sums<8> {
+  long long hi[32];
+  int lo[32];
+  __device__ void clear() {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      hi[j] = 0;
+      lo[j] = 0;
+    }
+  }
+  __device__ void fold(uint32_t taddr, int lw, int cBeg);
+  __device__ double value(int j, int e) const;
+  __device__ void storeLo(int *p, int j) const { *p = lo[j]; }
+};
+template <>
+__device__ __forceinline__ void Sums<6>::fold(uint32_t taddr, int lw,
+                                              int cBeg) {
+  long long *acc = hi;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const uint32_t ta =
@@ -416,6 +595,64 @@ __device__ __forceinline__ double scaledDouble(long long a, int e) {
                                           (keep & 0xFFFFFFFFFFFFFull)));
 }
 
+// the same of a 128-bit sum: its leading 62 bits, with a sticky last bit for
+// what is cut off
+__device__ __forceinline__ double scaledDouble128(__int128 a, int e) {
+  const bool neg = a < 0;
+  const unsigned __int128 m = neg ? -(unsigned __int128)a : (unsigned __int128)a;
+  const unsigned long long top = (unsigned long long)(m >> 62);
+  unsigned long long w = (unsigned long long)m;
+  int sh = 0;
+  if (top) {
+    sh = 64 - __clzll(top);
+    w = (unsigned long long)(m >> sh);
+    if (m & (((unsigned __int128)1 << sh) - 1)) w |= 1ull;
+  }
+  return scaledDouble(neg ? -(long long)w : (long long)w, e + sh);
+}
+
+template <>
+__device__ __forceinline__ double Sums<6>::value(int j, int e) const {
+  return scaledDouble(hi[j], e);
+}
+__device__ __forceinline__ void Sums<8>::fold(uint32_t taddr, int lw,
+                                              int cBeg) {
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const uint32_t ta =
+        taddr + ((uint32_t)(lw * 32) << 16) + (uint32_t)(cBeg + 8 * h);
+    int pr[4][8];
+#pragma unroll
+    for (int pl = 0; pl < 4; ++pl) {
+      uint32_t a[8], b[8];
+      tmemLoad8(ta + (uint32_t)(2 * pl * kN), a);
+      tmemLoad8(ta + (uint32_t)((2 * pl + 1) * kN), b);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        pr[pl][j] = __float2int_rn(__uint_as_float(a[j])) * 128 +
+                    __float2int_rn(__uint_as_float(b[j]));
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int t = lo[8 * h + j] + pr[3][j];
+      const int c = (t + (1 << 13)) >> 14;
+      lo[8 * h + j] = t - (c << 14);
+      hi[8 * h + j] += ((long long)pr[0][j] << 28) +
+                       ((long long)pr[1][j] << 14) + (long long)pr[2][j] +
+                       (long long)c;
+    }
+  }
+}
+// rounded from all bits while hi 2^14 + lo fits 62 bits; a larger hi keeps
+// 6 bits of lo, then none: below half a unit in the last place of a double
+__device__ __forceinline__ double Sums<8>::value(int j, int e) const {
+  const long long h = hi[j], a = h < 0 ? -h : h;
+  if (a < (1ll << 47)) return scaledDouble((h << 14) + lo[j], e);
+  if (a < (1ll << 55)) return scaledDouble((h << 6) + (lo[j] >> 8), e + 8);
+  return scaledDouble(h, e + 14);
+}
+
 __device__ __forceinline__ void tmemAlloc(uint32_t *slot) {
   asm volatile(
       "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::
@@ -447,7 +684,8 @@ __device__ __forceinline__ void bulkCopy(uint32_t dst, const void *src,
 // issues copies and MMAs and waits on every phase of mma and full in order;
 // the other threads wait only on fold, once per block, and every block ends
 // with a CTA barrier, so no barrier runs two phases ahead of a waiter.
-struct Pipe {
+template <int kDig> struct Pipe {
+  static constexpr int kStages = Fmt<kDig>::kStages, kBuf = Fmt<kDig>::kBuf;
   uint64_t *bar;
   uint32_t *tslot;
   int committed = 0, landedN = 0, issued = 0; // thread 0's counts of slabs
@@ -532,22 +770,35 @@ struct Pipe {
 };
 
 
+// every complex row of M tile mt lies below every complex column of N tile nt
+__host__ __device__ constexpr bool tileBelow(int mt, int nt) {
+  return mt * (kM / 2) > nt * (kN / 2) + kN / 2 - 1;
+}
+
 // C partials of one (M tile mt, N tile nt, row chunk): the digit tiles of
 // S^T (imgA, tile mt) and T^T (imgB, half nt & 1 of tile nt >> 1) over the
 // chunk's slabs (for a Gram of a block with itself imgB is imgA). Thread 0
 // runs the pipeline (bulk copies, MMAs, commits); all warps join at the
 // folds.
+// self: the Gram of a block with itself is Hermitian, so tiles below the
+// diagonal are left out (exactGramReduce mirrors the others; the sums are
+// exact, so the mirrored values are the ones those tiles would give). flag
+// (may be null): non-zero leaves the product to the plain kernel.
+template <int kDig>
 __global__ void __launch_bounds__(kThr, 1)
     exactGramKernel(const unsigned char *__restrict__ imgA,
                     const unsigned char *__restrict__ imgB, int p, int q,
                     int nslab, int slabsPerChunk,
-                    const int *__restrict__ eA,
-                    const int *__restrict__ eB, double *__restrict__ part,
-                    int *err) {
+                    long long *__restrict__ partHi, int *__restrict__ partLo,
+                    int self, const int *flag, int *err) {
+  constexpr int kTile = Fmt<kDig>::kTile, kBuf = Fmt<kDig>::kBuf,
+                kStages = Fmt<kDig>::kStages;
   extern __shared__ __align__(1024) unsigned char sm[];
-  Pipe P(sm);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int mt = blockIdx.x, nt = blockIdx.y, chunk = blockIdx.z;
+  if (self && tileBelow(mt, nt)) return;
+  if (flag && *flag) return;
+  Pipe<kDig> P(sm);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g0 = chunk * slabsPerChunk;
   const int ns = min(nslab, g0 + slabsPerChunk) - g0;
   const unsigned char *srcA = imgA + ((size_t)mt * nslab + g0) * kTile;
@@ -565,16 +816,15 @@ __global__ void __launch_bounds__(kThr, 1)
                P.full(st));
   };
   P.init(warp, tid);
+  constexpr int kAhead = kStages - 1; // slabs copied ahead of the MMAs
   if (tid == 0) {
-    copySlab(0);
-    if (ns > 1) copySlab(1);
-    P.issued = ns > 1 ? 2 : 1;
+    P.issued = min(ns, kAhead);
+    for (int s = 0; s < P.issued; ++s) copySlab(s);
   }
   const uint32_t taddr = P.taddr();
   const int lw = warp & 3, cBeg = (warp >> 2) * (kN / 2);
-  long long acc[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = 0;
+  Sums<kDig> acc;
+  acc.clear();
   bool ok = true;
   int fold = 0;
 
@@ -588,15 +838,15 @@ __global__ void __launch_bounds__(kThr, 1)
         if (!P.landed(s)) {
           ok = false;
         } else {
-          issueSlab(taddr, base, base + kDig * kABytes, s % kFold == 0);
+          issueSlab<kDig>(taddr, base, base + kDig * kABytes, s % kFold == 0);
           P.commit(s, foldPt);
-          // refill: slab s + 2 goes to the stage that the MMAs of slab s - 1
-          // read
-          if (s + 2 < ns) {
+          // refill: slab s + kAhead goes to the stage that the MMAs of slab
+          // s - 1 read
+          if (s + kAhead < ns) {
             if (s >= 1 && !P.mmaDone(s - 1))
               ok = false;
             else {
-              copySlab(s + 2);
+              copySlab(s + kAhead);
               ++P.issued;
             }
           }
@@ -609,21 +859,22 @@ __global__ void __launch_bounds__(kThr, 1)
         ok = false;
         break;
       }
-      foldLevels(taddr, lw, cBeg, acc);
+      acc.fold(taddr, lw, cBeg);
       P.foldDone();
     }
   }
   ok = P.finish(tid, ok);
   if (ok) {
-    // value = sum 2^(eA + eB - 7 (kDig+1))
     const int gr = mt * kM + lw * 32 + lane;
     if (gr < 2 * p) {
-      double *dst = part + ((size_t)chunk * 2 * p + gr) * (2 * q);
-      const int er = eA[gr] - 7 * (kDig + 1);
+      const size_t o = ((size_t)chunk * 2 * p + gr) * (2 * q);
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int gc = nt * kN + cBeg + j;
-        if (gc < 2 * q) dst[gc] = scaledDouble(acc[j], er + eB[gc]);
+        if (gc < 2 * q) {
+          partHi[o + gc] = acc.hi[j];
+          acc.storeLo(partLo + o + gc, j);
+        }
       }
     }
   } else if (tid == 0) {
@@ -632,28 +883,126 @@ __global__ void __launch_bounds__(kThr, 1)
   P.release(warp, taddr);
 }
 
-// one warp per output element: lane l sums chunks l, l + 32, ...; the lane
-// sums are combined in a fixed shuffle order (deterministic)
-__global__ void exactGramReduce(const double *__restrict__ part, int chunks,
-                                int p, int q, double2 *__restrict__ C,
-                                int ldc) {
+// Chunk partials: the exact sums as 64-bit integers (partHi) and, with 8
+// digits, their low parts (partLo; value = hi 2^14 + lo). They are added in
+// 128-bit integers and rounded once, so the result does not depend on the
+// chunking and the FP64 pipe (two operations per clock) stays out of it. The
+// real and the imaginary part each join two such sums. One warp per output element: lane l takes the chunks l,
+// l + 32, ... self: elements below the diagonal are the conjugates of those
+// above it.
+template <int kDig>
+__global__ void exactGramReduce(const long long *__restrict__ partHi,
+                                const int *__restrict__ partLo, int chunks,
+                                int p, int q, const int *__restrict__ eA,
+                                const int *__restrict__ eB,
+                                double2 *__restrict__ C, int ldc, int self,
+                                const long long *__restrict__ sq,
+                                const int *flag) {
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (e >= p * q) return;
-  const int i = e % p, j = e / p;
-  const size_t W = 2 * (size_t)q, H = 2 * (size_t)p;
-  double re = 0, im = 0;
-  for (int ch = lane; ch < chunks; ch += 32) {
-    const double *P = part + (size_t)ch * H * W;
-    re += P[(size_t)(2 * i) * W + 2 * j] + P[(size_t)(2 * i + 1) * W + 2 * j + 1];
-    im += P[(size_t)(2 * i) * W + 2 * j + 1] - P[(size_t)(2 * i + 1) * W + 2 * j];
+  if (e >= p * q || (flag && *flag)) return;
+  int i = e % p, j = e / p;
+  const bool mirror = self && i > j;
+  if (mirror) {
+    const int t = i;
+    i = j;
+    j = t;
   }
+  const size_t W = 2 * (size_t)q, step = 2 * (size_t)p * W;
+  // Re Re, Im Im, Re Im, Im Re
+  const size_t o0 = (size_t)(2 * i) * W + 2 * j;
+  const size_t off[4] = {o0, o0 + W + 1, o0 + 1, o0 + W};
+  __int128 t[4] = {0, 0, 0, 0};
+  for (int ch = lane; ch < chunks; ch += 32)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    re += __shfl_xor_sync(0xffffffffu, re, o);
-    im += __shfl_xor_sync(0xffffffffu, im, o);
+    for (int x = 0; x < 4; ++x) {
+      const size_t o = (size_t)ch * step + off[x];
+      t[x] += kDig == 8 ? ((__int128)partHi[o] << 14) + partLo[o]
+                        : (__int128)partHi[o];
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const unsigned long long lo = __shfl_xor_sync(
+          0xffffffffu, (unsigned long long)t[x], o);
+      const long long hi =
+          __shfl_xor_sync(0xffffffffu, (long long)(t[x] >> 64), o);
+      t[x] += ((__int128)hi << 64) | (__int128)(unsigned __int128)lo;
+    }
+  if (lane != 0) return;
+  int unit = 7 * (kDig + 1);
+  if (kDig == 8 && self && i == j) { // with level 8 of the squares
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      t[x] = (t[x] << 7) + (x < 2 ? sq[2 * i + x] : 0ll);
+    unit += 7;
   }
-  if (lane == 0) C[(size_t)j * ldc + i] = make_double2(re, im);
+  double v[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int ei = 2 * i + (x & 1), ej = 2 * j + (x == 1 || x == 2 ? 1 : 0);
+    v[x] = scaledDouble128(t[x], eA[ei] + eB[ej] - unit);
+  }
+  const double re = v[0] + v[1], im = v[2] - v[3];
+  if (mirror)
+    C[(size_t)i * ldc + j] = make_double2(re, -im);
+  else
+    C[(size_t)j * ldc + i] = make_double2(re, im);
+}
+
+// Plain FP64 forms of the two products for operands outside the digit
+// formats (flag set by colExpKernel / vcMaxKernel): infinities and NaNs come
+// out as an FP64 sum gives them. One warp per element of C, one thread per
+// element of Y; they return at once while the flag is clear.
+__global__ void plainGramKernel(const double2 *__restrict__ A, size_t lda,
+                                int p, const double2 *__restrict__ B,
+                                size_t ldb, int q, size_t N,
+                                double2 *__restrict__ C, int ldc,
+                                const int *flag) {
+  if (!*flag) return;
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); e < p * q;
+       e += warps) {
+    const double2 *a = A + (size_t)(e % p) * lda;
+    const double2 *b = B + (size_t)(e / p) * ldb;
+    double re = 0, im = 0;
+    for (size_t r = lane; r < N; r += 32) {
+      const double2 x = a[r], y = b[r];
+      re += x.x * y.x + x.y * y.y;
+      im += x.x * y.y - x.y * y.x;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (lane == 0) C[(size_t)(e / p) * ldc + e % p] = make_double2(re, im);
+  }
+}
+__global__ void plainVCKernel(const double2 *__restrict__ V, size_t ldv, int m,
+                              const double2 *__restrict__ Cm, int ldc, int k,
+                              double2 *__restrict__ Y, size_t ldy, size_t N,
+                              int accum, const int *flag) {
+  if (!*flag) return;
+  const size_t total = N * (size_t)k;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
+       e += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = e % N, j = e / N;
+    double2 s = make_double2(0.0, 0.0);
+    for (int l = 0; l < m; ++l) {
+      const double2 v = V[(size_t)l * ldv + r], c = Cm[j * ldc + l];
+      s.x += v.x * c.x - v.y * c.y;
+      s.y += v.x * c.y + v.y * c.x;
+    }
+    double2 &y = Y[j * ldy + r];
+    if (accum) {
+      s.x += y.x;
+      s.y += y.y;
+    }
+    y = s;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -674,7 +1023,7 @@ __global__ void exactGramReduce(const double *__restrict__ part, int chunks,
 // and the largest exponent is reduced over the warp
 __global__ void vcMaxKernel(const double2 *__restrict__ Cm, int ldc, int m,
                             int k, const int *__restrict__ eA, double *scB,
-                            int *eB) {
+                            int *eB, int *flag) {
   const int jr = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (jr >= 2 * k) return;
@@ -682,6 +1031,7 @@ __global__ void vcMaxKernel(const double2 *__restrict__ Cm, int ldc, int m,
   int emax = -100000;
   for (int c = lane; c < m; c += 32) {
     const double2 t = Cm[(size_t)j * ldc + c];
+    if (flag && (expOutside(t.x) || expOutside(t.y))) *flag = 1;
     // rows 2c, 2c+1 of column jr: (Re, -Im) for b = 0, (Im, Re) for b = 1
     const double v0 = b ? t.y : t.x, v1 = b ? t.x : -t.y;
     int e0 = -100000, e1 = -100000;
@@ -699,10 +1049,13 @@ __global__ void vcMaxKernel(const double2 *__restrict__ Cm, int ldc, int m,
   }
 }
 
+template <int kDig>
 __global__ void vcPrepKernel(const double2 *__restrict__ Cm, int ldc, int m,
                              int k, const int *__restrict__ eA,
                              const int *__restrict__ eB, int nslab,
-                             unsigned char *__restrict__ dig) {
+                             unsigned char *__restrict__ dig,
+                             const int *flag) {
+  if (flag && *flag) return;
   const int ntile = (2 * k + kN - 1) / kN;
   const size_t total = (size_t)nslab * kSlab * ntile * kN;
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -714,11 +1067,11 @@ __global__ void vcPrepKernel(const double2 *__restrict__ Cm, int ldc, int m,
     const int c = cr >> 1, a = cr & 1, j = jr >> 1, b = jr & 1;
     const double2 t = Cm[(size_t)j * ldc + c];
     const double v = b ? (a ? t.x : t.y) : (a ? -t.y : t.x);
-    // v 2^eA[cr] 2^-eB[jr] scaled to 42 bits: scaledInt(v, eB - eA)
-    w = scaledInt(v, eB[jr] - eA[cr]);
+    // v 2^eA[cr] 2^-eB[jr] scaled to kBits bits: scaledInt(v, eB - eA)
+    w = scaledInt<Fmt<kDig>::kBits>(v, eB[jr] - eA[cr]);
   }
   float d[kDig];
-  digits(w, d);
+  digits<kDig>(w, d);
   const int s = cr / kSlab, kk = cr % kSlab, nt = jr / kN, jj = jr % kN;
   unsigned char *base =
       dig + ((size_t)(nt * nslab + s) * kDig) * (size_t)kBBytes;
@@ -735,14 +1088,20 @@ __global__ void vcPrepKernel(const double2 *__restrict__ Cm, int ldc, int m,
 // so the copies of the next tile overlap the fold and the stores of the
 // current one. A: the digit image of V (imgV, tile (mt, s)); B: the
 // precomputed digit image of C (dig, tile (nt, s)).
+// eR (8 digits): the row exponents of digitizeVCRowKernel.
+template <int kDig>
 __global__ void __launch_bounds__(kThr, 1)
     exactVCKernel(const unsigned char *__restrict__ imgV,
                   const unsigned char *__restrict__ dig,
-                  const int *__restrict__ eB, int k, int nslab,
-                  int ntiles, int tiles, double2 *__restrict__ Y, size_t ldy,
-                  size_t N, int accum, int *err) {
+                  const int *__restrict__ eB, const int *__restrict__ eR,
+                  int k, int nslab, int ntiles, int tiles,
+                  double2 *__restrict__ Y, size_t ldy, size_t N, int accum,
+                  const int *flag, int *err) {
+  constexpr int kTile = Fmt<kDig>::kTile, kBuf = Fmt<kDig>::kBuf,
+                kStages = Fmt<kDig>::kStages;
   extern __shared__ __align__(1024) unsigned char sm[];
-  Pipe P(sm);
+  if (flag && *flag) return;
+  Pipe<kDig> P(sm);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = gridDim.x;
   const int myTiles = (tiles - (int)blockIdx.x + G - 1) / G;
@@ -761,16 +1120,15 @@ __global__ void __launch_bounds__(kThr, 1)
              kDig * kBBytes, P.full(st));
   };
   P.init(warp, tid);
-  if (tid == 0 && total > 0) {
-    copyStep(0);
-    if (total > 1) copyStep(1);
-    P.issued = total > 1 ? 2 : 1;
+  constexpr int kAhead = kStages - 1;
+  if (tid == 0) {
+    P.issued = min(total, kAhead);
+    for (int i = 0; i < P.issued; ++i) copyStep(i);
   }
   const uint32_t taddr = P.taddr();
   const int lw = warp & 3, cBeg = (warp >> 2) * (kN / 2);
-  long long acc[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) acc[j] = 0;
+  Sums<kDig> acc;
+  acc.clear();
   bool ok = true;
   int fold = 0;
 
@@ -783,13 +1141,13 @@ __global__ void __launch_bounds__(kThr, 1)
         if (!P.landed(i)) {
           ok = false;
         } else {
-          issueSlab(taddr, base, base + kDig * kABytes, s % kFold == 0);
+          issueSlab<kDig>(taddr, base, base + kDig * kABytes, s % kFold == 0);
           P.commit(i, foldPt);
-          if (i + 2 < total) {
+          if (i + kAhead < total) {
             if (i >= 1 && !P.mmaDone(i - 1))
               ok = false;
             else {
-              copyStep(i + 2);
+              copyStep(i + kAhead);
               ++P.issued;
             }
           }
@@ -802,21 +1160,22 @@ __global__ void __launch_bounds__(kThr, 1)
         ok = false;
         break;
       }
-      foldLevels(taddr, lw, cBeg, acc);
+      acc.fold(taddr, lw, cBeg);
       P.foldDone();
       if (s == nslab - 1) {
-        // Y[j][r] = (acc[2j] 2^eB[2j], acc[2j+1] 2^eB[2j+1]) 2^(-7 (kDig+1))
-        constexpr int ew = -7 * (kDig + 1);
+        // Y[j][r] = (sum[2j] 2^eB[2j], sum[2j+1] 2^eB[2j+1]) 2^eR[r]
+        // 2^(-7 (kDig+1))
         const int tile = (int)blockIdx.x + (i / nslab) * G;
         const int mt = tile / ntiles, nt = tile % ntiles;
         const size_t r = (size_t)mt * kM + lw * 32 + lane;
         if (r < N) {
+          const int ew = -7 * (kDig + 1) + (kDig == 8 ? eR[r] : 0);
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const int jr = nt * kN + cBeg + j;
             if (jr < 2 * k) {
-              double2 v = make_double2(scaledDouble(acc[j], ew + eB[jr]),
-                                       scaledDouble(acc[j + 1], ew + eB[jr + 1]));
+              double2 v = make_double2(acc.value(j, ew + eB[jr]),
+                                       acc.value(j + 1, ew + eB[jr + 1]));
               double2 &y = Y[(size_t)(jr >> 1) * ldy + r];
               if (accum) {
                 v.x += y.x;
@@ -826,8 +1185,7 @@ __global__ void __launch_bounds__(kThr, 1)
             }
           }
         }
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = 0;
+        acc.clear();
       }
     }
   }
@@ -839,9 +1197,12 @@ __global__ void __launch_bounds__(kThr, 1)
 // rows per chunk of the Gram grid: a multiple of one fold block and at most
 // kMaxFolds blocks (the 64-bit sums), chosen to minimise the waves of one
 // CTA per SM times the rows of a chunk (plus a fixed cost per CTA)
-int chunkRows(size_t N, int p, int q) {
-  const size_t tiles =
-      (size_t)((2 * p + kM - 1) / kM) * (size_t)((2 * q + kN - 1) / kN);
+int chunkRows(size_t N, int p, int q, bool self) {
+  const int mts = (2 * p + kM - 1) / kM, nts = (2 * q + kN - 1) / kN;
+  size_t tiles = (size_t)mts * nts;
+  if (self)
+    for (int mt = 0; mt < mts; ++mt)
+      for (int nt = 0; nt < nts; ++nt) tiles -= tileBelow(mt, nt) ? 1 : 0;
   const size_t blk = (size_t)kSlab * kFold;
   const size_t sms = (size_t)smCount();
   size_t best = blk;
@@ -859,12 +1220,123 @@ int chunkRows(size_t N, int p, int q) {
   return (int)best;
 }
 
-size_t gramImageBytes(size_t N, int p) {
+size_t gramImageBytes(size_t N, int p, int digits) {
   const size_t nslab = (N + kSlab - 1) / kSlab;
-  return nslab * (size_t)((2 * p + kM - 1) / kM) * kTile;
+  return nslab * (size_t)((2 * p + kM - 1) / kM) * digits * kABytes;
 }
+// column scales (doubles) and exponents (ints) of both operands, the flag,
+// the level-8 squares
 size_t gramHeaderBytes(int p, int q) {
   return ((sizeof(double) * (4 * (size_t)(p + q) + 8)) + 255) & ~(size_t)255;
+}
+size_t vcHeaderBytes(int m, int k) {
+  return ((size_t)24 * (2 * m + 2 * k) + 64 + 255) & ~(size_t)255;
+}
+
+template <int kDig>
+void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
+                size_t ldb, int q, size_t N, double2 *C, int ldc,
+                double *scratch, cudaStream_t s) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(exactGramKernel<kDig>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         Fmt<kDig>::kSmem);
+    return true;
+  }();
+  (void)attr;
+  const bool self = A == B && lda == ldb && p == q;
+  double *scA = scratch, *scB = scA + 2 * (size_t)p;
+  int *eA = reinterpret_cast<int *>(scB + 2 * (size_t)q);
+  int *eB = eA + 2 * (size_t)p;
+  // the FP64 form hands operands outside the digit format to plainGramKernel
+  int *flag = kDig == 8 ? eB + 2 * (size_t)q : nullptr;
+  // 2p sums behind the flag (zeroed with the header)
+  auto *sq = kDig == 8 && self ? reinterpret_cast<unsigned long long *>(
+                                     scratch + 3 * (size_t)(p + q) + 1)
+                               : nullptr;
+  const size_t head = gramHeaderBytes(p, q);
+  unsigned char *imgA = reinterpret_cast<unsigned char *>(scratch) + head;
+  unsigned char *imgB = imgA + gramImageBytes(N, p, kDig);
+  long long *partHi =
+      reinterpret_cast<long long *>(imgB + gramImageBytes(N, q, kDig));
+  const int nslab = (int)((N + kSlab - 1) / kSlab);
+  cudaMemsetAsync(scratch, 0, head, s);
+  colMax(A, lda, p, N, scA, eA, flag, s);
+  if (!self) colMax(B, ldb, q, N, scB, eB, flag, s);
+  digitizeGramKernel<kDig>
+      <<<dim3(nslab, (2 * p + kM - 1) / kM), 256, 0, s>>>(
+          A, lda, p, N, eA, nslab, imgA, flag, sq);
+  if (self) {
+    imgB = imgA;
+    eB = eA;
+  } else {
+    digitizeGramKernel<kDig>
+        <<<dim3(nslab, (2 * q + kM - 1) / kM), 256, 0, s>>>(
+            B, ldb, q, N, eB, nslab, imgB, flag, nullptr);
+  }
+  const int rows = chunkRows(N, p, q, self);
+  const int spc = rows / kSlab;
+  const int chunks = (nslab + spc - 1) / spc;
+  dim3 grid((2 * p + kM - 1) / kM, (2 * q + kN - 1) / kN, chunks);
+  int *partLo = reinterpret_cast<int *>(partHi + (size_t)chunks * 4 * p * q);
+  exactGramKernel<kDig><<<grid, kThr, Fmt<kDig>::kSmem, s>>>(
+      imgA, imgB, p, q, nslab, spc, partHi, partLo, self ? 1 : 0, flag,
+      exactGramErrWord());
+  exactGramReduce<kDig>
+      <<<(unsigned)(((size_t)p * q * 32 + 255) / 256), 256, 0, s>>>(
+          partHi, partLo, chunks, p, q, eA, eB, C, ldc, self ? 1 : 0,
+          reinterpret_cast<const long long *>(sq), flag);
+  if (flag)
+    plainGramKernel<<<2 * smCount(), 256, 0, s>>>(A, lda, p, B, ldb, q, N, C,
+                                                  ldc, flag);
+}
+
+template <int kDig>
+void vcDigits(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
+              int k, double2 *Y, size_t ldy, size_t N, void *scratch,
+              cudaStream_t s, bool accum) {
+  static const bool attr = [] {
+    cudaFuncSetAttribute(exactVCKernel<kDig>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         Fmt<kDig>::kSmem);
+    return true;
+  }();
+  (void)attr;
+  const int nslab = (2 * m + kSlab - 1) / kSlab;
+  const int ntile = (2 * k + kN - 1) / kN;
+  const int mtile = (int)((N + kM - 1) / kM);
+  unsigned char *base = static_cast<unsigned char *>(scratch);
+  double *scA = reinterpret_cast<double *>(base);
+  double *scB = scA + 2 * (size_t)m;
+  int *eA = reinterpret_cast<int *>(scB + 2 * (size_t)k);
+  int *eB = eA + 2 * (size_t)m;
+  int *flag = kDig == 8 ? eB + 2 * (size_t)k : nullptr;
+  const size_t head = vcHeaderBytes(m, k);
+  unsigned char *dig = base + head;
+  unsigned char *imgV = dig + (size_t)ntile * nslab * kDig * kBBytes;
+  int *eR = reinterpret_cast<int *>(imgV +
+                                    (size_t)mtile * nslab * Fmt<kDig>::kTile);
+  cudaMemsetAsync(base, 0, head, s);
+  colMax(V, ldv, m, N, scA, eA, flag, s);
+  vcMaxKernel<<<(2 * k + 3) / 4, 128, 0, s>>>(Cm, ldc, m, k, eA, scB, eB,
+                                              flag);
+  const size_t total = (size_t)nslab * kSlab * ntile * kN;
+  vcPrepKernel<kDig><<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
+      Cm, ldc, m, k, eA, eB, nslab, dig, flag);
+  if (kDig == 8)
+    digitizeVCRowKernel<<<mtile, 256, 0, s>>>(V, ldv, m, N, eA, nslab, imgV,
+                                              eR, flag);
+  else
+    digitizeVCKernel<<<dim3(mtile, nslab), 256, 0, s>>>(V, ldv, m, N, eA,
+                                                        nslab, imgV);
+  const int tiles = mtile * ntile;
+  const int G = std::min(tiles, smCount());
+  exactVCKernel<kDig><<<G, kThr, Fmt<kDig>::kSmem, s>>>(
+      imgV, dig, eB, eR, k, nslab, ntile, tiles, Y, ldy, N, accum ? 1 : 0,
+      flag, exactGramErrWord());
+  if (flag)
+    plainVCKernel<<<2 * smCount(), 256, 0, s>>>(V, ldv, m, Cm, ldc, k, Y, ldy,
+                                                N, accum ? 1 : 0, flag);
 }
 
 } // namespace
@@ -874,19 +1346,29 @@ size_t gramHeaderBytes(int p, int q) {
 // partials. The row chunking gives a product with fewer output tiles more
 // chunks, so a narrower product can need more partials than the widest one;
 // the bound is the largest over every (M tiles, N tiles) count up to those
-// of (p, q), each with its widest p', q'.
-size_t exactGramScratchDoubles(size_t N, int p, int q) {
+// of (p, q), each with its widest p', q' (and, for equal widths, over the
+// tiles on and above the diagonal alone).
+size_t exactGramScratchDoubles(size_t N, int p, int q, int digits) {
   const int mtiles = (2 * p + kM - 1) / kM, ntiles = (2 * q + kN - 1) / kN;
   size_t part = 0;
   for (int a = 1; a <= mtiles; ++a)
     for (int b = 1; b <= ntiles; ++b) {
       const int pp = std::min(p, a * kM / 2), qq = std::min(q, b * kN / 2);
-      const size_t rows = chunkRows(N, pp, qq);
+      const size_t rows = chunkRows(N, pp, qq, false);
       const size_t chunks = (N + rows - 1) / rows;
       part = std::max(part, chunks * 4 * (size_t)pp * qq);
     }
-  const size_t bytes = gramHeaderBytes(p, q) + gramImageBytes(N, p) +
-                       gramImageBytes(N, q) + sizeof(double) * part + 256;
+  for (int b = 1; b <= ntiles; ++b) {
+    const int w = std::min(std::min(p, q), b * kN / 2);
+    const size_t rows = chunkRows(N, w, w, true);
+    const size_t chunks = (N + rows - 1) / rows;
+    part = std::max(part, chunks * 4 * (size_t)w * w);
+  }
+  const size_t bytes = gramHeaderBytes(p, q) + gramImageBytes(N, p, digits) +
+                       gramImageBytes(N, q, digits) +
+                       (sizeof(long long) + (digits == 8 ? sizeof(int) : 0)) *
+                           part +
+                       256;
   return (bytes + sizeof(double) - 1) / sizeof(double);
 }
 
@@ -900,65 +1382,34 @@ int *exactGramErrWord() {
   return d;
 }
 
-// C = A^H B on the tensor cores to ~1e-13 relative (see the file comment);
-// scratch holds exactGramScratchDoubles(N, p, q) doubles (256-byte aligned).
-// A Gram of a block with itself (A == B, same ld and width) digitises it once.
+// C = A^H B on the tensor cores with 6 digits (~1e-13 relative) or 8 (at
+// least FP64's accuracy; see the file comment); scratch holds
+// exactGramScratchDoubles(N, p, q, digits) doubles (256-byte aligned). A Gram
+// of a block with itself (A == B, same ld and width) digitises it once.
 void gramTCExact(const double2 *A, size_t lda, int p, const double2 *B,
                  size_t ldb, int q, size_t N, double2 *C, int ldc,
-                 double *scratch, cudaStream_t s) {
+                 double *scratch, cudaStream_t s, int digits) {
   if (p == 0 || q == 0 || N == 0) return;
-  static const bool attr = [] {
-    cudaFuncSetAttribute(exactGramKernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    return true;
-  }();
-  (void)attr;
-  const bool self = A == B && lda == ldb && p == q;
-  double *scA = scratch, *scB = scA + 2 * (size_t)p;
-  int *eA = reinterpret_cast<int *>(scB + 2 * (size_t)q);
-  int *eB = eA + 2 * (size_t)p;
-  unsigned char *imgA =
-      reinterpret_cast<unsigned char *>(scratch) + gramHeaderBytes(p, q);
-  unsigned char *imgB = imgA + gramImageBytes(N, p);
-  double *part = reinterpret_cast<double *>(imgB + gramImageBytes(N, q));
-  const int nslab = (int)((N + kSlab - 1) / kSlab);
-  colMax(A, lda, p, N, scA, eA, s);
-  digitizeGramKernel<<<dim3(nslab, (2 * p + kM - 1) / kM), 256, 0, s>>>(
-      A, lda, p, N, eA, nslab, imgA);
-  if (self) {
-    imgB = imgA;
-    eB = eA;
-  } else {
-    colMax(B, ldb, q, N, scB, eB, s);
-    digitizeGramKernel<<<dim3(nslab, (2 * q + kM - 1) / kM), 256, 0, s>>>(
-        B, ldb, q, N, eB, nslab, imgB);
-  }
-  const int rows = chunkRows(N, p, q);
-  const int spc = rows / kSlab;
-  const int chunks = (nslab + spc - 1) / spc;
-  dim3 grid((2 * p + kM - 1) / kM, (2 * q + kN - 1) / kN, chunks);
-  exactGramKernel<<<grid, kThr, kSmem, s>>>(imgA, imgB, p, q, nslab, spc,
-                                            eA, eB, part,
-                                            exactGramErrWord());
-  exactGramReduce<<<(unsigned)(((size_t)p * q * 32 + 255) / 256), 256, 0, s>>>(
-      part, chunks, p, q, C, ldc);
+  (digits == 8 ? gramDigits<8> : gramDigits<6>)(A, lda, p, B, ldb, q, N, C,
+                                                ldc, scratch, s);
 }
 
 // scratch of gemmVCExact in bytes: A column scales / exponents (2m), B
-// column scales / exponents (2k), the digit image of B and that of V
-size_t exactVCScratchBytes(size_t N, int m, int k) {
+// column scales / exponents (2k), the digit image of B and that of V, and
+// the row exponents
+size_t exactVCScratchBytes(size_t N, int m, int k, int digits) {
   const size_t nslab = (2 * (size_t)m + kSlab - 1) / kSlab;
   const size_t ntile = (2 * (size_t)k + kN - 1) / kN;
   const size_t mtile = (N + kM - 1) / kM;
-  return 512 + 16 * (size_t)(2 * m + 2 * k) + ntile * nslab * kDig * kBBytes +
-         mtile * nslab * kTile;
+  return 512 + vcHeaderBytes(m, k) + ntile * nslab * digits * kBBytes +
+         mtile * nslab * digits * kABytes + N * sizeof(int);
 }
 
-// Y = V C (accum: Y += V C) to ~1e-12 relative of the column maxima (see
-// above)
+// Y = V C (accum: Y += V C) to ~1e-12 relative of the column maxima (6
+// digits) or FP64's accuracy (8 digits; see above)
 void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *Cm,
                  int ldc, int k, double2 *Y, size_t ldy, size_t N,
-                 void *scratch, cudaStream_t s, bool accum) {
+                 void *scratch, cudaStream_t s, bool accum, int digits) {
   if (k == 0 || N == 0) return;
   if (m == 0) {
     if (accum) return;
@@ -966,35 +1417,8 @@ void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *Cm,
       cudaMemsetAsync(Y + (size_t)j * ldy, 0, N * sizeof(double2), s);
     return;
   }
-  static const bool attr = [] {
-    cudaFuncSetAttribute(exactVCKernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    return true;
-  }();
-  (void)attr;
-  const int nslab = (2 * m + kSlab - 1) / kSlab;
-  const int ntile = (2 * k + kN - 1) / kN;
-  const int mtile = (int)((N + kM - 1) / kM);
-  unsigned char *base = static_cast<unsigned char *>(scratch);
-  double *scA = reinterpret_cast<double *>(base);
-  double *scB = scA + 2 * (size_t)m;
-  int *eA = reinterpret_cast<int *>(scB + 2 * (size_t)k);
-  int *eB = eA + 2 * (size_t)m;
-  unsigned char *dig =
-      base + (((size_t)16 * (2 * m + 2 * k) + 255) & ~(size_t)255);
-  unsigned char *imgV = dig + (size_t)ntile * nslab * kDig * kBBytes;
-  colMax(V, ldv, m, N, scA, eA, s);
-  vcMaxKernel<<<(2 * k + 3) / 4, 128, 0, s>>>(Cm, ldc, m, k, eA, scB, eB);
-  const size_t total = (size_t)nslab * kSlab * ntile * kN;
-  vcPrepKernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
-      Cm, ldc, m, k, eA, eB, nslab, dig);
-  digitizeVCKernel<<<dim3(mtile, nslab), 256, 0, s>>>(V, ldv, m, N, eA, nslab,
-                                                      imgV);
-  const int tiles = mtile * ntile;
-  const int G = std::min(tiles, smCount());
-  exactVCKernel<<<G, kThr, kSmem, s>>>(imgV, dig, eB, k, nslab, ntile, tiles,
-                                       Y, ldy, N, accum ? 1 : 0,
-                                       exactGramErrWord());
+  (digits == 8 ? vcDigits<8> : vcDigits<6>)(V, ldv, m, Cm, ldc, k, Y, ldy, N,
+                                            scratch, s, accum);
 }
 
 } // namespace ncgm
