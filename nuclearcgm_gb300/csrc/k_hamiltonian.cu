@@ -13,10 +13,9 @@
 // (skyrme_u.cpp:15-24), SkyrmeSO (skyrme_so.cpp:12-58) and
 // LocalCoulombPotential (local_coulomb_potential.cpp:12-41) summed.
 //
-// This file holds the FP64 kernel stencilPoint (one thread per (point,
-// column), neighbours through the L1/L2 caches; GB300's FP64 pipe, not HBM,
-// bounds it), the per-point coefficient builders and the Woods-Saxon guess
-// fields. The HBM-bound FP32 kernel is in k_stencil32.cu.
+// This file holds the FP64 product of small lattices, the per-point coefficient
+// builders and the Woods-Saxon guess fields. The FP64 product is otherwise in
+// k_stencil64.cu, the FP32 one in k_stencil32.cu.
 #include "ncgm_internal.cuh"
 #include "stencil_core.cuh"
 
@@ -32,44 +31,34 @@ namespace {
 constexpr double kHbar = 197.327053;
 constexpr double kMass = 938.91869;
 
-template <class T> struct V4;
-template <> struct V4<double> { using type = double4_32a; };
-template <> struct V4<float> { using type = float4; };
-
-template <class T>
-__device__ __forceinline__ Spinor<T> ldSpinor(const typename V4<T>::type *p) {
-  typename V4<T>::type v = *p;
-  return {v.x, v.y, v.z, v.w};
-}
-
-// ---- simple kernel: one thread per (point, column) ----------------------
-template <class T>
+// Small lattices: one thread per (point, column), neighbours through L1/L2.
 __global__ void __launch_bounds__(256)
-    stencilPoint(const typename V4<T>::type *__restrict__ X,
-                 typename V4<T>::type *__restrict__ Y,
-                 const typename V4<T>::type *__restrict__ coef, int n,
-                 size_t ns, T shift) {
-  using Vt = typename V4<T>::type;
+    stencilPoint(const double4_32a *__restrict__ X,
+                 double4_32a *__restrict__ Y,
+                 const double4_32a *__restrict__ coef, int n, size_t ns,
+                 double shift) {
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (p >= ns) return;
   const int col = blockIdx.y;
-  const Vt *x = X + (size_t)col * ns;
+  const double4_32a *x = X + (size_t)col * ns;
   const int i = (int)(p % n), j = (int)((p / n) % n), k = (int)(p / ((size_t)n * n));
   const size_t sy = n, sz = (size_t)n * n;
-  auto at = [&](int di, int dj, int dk) -> Spinor<T> {
+  auto at = [&](int di, int dj, int dk) -> Spinor<double> {
     int ii = i + di, jj = j + dj, kk = k + dk;
     if (ii < 0 || ii >= n || jj < 0 || jj >= n || kk < 0 || kk >= n)
-      return {T(0), T(0), T(0), T(0)};
+      return {0.0, 0.0, 0.0, 0.0};
     const long long q = (long long)p + di + dj * (long long)sy + dk * (long long)sz;
-    return ldSpinor<T>(x + q);
+    const double4_32a v = x[q];
+    return {v.x, v.y, v.z, v.w};
   };
-  Vt c0 = coef[2 * p], c1 = coef[2 * p + 1];
-  T c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-  Spinor<T> o = pointH<T>(c, shift, at(0, 0, 0), at(1, 0, 0), at(-1, 0, 0),
-                          at(2, 0, 0), at(-2, 0, 0), at(0, 1, 0), at(0, -1, 0),
-                          at(0, 2, 0), at(0, -2, 0), at(0, 0, 1), at(0, 0, -1),
-                          at(0, 0, 2), at(0, 0, -2));
-  Y[(size_t)col * ns + p] = Vt{o.r0, o.i0, o.r1, o.i1};
+  const double4_32a c0 = coef[2 * p], c1 = coef[2 * p + 1];
+  double c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+  Spinor<double> o =
+      pointH<double>(c, shift, at(0, 0, 0), at(1, 0, 0), at(-1, 0, 0),
+                     at(2, 0, 0), at(-2, 0, 0), at(0, 1, 0), at(0, -1, 0),
+                     at(0, 2, 0), at(0, -2, 0), at(0, 0, 1), at(0, 0, -1),
+                     at(0, 0, 2), at(0, 0, -2));
+  Y[(size_t)col * ns + p] = double4_32a{o.r0, o.i0, o.r1, o.i1};
 }
 
 // ---- coefficient builders -------------------------------------------------
@@ -179,9 +168,11 @@ int buildCoefficients(ncgm_ctx *ctx, int species, const double *f,
     NCGM_CUDA(cudaMalloc(&F.coef64, ctx->ns * 8 * sizeof(double)));
     NCGM_CUDA(cudaMalloc(&F.coef32, ctx->ns * 8 * sizeof(float)));
     NCGM_CUDA(cudaMalloc(&F.coef32s, ctx->ns * 8 * sizeof(float)));
+    NCGM_CUDA(cudaMalloc(&F.coefInt, intCoefBytes(ctx->ns)));
   }
   buildCoefKernel<<<(unsigned)((ctx->ns + 255) / 256), 256, 0, ctx->stream>>>(
       f, gradf, U, W, UC, ctx->ns, ctx->h, F.coef64, F.coef32, F.coef32s);
+  buildIntCoefficients(F.coef64, ctx->ns, F.coefInt, ctx->stream);
   NCGM_CUDA(cudaGetLastError());
   F.ready = true;
   return NCGM_OK;
@@ -203,11 +194,22 @@ int buildWoodsSaxon(ncgm_ctx *ctx, int species, int A, int Z, double V0,
 
 void applyH64(ncgm_ctx *ctx, int species, const double2 *X, double2 *Y,
               int ncols, double shift, cudaStream_t s) {
+  const SpeciesFields &F = ctx->sp[species];
+  // A tile of the integer form shares one scale. On a fine mesh it spans 4 to
+  // 5 fm and every digit of FP64 survives; on lattices of fewer than 15
+  // points per axis the mesh is coarse, a tile covers half of the box, and
+  // an orbital falls by more than the spare bits inside it. Those keep the
+  // FP64 kernel (12^3 x 4 columns: 16 us against 10; 16^3 x 16: 27 against 12;
+  // 36^3 x 60: 760 against 213).
+  if (ctx->n >= 15) {
+    applyHInt(X, Y, F.coef64, F.coefInt, ctx->n, ncols, shift, s);
+    return;
+  }
   dim3 grid((unsigned)((ctx->ns + 255) / 256), ncols);
-  stencilPoint<double><<<grid, 256, 0, s>>>(
-      reinterpret_cast<const double4_32a *>(X), reinterpret_cast<double4_32a *>(Y),
-      reinterpret_cast<const double4_32a *>(ctx->sp[species].coef64), ctx->n,
-      ctx->ns, shift);
+  stencilPoint<<<grid, 256, 0, s>>>(
+      reinterpret_cast<const double4_32a *>(X),
+      reinterpret_cast<double4_32a *>(Y),
+      reinterpret_cast<const double4_32a *>(F.coef64), ctx->n, ctx->ns, shift);
 }
 
 int stencilErrorFlag() {

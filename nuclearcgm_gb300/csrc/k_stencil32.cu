@@ -1,6 +1,6 @@
 // FP32 H.X stencil: persistent streaming kernel on TMA tensor tiles.
 //
-// Same operator as stencilPoint in k_hamiltonian.cu (the matrix-free form of
+// Same operator as the FP64 product of k_stencil64.cu (the matrix-free form of
 // Hamiltonian::buildMatrix, src/hamiltonian/hamiltonian.cpp:303-372), built
 // for HBM bandwidth on GB300:
 //  * A 5-D tensor map views X as [col][k][j][i][4 floats]. One TMA box is a

@@ -41,6 +41,7 @@ struct SpeciesFields {
   double *coef64 = nullptr; // ns x 8
   float *coef32 = nullptr;  // ns x 8
   float *coef32s = nullptr; // 2 x ns x 4: lo halves of all points, then hi
+  void *coefInt = nullptr;  // integer form of coef64 (k_stencil64.cu)
   bool ready = false;
 };
 
@@ -84,6 +85,15 @@ int buildWoodsSaxon(ncgm_ctx *ctx, int species, int A, int Z, double V0,
 // Y = (H + shift) X on device buffers, ncols columns, leading dim N.
 void applyH64(ncgm_ctx *ctx, int species, const double2 *X, double2 *Y,
               int ncols, double shift, cudaStream_t s);
+// The FP64 product on the integer pipes (k_stencil64.cu): X, Y 16-byte
+// aligned; intCoef: intCoefBytes(ns) bytes filled by buildIntCoefficients from
+// the same coef64.
+size_t intCoefBytes(size_t ns);
+void buildIntCoefficients(const double *coef64, size_t ns, void *buf,
+                          cudaStream_t s);
+void applyHInt(const double2 *X, double2 *Y, const double *coef64,
+               const void *intCoef, int n, int ncols, double shift,
+               cudaStream_t s);
 void applyH32(ncgm_ctx *ctx, int species, const float2 *X, float2 *Y,
               int ncols, float shift, cudaStream_t s);
 // Non-zero when a stencil's bounded wait gave up since the last reset.
