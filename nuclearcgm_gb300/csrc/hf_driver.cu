@@ -1633,11 +1633,19 @@ extern "C" int ncgm_densities(ncgm_ctx *ctx, const double *Phi, int ncols,
       return NCGM_ERR_ARG;
     }
     const size_t N = ctx->N, ns = ctx->ns;
-    double2 *dX = static_cast<double2 *>(ctx->buf(23, N * ncols * sizeof(double2)));
     double *d = static_cast<double *>(ctx->buf(24, 12 * ns * sizeof(double)));
-    if (!dX || !d) return NCGM_ERR_NOMEM;
-    NCGM_CUDA(cudaMemcpyAsync(dX, Phi, N * ncols * sizeof(double2),
-                              cudaMemcpyDefault, ctx->stream));
+    if (!d) return NCGM_ERR_NOMEM;
+    // columns on the device are read where they are, when the 16-byte loads
+    // allow it
+    const double2 *dX = reinterpret_cast<const double2 *>(Phi);
+    if (!isDevicePtr(Phi) || reinterpret_cast<uintptr_t>(Phi) % 16) {
+      double2 *b = static_cast<double2 *>(
+          ctx->buf(23, N * ncols * sizeof(double2)));
+      if (!b) return NCGM_ERR_NOMEM;
+      NCGM_CUDA(cudaMemcpyAsync(b, Phi, N * ncols * sizeof(double2),
+                                cudaMemcpyDefault, ctx->stream));
+      dX = b;
+    }
     densities(dX, N, ncols, ctx->n, ctx->h, d, d + ns, d + 2 * ns, d + 11 * ns,
               ctx->stream);
     NCGM_CUDA(cudaMemcpyAsync(rho, d, ns * sizeof(double), cudaMemcpyDefault,

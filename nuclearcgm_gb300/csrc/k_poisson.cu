@@ -22,6 +22,8 @@
 
 namespace ncgm {
 
+int smCount();
+
 namespace {
 
 __device__ __forceinline__ double trapW(size_t p, int n) {
@@ -67,70 +69,76 @@ __global__ void quadKernel(const double *rho, int n, double a, double h,
   }
 }
 
-// halo potential at halo index (a, b, c) of the (n+4)^3 box
+// halo potential at halo index (a, b, c) of the (n+4)^3 box: e^2 (Z + Y20 Q20
+// + 2 Y22 Q22) / r. With cos(theta) = z / r the harmonics are rational, Y20 ~
+// 3 z^2 / r^2 - 1 and cos(2 phi) sin^2(theta) = (x^2 - y^2) / r^2: the angles
+// themselves (acos, atan2 and their cosines) took 212 us of a 48^3 solve, this
+// form 62 (see haloKernel for the rest). The box lies outside the lattice, so
+// r > 0.
 __device__ __forceinline__ double haloV(int ia, int ib, int ic, double A,
                                         double h, double Z, double Q20,
                                         double Q22) {
   const double x = -A - 2 * h + ia * h, y = -A - 2 * h + ib * h,
                z = -A - 2 * h + ic * h;
-  double r = sqrt(x * x + y * y + z * z);
-  const double rr = r;
-  if (r < 1e-9) r = 1e-9;
-  const double theta = acos(z / rr);
-  const double phi = atan2(y, x);
-  const double y20 = sqrt(5.0 / (16.0 * M_PI)) * (3.0 * cos(theta) * cos(theta) - 1.0);
-  const double y22 = sqrt(15.0 / (32.0 * M_PI)) * cos(2 * phi) * sin(theta) * sin(theta);
-  double v = (kE2Poisson * Z) / r;
-  v += kE2Poisson * (y20 * Q20 + 2.0 * y22 * Q22) / r;
-  return v;
+  const double xx = x * x, yy = y * y, zz = z * z, r2 = xx + yy + zz;
+  const double i2 = 1.0 / r2;
+  const double y20 = sqrt(5.0 / (16.0 * M_PI)) * (3.0 * zz * i2 - 1.0);
+  const double y22 = sqrt(15.0 / (32.0 * M_PI)) * ((xx - yy) * i2);
+  return kE2Poisson * (Z + y20 * Q20 + 2.0 * y22 * Q22) / sqrt(r2);
 }
 
-__global__ void rhsKernel(const double *rho, int n, double A, double h,
-                          double Z, const double *q, double *rhs) {
+// out[t] = sum of the nblk partials t, one warp per term (fixed order)
+__global__ void sumTermsKernel(const double *partials, int nblk, double *out) {
+  const double *p = partials + (size_t)blockIdx.x * nblk;
+  double v = 0;
+  for (int b = threadIdx.x; b < nblk; b += 32) v += p[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (threadIdx.x == 0) out[blockIdx.x] = v;
+}
+
+// The halo layers next to the six faces: H[((2 f + layer) n + u) n + v] for
+// face f (first, second, third index at its low, then at its high end), layer
+// 0 adjacent to the lattice and 1 outside it, (u, v) the other two indices in
+// order. One value per thread: evaluated inside rhsKernel, where one lane of
+// a warp needs the value of a face and the others wait, they took 62 us of a
+// 48^3 solve, here 5.
+__global__ void haloKernel(int n, double A, double h, double Z,
+                           const double *q, double *H) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 12 * n * n) return;
+  const int v = e % n, u = e / n % n, layer = e / (n * n) & 1,
+            f = e / (2 * n * n);
+  const int x = f & 1 ? n + 2 + layer : 1 - layer;
+  const int ia = f < 2 ? x : u + 2, ib = f < 2 ? u + 2 : (f < 4 ? x : v + 2),
+            ic = f < 4 ? v + 2 : x;
+  H[e] = haloV(ia, ib, ic, A, h, Z, q[0], q[1]);
+}
+
+__global__ void rhsKernel(const double *rho, int n, double h,
+                          const double *__restrict__ H, double *rhs) {
   const size_t ns = (size_t)n * n * n;
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (e >= ns) return;
-  const double Q20 = q[0], Q22 = q[1];
-  const double hh = h * h;
+  const double near = (16.0 / 12.0) / (h * h), far = (1.0 / 12.0) / (h * h);
   const double eps0inv = kE2Poisson * 4 * M_PI;
   double v = -eps0inv * rho[e];
   // rhs index e = a n^2 + b n + c (the reference's face lambda)
-  const int a = (int)(e / ((size_t)n * n)), b = (int)((e / n) % n),
-            c = (int)(e % n);
-  auto H = [&](int ia, int ib, int ic) {
-    return haloV(ia, ib, ic, A, h, Z, Q20, Q22);
-  };
+  const int x[3] = {(int)(e / ((size_t)n * n)), (int)((e / n) % n),
+                    (int)(e % n)};
   // faces in the reference's order: first, second, third lambda index
-  if (a == 0) {
-    v -= (16.0 / 12.0) * H(1, b + 2, c + 2) / hh;
-    v += (1.0 / 12.0) * H(0, b + 2, c + 2) / hh;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int u = d == 0 ? x[1] : x[0], w = d == 2 ? x[1] : x[2];
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int dist = side ? n - 1 - x[d] : x[d];
+      const double *f = H + (size_t)(2 * (2 * d + side)) * n * n +
+                        (size_t)u * n + w;
+      if (dist == 0) v = fma(-near, f[0], fma(far, f[(size_t)n * n], v));
+      if (dist == 1) v = fma(far, f[0], v);
+    }
   }
-  if (a == 1) v += (1.0 / 12.0) * H(1, b + 2, c + 2) / hh;
-  if (a == n - 1) {
-    v -= (16.0 / 12.0) * H(n + 2, b + 2, c + 2) / hh;
-    v += (1.0 / 12.0) * H(n + 3, b + 2, c + 2) / hh;
-  }
-  if (a == n - 2) v += (1.0 / 12.0) * H(n + 2, b + 2, c + 2) / hh;
-  if (b == 0) {
-    v -= (16.0 / 12.0) * H(a + 2, 1, c + 2) / hh;
-    v += (1.0 / 12.0) * H(a + 2, 0, c + 2) / hh;
-  }
-  if (b == 1) v += (1.0 / 12.0) * H(a + 2, 1, c + 2) / hh;
-  if (b == n - 1) {
-    v -= (16.0 / 12.0) * H(a + 2, n + 2, c + 2) / hh;
-    v += (1.0 / 12.0) * H(a + 2, n + 3, c + 2) / hh;
-  }
-  if (b == n - 2) v += (1.0 / 12.0) * H(a + 2, n + 2, c + 2) / hh;
-  if (c == 0) {
-    v -= (16.0 / 12.0) * H(a + 2, b + 2, 1) / hh;
-    v += (1.0 / 12.0) * H(a + 2, b + 2, 0) / hh;
-  }
-  if (c == 1) v += (1.0 / 12.0) * H(a + 2, b + 2, 1) / hh;
-  if (c == n - 1) {
-    v -= (16.0 / 12.0) * H(a + 2, b + 2, n + 2) / hh;
-    v += (1.0 / 12.0) * H(a + 2, b + 2, n + 3) / hh;
-  }
-  if (c == n - 2) v += (1.0 / 12.0) * H(a + 2, b + 2, n + 2) / hh;
   rhs[e] = v;
 }
 
@@ -188,17 +196,67 @@ __global__ void cgInitKernel(const double *rhs, const double *y, double *r,
   }
 }
 
-// scalars: s[0] = rr, s[1] = bb, s[2] = pAp, s[3] = done
-__global__ void cgScalarInit(const double *partials, int nblk, double *s) {
-  if (threadIdx.x) return;
+// r = p = b + L U in one pass (b = -rhs), partials |r|^2 and |b|^2: negLapKernel
+// and cgInitKernel together, same arithmetic
+__global__ void __launch_bounds__(256)
+    residualKernel(const double *__restrict__ rhs,
+                   const double *__restrict__ x, double *__restrict__ r,
+                   double *__restrict__ p, int n, double h,
+                   double *partials) {
+  __shared__ double sh[256];
+  const size_t ns = (size_t)n * n * n;
+  const double hh = h * h;
+  const double c0 = (90.0 / 12.0) / hh, c1 = -(16.0 / 12.0) / hh,
+               c2 = (1.0 / 12.0) / hh;
   double rr = 0, bb = 0;
-  for (int b = 0; b < nblk; ++b) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < ns;
+       q += (size_t)gridDim.x * blockDim.x) {
+    const int pos[3] = {(int)(q % n), (int)((q / n) % n),
+                        (int)(q / ((size_t)n * n))};
+    double s = c0 * x[q];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const size_t st = a == 0 ? 1 : (a == 1 ? (size_t)n : (size_t)n * n);
+      const int i = pos[a];
+      const double m1 = i >= 1 ? x[q - st] : 0.0, m2 = i >= 2 ? x[q - 2 * st] : 0.0;
+      const double p1 = i + 1 < n ? x[q + st] : 0.0,
+                   p2 = i + 2 < n ? x[q + 2 * st] : 0.0;
+      s = fma(c2, p2, fma(c1, p1, fma(c2, m2, fma(c1, m1, s))));
+    }
+    const double b = -rhs[q], v = b - s;
+    r[q] = v;
+    p[q] = v;
+    rr += v * v;
+    bb += b * b;
+  }
+  double s0 = blockReduce(rr, sh), s1 = blockReduce(bb, sh);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = s0;
+    partials[gridDim.x + blockIdx.x] = s1;
+  }
+}
+
+// scalars: s[0] = rr, s[1] = bb, s[2] = pAp, s[3] = done
+// s[6] = the residual is below the tolerance (the next refinement leaves U as
+// it is), s[7] = refinements that ran (first: none yet)
+__global__ void cgScalarInit(const double *partials, int nblk, double tol2,
+                             int first, double *s) {
+  double rr = 0, bb = 0;
+  for (int b = threadIdx.x; b < nblk; b += 32) {
     rr += partials[b];
     bb += partials[nblk + b];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    rr += __shfl_xor_sync(0xffffffffu, rr, o);
+    bb += __shfl_xor_sync(0xffffffffu, bb, o);
+  }
+  if (threadIdx.x) return;
   s[0] = rr;
   s[1] = bb;
   s[3] = (bb == 0.0) ? 1.0 : 0.0;
+  s[7] = first ? 0.0 : s[7] + (s[6] == 0.0 ? 1.0 : 0.0);
+  s[6] = (bb == 0.0 || rr <= tol2 * bb) ? 1.0 : 0.0;
 }
 
 // alpha = rr / pAp; x += alpha p; r -= alpha Ap; partial |r|^2
@@ -267,33 +325,70 @@ __global__ void cgCommit(double *s) {
 // = eigenvector j, column-major, n x n). scaleD: divide by the eigenvalue sum
 // (d_i + d_j + d_k) / h^2 (last forward pass); accum: out[p] += result (last
 // inverse pass, into the potential) instead of out[p] = result.
+// done: a non-zero value leaves the pass out (the residual was already below
+// the tolerance).
+// Bound by the FP64 pipe (n^4 FMAs a pass: 9 us for n = 48). A block takes
+// four or eight lines of the axis into shared memory and a thread owns one
+// index a of four of them, so a weight is read once for four independent FMA
+// chains. One output per thread with its one chain of n dependent FMAs on 120
+// blocks took 32 us.
+constexpr int kLines = 4; // lines per thread
 __global__ void axisTransformKernel(const double *__restrict__ in,
                                     double *__restrict__ out,
                                     const double *__restrict__ Wd, int n,
-                                    int axis, int inverse, int scaleD,
-                                    double hh, int accum) {
-  extern __shared__ double cs[]; // cs[t n + a] = C[a][t], then d (n)
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int t = e / n, a = e % n;
-    cs[e] = inverse ? Wd[(size_t)t * n + a] : Wd[(size_t)a * n + t];
-  }
-  for (int e = threadIdx.x; e < n; e += blockDim.x) cs[n * n + e] = Wd[n * n + e];
-  __syncthreads();
-  const size_t ns = (size_t)n * n * n;
+                                    int lines, int axis, int inverse,
+                                    int scaleD, double hh, int accum,
+                                    const double *done) {
+  // C[a][t] at t (n + 1) + a (the odd pitch keeps the transposed copy free of
+  // bank conflicts), d (n), the lines (line l, index t at t lines + l)
+  extern __shared__ double cs[];
+  if (*done != 0.0) return;
+  const int pitch = n + 1;
+  double *d = cs + n * pitch, *ln = d + n;
+  const int all = n * n, l0 = blockIdx.x * lines;
   const size_t stride = axis == 0 ? 1 : (axis == 1 ? (size_t)n : (size_t)n * n);
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < ns;
-       p += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(p % n), j = (int)((p / n) % n),
-              k = (int)(p / ((size_t)n * n));
-    const int a = axis == 0 ? i : (axis == 1 ? j : k);
-    const double *base = in + (p - (size_t)a * stride);
-    double v = 0.0;
-    for (int t = 0; t < n; ++t) v = fma(cs[t * n + a], base[(size_t)t * stride], v);
-    if (scaleD) v /= (cs[n * n + i] + cs[n * n + j] + cs[n * n + k]) / hh;
+  // first point of line l
+  auto base = [&](int l) -> size_t {
+    return axis == 0 ? (size_t)l * n
+                     : (axis == 1 ? (size_t)(l / n) * n * n + l % n : (size_t)l);
+  };
+  for (int e = threadIdx.x; e < n * lines; e += blockDim.x) {
+    // neighbouring threads read neighbouring points
+    const int l = axis == 0 ? e / n : e % lines,
+              t = axis == 0 ? e % n : e / lines;
+    ln[t * lines + l] =
+        l0 + l < all ? in[base(l0 + l) + (size_t)t * stride] : 0.0;
+  }
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    // W[u + n v]: C[u][v] of the inverse, C[v][u] of the forward transform
+    const int u = e % n, v = e / n;
+    cs[inverse ? v * pitch + u : u * pitch + v] = Wd[e];
+  }
+  for (int e = threadIdx.x; e < n; e += blockDim.x) d[e] = Wd[n * n + e];
+  __syncthreads();
+  if ((int)threadIdx.x >= n * (lines / kLines)) return;
+  const int a = threadIdx.x % n, g = (int)threadIdx.x / n * kLines;
+  double v[kLines];
+#pragma unroll
+  for (int q = 0; q < kLines; ++q) v[q] = 0.0;
+#pragma unroll 4
+  for (int t = 0; t < n; ++t) {
+    const double c = cs[t * pitch + a];
+#pragma unroll
+    for (int q = 0; q < kLines; ++q)
+      v[q] = fma(c, ln[t * lines + g + q], v[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < kLines; ++q) {
+    const int l = l0 + g + q;
+    if (l >= all) continue;
+    const size_t p = base(l) + (size_t)a * stride;
+    if (scaleD) // axis 2: l = i + n j, a = k
+      v[q] = v[q] * hh / (d[l % n] + d[l / n] + d[a]);
     if (accum)
-      out[p] += v;
+      out[p] += v[q];
     else
-      out[p] = v;
+      out[p] = v[q];
   }
 }
 
@@ -319,9 +414,10 @@ __global__ void exchangeKernel(const double *rhoP, const double *Ud,
                                double *UC, size_t ns) {
   size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (e >= ns) return;
-  double v = 0.0;
-  v -= kE2Poisson * pow(3.0 / M_PI, 1.0 / 3.0) * pow(rhoP[e], 1.0 / 3.0);
-  UC[e] = Ud[e] + v;
+  // a negative density gives a NaN, as the power 1/3 does
+  const double r = rhoP[e];
+  const double c = r < 0.0 ? nan("") : cbrt(r);
+  UC[e] = Ud[e] - kE2Poisson * cbrt(3.0 / M_PI) * c;
 }
 
 } // namespace
@@ -352,7 +448,7 @@ bool axisTransformReady() {
     if (d == dev) return true;
   if (cudaFuncSetAttribute(axisTransformKernel,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (80 * 80 + 80) * (int)sizeof(double)) !=
+                           (80 * 81 + 80 + 80 * 2 * kLines) * (int)sizeof(double)) !=
       cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -408,59 +504,65 @@ int poissonSolve(const PoissonArgs &P, cudaStream_t s, int *iterations) {
   double *rhs = P.work + 16 + 4 * nblk;
   double *r = rhs + ns, *p = r + ns, *Ap = p + ns;
   quadKernel<<<nblk, 256, 0, s>>>(P.rhoP, n, P.a, P.h, part);
-  // reduce Q20, Q22 (2 values)
-  {
-    std::vector<double> hp(2 * nblk);
-    cudaMemcpyAsync(hp.data(), part, sizeof(double) * 2 * nblk,
-                    cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return NCGM_ERR_CUDA;
-    double qq[2] = {0, 0};
-    for (int b = 0; b < nblk; ++b) {
-      qq[0] += hp[b];
-      qq[1] += hp[nblk + b];
-    }
-    cudaMemcpyAsync(q, qq, sizeof(double) * 2, cudaMemcpyHostToDevice, s);
-  }
-  rhsKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(P.rhoP, n, P.a, P.h,
-                                                          P.Z, q, rhs);
+  sumTermsKernel<<<2, 32, 0, s>>>(part, nblk, q); // Q20, Q22
+  // the halo values lie in r, p, Ap (free until the first residual; the
+  // work array's slack covers 12 n^2 > 3 n^3 at n < 4)
+  haloKernel<<<(unsigned)((12 * n * n + 127) / 128), 128, 0, s>>>(
+      n, P.a, P.h, P.Z, q, r);
+  rhsKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(P.rhoP, n, P.h, r,
+                                                          rhs);
   if (!P.warm) cudaMemsetAsync(P.U, 0, ns * sizeof(double), s);
-  negLapKernel<<<nblk, 256, 0, s>>>(P.U, Ap, n, P.h, nullptr);
-  cgInitKernel<<<nblk, 256, 0, s>>>(rhs, Ap, r, p, ns, part);
-  cgScalarInit<<<1, 32, 0, s>>>(part, nblk, sc);
   const double tol2 = P.tol * P.tol;
+  // residual of U, its norms and the refinement's done flag (two partials per
+  // block: they fill `part` and `part2`)
+  auto residual = [&](bool first) {
+    residualKernel<<<2 * nblk, 256, 0, s>>>(rhs, P.U, r, p, n, P.h, part);
+    cgScalarInit<<<1, 32, 0, s>>>(part, 2 * nblk, tol2, first ? 1 : 0, sc);
+  };
+  residual(true);
   int it = 0;
   const int maxit = std::max(100, (int)std::min<size_t>(4 * ns, 20000));
   // fast solver: refinement steps with the separable inverse (p and Ap serve
-  // as the transform's temporaries); NCGM_POISSON_FAST=0 keeps plain CG
+  // as the transform's temporaries); NCGM_POISSON_FAST=0 keeps plain CG. A
+  // step whose residual is already below the tolerance is skipped on the
+  // device, so the host reads the norms once per step, after it.
   const char *fenv = std::getenv("NCGM_POISSON_FAST");
   const double *Wd = (fenv && fenv[0] == '0') ? nullptr : poissonEigen(n, s);
   bool solved = false;
   if (Wd && axisTransformReady()) {
-    const size_t smem = ((size_t)n * n + n) * sizeof(double);
-    const double hh = P.h * P.h;
+    // eight lines per block when that still gives every SM one
+    const int lines = n * n >= 2 * kLines * smCount() ? 2 * kLines : kLines;
+    const size_t smem =
+        ((size_t)n * (n + 1) + n + (size_t)n * lines) * sizeof(double);
+    const unsigned gb = (unsigned)((n * n + lines - 1) / lines);
+    const int thr = (n * (lines / kLines) + 31) / 32 * 32;
+    auto axisPass = [&](const double *in, double *out, int axis, int inverse,
+                        int scaleD, int accum) {
+      axisTransformKernel<<<gb, thr, smem, s>>>(in, out, Wd, n, lines, axis,
+                                                inverse, scaleD, P.h * P.h,
+                                                accum, sc + 6);
+    };
     for (int ref = 0; ref < 4; ++ref) {
-      double hs2[2];
-      cudaMemcpyAsync(hs2, sc, sizeof(double) * 2, cudaMemcpyDeviceToHost, s);
-      if (cudaStreamSynchronize(s) != cudaSuccess) return NCGM_ERR_CUDA;
-      if (!std::isfinite(hs2[0])) return NCGM_ERR_NAN;
-      if (hs2[1] == 0.0 || hs2[0] <= tol2 * hs2[1]) {
-        solved = true;
-        break;
-      }
-      axisTransformKernel<<<nblk, 256, smem, s>>>(r, p, Wd, n, 0, 0, 0, hh, 0);
-      axisTransformKernel<<<nblk, 256, smem, s>>>(p, Ap, Wd, n, 1, 0, 0, hh, 0);
-      axisTransformKernel<<<nblk, 256, smem, s>>>(Ap, p, Wd, n, 2, 0, 1, hh, 0);
-      axisTransformKernel<<<nblk, 256, smem, s>>>(p, Ap, Wd, n, 0, 1, 0, hh, 0);
-      axisTransformKernel<<<nblk, 256, smem, s>>>(Ap, p, Wd, n, 1, 1, 0, hh, 0);
-      axisTransformKernel<<<nblk, 256, smem, s>>>(p, P.U, Wd, n, 2, 1, 0, hh, 1);
+      axisPass(r, p, 0, 0, 0, 0);
+      axisPass(p, Ap, 1, 0, 0, 0);
+      axisPass(Ap, p, 2, 0, 1, 0);
+      axisPass(p, Ap, 0, 1, 0, 0);
+      axisPass(Ap, p, 1, 1, 0, 0);
+      axisPass(p, P.U, 2, 1, 0, 1);
       // a failed launch leaves U as it was (all six passes share one
       // configuration): rebuild the residual from U and finish with CG
       const bool launched = cudaGetLastError() == cudaSuccess;
-      negLapKernel<<<nblk, 256, 0, s>>>(P.U, Ap, n, P.h, nullptr);
-      cgInitKernel<<<nblk, 256, 0, s>>>(rhs, Ap, r, p, ns, part);
-      cgScalarInit<<<1, 32, 0, s>>>(part, nblk, sc);
+      residual(false);
+      double h[8];
+      cudaMemcpyAsync(h, sc, sizeof(h), cudaMemcpyDeviceToHost, s);
+      if (cudaStreamSynchronize(s) != cudaSuccess) return NCGM_ERR_CUDA;
+      if (!std::isfinite(h[0])) return NCGM_ERR_NAN;
       if (!launched) break;
-      ++it;
+      it = (int)h[7];
+      if (h[6] != 0.0) {
+        solved = true;
+        break;
+      }
     }
   }
 
@@ -594,12 +696,14 @@ int poissonSolveNoAlloc(const PoissonArgs &P, cudaStream_t s,
   if (cudaMemcpyAsync(q, qq, sizeof(qq), cudaMemcpyHostToDevice, s) !=
       cudaSuccess)
     return NCGM_ERR_CUDA;
-  rhsKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(P.rhoP, n, P.a, P.h,
-                                                          P.Z, q, rhs);
+  haloKernel<<<(unsigned)((12 * n * n + 127) / 128), 128, 0, s>>>(
+      n, P.a, P.h, P.Z, q, r);
+  rhsKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(P.rhoP, n, P.h, r,
+                                                          rhs);
   negLapKernel<<<nblk, 256, 0, s>>>(P.U, Ap, n, P.h, nullptr);
   cgInitKernel<<<nblk, 256, 0, s>>>(rhs, Ap, r, p, ns, part);
-  cgScalarInit<<<1, 32, 0, s>>>(part, nblk, sc);
   const double tol2 = P.tol * P.tol;
+  cgScalarInit<<<1, 32, 0, s>>>(part, nblk, tol2, 1, sc);
   int it = 0;
   const int maxit = std::max(100, (int)std::min<size_t>(4 * ns, 20000));
   double hs[8];
