@@ -119,12 +119,6 @@ __global__ void colStatsFinish(const double *part, int nb, double *res2,
   xax[c] = b;
 }
 
-__global__ void extractDiag(const double *coef, size_t ns, double *d) {
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < ns;
-       p += (size_t)gridDim.x * blockDim.x)
-    d[p] = coef[8 * p];
-}
-
 struct Carve {
   char *p;
   size_t off = 0;
@@ -200,15 +194,6 @@ static int cholQR2(ncgm_ctx *ctx, const double2 *V, int k, double2 *Q,
   }
   if (keptOrig) *keptOrig = orig;
   return cols;
-}
-
-double *jacobiDiagonal(ncgm_ctx *ctx, int species, cudaStream_t s) {
-  double *d = static_cast<double *>(
-      ctx->buf(12 + species, ctx->ns * sizeof(double)));
-  if (!d) return nullptr;
-  extractDiag<<<(unsigned)std::min<size_t>(1024, (ctx->ns + 255) / 256), 256,
-                0, s>>>(ctx->sp[species].coef64, ctx->ns, d);
-  return d;
 }
 
 int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
@@ -300,9 +285,9 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
     applyH64(ctx, species, X, Y, cols, sh, s);
   };
   NCGM_CUDA(cudaMemsetAsync(dLive, 0, sizeof(int), s));
-  const double *dDiag = jacobiDiagonal(ctx, species, s);
-  if (!dDiag) return NCGM_ERR_NOMEM;
-  if (fp32) inverseDiagonal32(dDiag, prm.shift, ctx->ns, dInv32, s);
+  // the FP32 steps precondition with the first shift throughout
+  if (fp32 && !inverseJacobiDiagonal(ctx, species, prm.shift, dInv32, s))
+    return NCGM_ERR_NOMEM;
 
   // X = X_init.leftCols(nev), orthonormalised (solver.cpp:669,677)
   NCGM_CUDA(cudaMemcpyAsync(V, Xinit, N * (size_t)nev * sizeof(double2),
@@ -375,6 +360,9 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
     double2 *Wd = V + o * N;
     if (nact > 0) {
       std::vector<double> ls(nact);
+      const double *dInv =
+          inverseJacobiDiagonal(ctx, species, shift, nullptr, s);
+      if (!dInv) return NCGM_ERR_NOMEM;
       for (int k = 0; k < nact; ++k) ls[k] = Lambda[k] + shift;
       NCGM_CUDA(cudaMemcpyAsync(dLs, ls.data(), sizeof(double) * nact,
                                 cudaMemcpyHostToDevice, s));
@@ -408,7 +396,7 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
         pl.D0 = pD0;
         pl.useNet = dUse;
         pl.lamShift = dLs;
-        pl.coef = dDiag;
+        pl.inv = dInv;
         pl.arrive = dArrive;
         pl.shift = shift;
         pl.tol = prm.cg_tol;
@@ -436,7 +424,7 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
         pl.P = pP;
         pl.AP = pAP;
         pl.lamShift = dLs;
-        pl.coef = dDiag;
+        pl.inv = dInv;
         pl.arrive = dArrive;
         pl.shift = shift;
         pl.tol = prm.cg_tol;
@@ -476,7 +464,7 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
         // lose the digits of d that FP32 rounding already made noisy)
         pl.onlyCorrection = true;
         pl.lamShift = dLs;
-        pl.coef = dDiag;
+        pl.inv = dInv;
         pl.invd = dInv32;
         pl.arrive = dArrive;
         pl.shift = shift;

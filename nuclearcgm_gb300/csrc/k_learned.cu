@@ -1060,9 +1060,9 @@ int ncgm_lp_collect(ncgm_lp *lp, ncgm_ctx *ctx, int species, const double *X,
   pl.P = Pp;
   pl.AP = AP;
   pl.lamShift = dLs;
-  pl.coef = jacobiDiagonal(ctx, species, s);
+  pl.inv = inverseJacobiDiagonal(ctx, species, shift, nullptr, s);
   pl.arrive = reinterpret_cast<unsigned *>(live + 2);
-  if (!pl.coef) return NCGM_ERR_NOMEM;
+  if (!pl.inv) return NCGM_ERR_NOMEM;
   pl.shift = shift;
   pl.tol = cg_tol;
   pl.maxSteps = cg_steps;

@@ -27,23 +27,48 @@ template <class T> struct C2;
 template <> struct C2<double> { using type = double2; };
 template <> struct C2<float> { using type = float2; };
 
-__device__ double blockSum(double v, double *sh) {
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+// Sums of K values over the block, valid in thread 0, by the tree v_t += v_{t+s}
+// (s = 128, 64, ..., 1): three levels through shared memory with one barrier
+// each (a level writes the upper half that it adds, so levels do not share
+// addresses), the last five inside a warp. sh: K x kThreads.
+template <int K> __device__ void blockSums(double (&v)[K], double *sh) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int s = kThreads / 2; s >= 32; s >>= 1) {
+    if (t >= s && t < 2 * s)
+#pragma unroll
+      for (int k = 0; k < K; ++k) sh[k * kThreads + t] = v[k];
     __syncthreads();
+    if (t < s)
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] += sh[k * kThreads + t + s];
   }
-  double r = sh[0];
-  __syncthreads();
-  return r;
+  if (t < 32)
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        v[k] += __shfl_down_sync(0xffffffffu, v[k], s);
 }
 
-// inverse Jacobi diagonal: diag = c0 + shift, c0 = U + UC + 7.5 f / h^2
-// (the diagonal of H, one double per lattice point)
-__device__ inline double invDiag(const double *c0, size_t p, double shift) {
-  double d = c0[p] + shift;
-  return d != 0.0 ? 1.0 / d : 1.0;
+// Sums of the nblk (<= 128) block partials of a column, pp[b] and
+// pp[nblk + b], in block order, valid in thread 0. All partials come in one
+// round trip to L2; the serial sum then reads shared memory (read one after
+// the other from L2 they took 5 of the FP64 dot product's 17 us at 30^3 x 8
+// columns).
+__device__ double2 orderedSums(const double *pp, int nblk, double *sh) {
+  __syncthreads();
+  for (int b = threadIdx.x; b < 2 * nblk; b += kThreads) sh[b] = __ldcg(pp + b);
+  __syncthreads();
+  double2 r = make_double2(0.0, 0.0);
+  if (threadIdx.x == 0) {
+#pragma unroll 4
+    for (int b = 0; b < nblk; ++b) {
+      r.x += sh[b];
+      r.y += sh[nblk + b];
+    }
+  }
+  return r;
 }
 
 // Last-block test of a per-column reduction: every block has written its
@@ -71,9 +96,9 @@ __global__ void pcgInitKernel(const typename C2<T>::type *X, size_t ldx,
                               typename C2<T>::type *Wv,
                               typename C2<T>::type *R, typename C2<T>::type *Z,
                               typename C2<T>::type *P, size_t N,
-                              const double *lamShift, const double *coef,
-                              double shift, double *partials, int nblk) {
-  __shared__ double sh[kThreads];
+                              const double *lamShift, const double *inv,
+                              double *partials, int nblk) {
+  __shared__ double sh[3 * kThreads];
   const int col = blockIdx.y;
   const double ls = lamShift[col];
   double bb = 0, rr = 0, rz = 0;
@@ -84,7 +109,7 @@ __global__ void pcgInitKernel(const typename C2<T>::type *X, size_t ldx,
     auto t = Tx[o];
     double bx = (double)x.x * ls, by = (double)x.y * ls;
     double rx = bx - (double)t.x, ry = by - (double)t.y;
-    double m = invDiag(coef, i / 2, shift);
+    double m = inv[i / 2];
     double zx = m * rx, zy = m * ry;
     bb += bx * bx + by * by;
     rr += rx * rx + ry * ry;
@@ -94,12 +119,13 @@ __global__ void pcgInitKernel(const typename C2<T>::type *X, size_t ldx,
     Z[o] = {(T)zx, (T)zy};
     P[o] = {(T)zx, (T)zy};
   }
-  double s0 = blockSum(bb, sh), s1 = blockSum(rr, sh), s2 = blockSum(rz, sh);
+  double sum[3] = {bb, rr, rz};
+  blockSums(sum, sh);
   if (threadIdx.x == 0) {
     double *pp = partials + (size_t)col * nblk * 3;
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
-    pp[2 * nblk + blockIdx.x] = s2;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
+    pp[2 * nblk + blockIdx.x] = sum[2];
   }
 }
 
@@ -114,9 +140,9 @@ __global__ void pcgInitCorrKernel(const double2 *X64, const double2 *AX64,
                                   typename C2<T>::type *R,
                                   typename C2<T>::type *Z,
                                   typename C2<T>::type *P, size_t N,
-                                  const double *lamShift, const double *coef,
+                                  const double *lamShift, const double *inv,
                                   double shift, double *partials, int nblk) {
-  __shared__ double sh[kThreads];
+  __shared__ double sh[3 * kThreads];
   const int col = blockIdx.y;
   const double ls = lamShift[col], lam = ls - shift;
   double bb = 0, rr = 0, rz = 0;
@@ -126,7 +152,7 @@ __global__ void pcgInitCorrKernel(const double2 *X64, const double2 *AX64,
     double2 x = X64[o], ax = AX64[o];
     double bx = x.x * ls, by = x.y * ls;
     double rx = x.x * lam - ax.x, ry = x.y * lam - ax.y;
-    double m = invDiag(coef, i / 2, shift);
+    double m = inv[i / 2];
     double zx = m * rx, zy = m * ry;
     bb += bx * bx + by * by;
     rr += rx * rx + ry * ry;
@@ -136,12 +162,13 @@ __global__ void pcgInitCorrKernel(const double2 *X64, const double2 *AX64,
     Z[o] = {(T)zx, (T)zy};
     P[o] = {(T)zx, (T)zy};
   }
-  double s0 = blockSum(bb, sh), s1 = blockSum(rr, sh), s2 = blockSum(rz, sh);
+  double sum[3] = {bb, rr, rz};
+  blockSums(sum, sh);
   if (threadIdx.x == 0) {
     double *pp = partials + (size_t)col * nblk * 3;
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
-    pp[2 * nblk + blockIdx.x] = s2;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
+    pp[2 * nblk + blockIdx.x] = sum[2];
   }
 }
 
@@ -153,7 +180,7 @@ __global__ void pcgNetNormKernel(const double2 *X64, const double2 *AX64,
                                  const typename C2<T>::type *Td, size_t N,
                                  const double *lamShift, double shift,
                                  double *partials, int nblk) {
-  __shared__ double sh[kThreads];
+  __shared__ double sh[2 * kThreads];
   const int col = blockIdx.y;
   const double lam = lamShift[col] - shift;
   double a = 0, b = 0;
@@ -167,11 +194,12 @@ __global__ void pcgNetNormKernel(const double2 *X64, const double2 *AX64,
     a += (double)d.x * rx + (double)d.y * ry;
     b += (double)d.x * t.x + (double)d.y * t.y;
   }
-  double s0 = blockSum(a, sh), s1 = blockSum(b, sh);
+  double sum[2] = {a, b};
+  blockSums(sum, sh);
   if (threadIdx.x == 0) {
     double *pp = partials + (size_t)col * nblk * 2;
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
   }
 }
 
@@ -189,10 +217,10 @@ __global__ void pcgInitNetKernel(const double2 *X64, const double2 *AX64,
                                  typename C2<T>::type *R,
                                  typename C2<T>::type *Z,
                                  typename C2<T>::type *P, size_t N,
-                                 const double *lamShift, const double *coef,
+                                 const double *lamShift, const double *inv,
                                  double shift, const double *normPart,
                                  double *partials, int nblk, int *useNet) {
-  __shared__ double sh[kThreads];
+  __shared__ double sh[3 * kThreads];
   __shared__ double alpha;
   const int col = blockIdx.y;
   if (threadIdx.x == 0) {
@@ -219,7 +247,7 @@ __global__ void pcgInitNetKernel(const double2 *X64, const double2 *AX64,
     auto t = Td[o];
     rx -= al * (double)t.x;
     ry -= al * (double)t.y;
-    double m = invDiag(coef, i / 2, shift);
+    double m = inv[i / 2];
     double zx = m * rx, zy = m * ry;
     bb += bx * bx + by * by;
     rr += rx * rx + ry * ry;
@@ -229,12 +257,13 @@ __global__ void pcgInitNetKernel(const double2 *X64, const double2 *AX64,
     Z[o] = {(T)zx, (T)zy};
     P[o] = {(T)zx, (T)zy};
   }
-  double s0 = blockSum(bb, sh), s1 = blockSum(rr, sh), s2 = blockSum(rz, sh);
+  double sum[3] = {bb, rr, rz};
+  blockSums(sum, sh);
   if (threadIdx.x == 0) {
     double *pp = partials + (size_t)col * nblk * 3;
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
-    pp[2 * nblk + blockIdx.x] = s2;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
+    pp[2 * nblk + blockIdx.x] = sum[2];
   }
 }
 
@@ -285,7 +314,7 @@ __global__ void pcgDotKernel(const typename C2<T>::type *P,
                              const typename C2<T>::type *AP, size_t N,
                              PcgCol *st, double *partials, int nblk,
                              unsigned *arrive) {
-  __shared__ double sh[kThreads];
+  __shared__ double sh[2 * kThreads];
   const int col = blockIdx.y;
   if (st[col].done) return;
   double re = 0, im = 0;
@@ -312,11 +341,12 @@ __global__ void pcgDotKernel(const typename C2<T>::type *P,
       im += (double)p.x * a.y - (double)p.y * a.x;
     }
   }
-  double s0 = blockSum(re, sh), s1 = blockSum(im, sh);
+  double sum[2] = {re, im};
+  blockSums(sum, sh);
   double *pp = partials + (size_t)col * nblk * 3;
   if (threadIdx.x == 0) {
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
   }
   // the last block sums the partials in block order: alpha = absNew / p^H Ap
   // the last block sums the partials. FP32 plans: with all its threads (one
@@ -330,13 +360,14 @@ __global__ void pcgDotKernel(const typename C2<T>::type *P,
         r += __ldcg(pp + b);
         m += __ldcg(pp + nblk + b);
       }
-      r = blockSum(r, sh);
-      m = blockSum(m, sh);
-    } else if (threadIdx.x == 0) {
-      for (int b = 0; b < nblk; ++b) {
-        r += ((volatile double *)pp)[b];
-        m += ((volatile double *)pp)[nblk + b];
-      }
+      double t[2] = {r, m};
+      blockSums(t, sh);
+      r = t[0];
+      m = t[1];
+    } else {
+      const double2 t = orderedSums(pp, nblk, sh);
+      r = t.x;
+      m = t.y;
     }
     if (threadIdx.x == 0) {
       const double den = r * r + m * m;
@@ -356,11 +387,11 @@ __global__ void pcgUpdateKernel(typename C2<T>::type *Wv,
                                 typename C2<T>::type *Z,
                                 const typename C2<T>::type *P,
                                 const typename C2<T>::type *AP, size_t N,
-                                PcgCol *st, const double *diag, double shift,
+                                PcgCol *st, const double *inv,
                                 const float *invd, double *partials2,
                                 int nblk, unsigned *arrive, int *live,
                                 int *ndone) {
-  __shared__ double sh[kThreads];
+  __shared__ double sh[2 * kThreads];
   const int col = blockIdx.y;
   if (st[col].done) return;
   const double alr = st[col].alphaR, ali = st[col].alphaI;
@@ -405,7 +436,7 @@ __global__ void pcgUpdateKernel(typename C2<T>::type *Wv,
       double wy = (double)w.y + (alr * py + ali * px);
       double rx = (double)r.x - (alr * ax - ali * ay);
       double ry = (double)r.y - (alr * ay + ali * ax);
-      double m = invDiag(diag, i / 2, shift);
+      double m = inv[i / 2];
       double zx = m * rx, zy = m * ry;
       Wv[o] = {(T)wx, (T)wy};
       R[o] = {(T)rx, (T)ry};
@@ -414,11 +445,12 @@ __global__ void pcgUpdateKernel(typename C2<T>::type *Wv,
       rz += rx * zx + ry * zy;
     }
   }
-  double s0 = blockSum(rr, sh), s1 = blockSum(rz, sh);
+  double sum[2] = {rr, rz};
+  blockSums(sum, sh);
   double *pp = partials2 + (size_t)col * nblk * 2;
   if (threadIdx.x == 0) {
-    pp[blockIdx.x] = s0;
-    pp[nblk + blockIdx.x] = s1;
+    pp[blockIdx.x] = sum[0];
+    pp[nblk + blockIdx.x] = sum[1];
   }
   if (lastArrival(&arrive[col], nblk)) {
     double tr = 0, tz = 0;
@@ -427,13 +459,14 @@ __global__ void pcgUpdateKernel(typename C2<T>::type *Wv,
         tr += __ldcg(pp + b);
         tz += __ldcg(pp + nblk + b);
       }
-      tr = blockSum(tr, sh);
-      tz = blockSum(tz, sh);
-    } else if (threadIdx.x == 0) {
-      for (int b = 0; b < nblk; ++b) {
-        tr += ((volatile double *)pp)[b];
-        tz += ((volatile double *)pp)[nblk + b];
-      }
+      double t[2] = {tr, tz};
+      blockSums(t, sh);
+      tr = t[0];
+      tz = t[1];
+    } else {
+      const double2 t = orderedSums(pp, nblk, sh);
+      tr = t.x;
+      tz = t.y;
     }
     if (threadIdx.x != 0) return;
     PcgCol c = st[col];
@@ -448,27 +481,6 @@ __global__ void pcgUpdateKernel(typename C2<T>::type *Wv,
       atomicAdd(live, 1);
     }
     st[col] = c;
-  }
-}
-
-template <class T>
-__global__ void pcgPKernel(typename C2<T>::type *P,
-                           const typename C2<T>::type *Z, size_t N,
-                           const PcgCol *st) {
-  const int col = blockIdx.y;
-  if (st[col].done) return;
-  const double b = st[col].beta;
-  const float b32 = (float)b;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
-       i += (size_t)gridDim.x * blockDim.x) {
-    size_t o = (size_t)col * N + i;
-    auto z = Z[o];
-    auto p = P[o];
-    if (std::is_same<T, float>::value)
-      P[o] = {(T)((float)z.x + b32 * (float)p.x),
-              (T)((float)z.y + b32 * (float)p.y)};
-    else
-      P[o] = {(T)((double)z.x + b * p.x), (T)((double)z.y + b * p.y)};
   }
 }
 
@@ -542,8 +554,7 @@ void exitPollGive(ExitPoll *p, cudaStream_t s) {
 namespace {
 // the count of finished columns into the next host slot (one thread, after
 // a step's kernels): the host reads it without a copy or an event
-__global__ void pcgMarkKernel(const int *ndone, int *hostSlots,
-                              int *counter) {
+__device__ void markDone(const int *ndone, int *hostSlots, int *counter) {
   const int k = *counter;
   *counter = k + 1;
   if (k < kPollSlots) {
@@ -551,18 +562,61 @@ __global__ void pcgMarkKernel(const int *ndone, int *hostSlots,
     __threadfence_system();
   }
 }
+__global__ void pcgMarkKernel(const int *ndone, int *hostSlots,
+                              int *counter) {
+  markDone(ndone, hostSlots, counter);
+}
 
-__global__ void invDiag32Kernel(const double *c0, double shift, size_t ns,
-                                float *inv) {
+// p = z + beta p; one thread also hands the count of finished columns to the
+// host
+template <class T>
+__global__ void pcgPKernel(typename C2<T>::type *P,
+                           const typename C2<T>::type *Z, size_t N,
+                           const PcgCol *st, const int *ndone, int *hostSlots,
+                           int *counter) {
+  const int col = blockIdx.y;
+  // the columns that finished in this step are counted by now
+  if (counter && blockIdx.x == 0 && col == 0 && threadIdx.x == 0)
+    markDone(ndone, hostSlots, counter);
+  if (st[col].done) return;
+  const double b = st[col].beta;
+  const float b32 = (float)b;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N;
+       i += (size_t)gridDim.x * blockDim.x) {
+    size_t o = (size_t)col * N + i;
+    auto z = Z[o];
+    auto p = P[o];
+    if (std::is_same<T, float>::value)
+      P[o] = {(T)((float)z.x + b32 * (float)p.x),
+              (T)((float)z.y + b32 * (float)p.y)};
+    else
+      P[o] = {(T)((double)z.x + b * p.x), (T)((double)z.y + b * p.y)};
+  }
+}
+
+// Inverse Jacobi diagonal, tabulated once per solve: an FP64 division costs
+// about ten operations of a pipe that retires two a clock per SM, and the step
+// kernels are bound by it (pcgUpdateKernel, 30^3 x 8 columns: 20.8 -> 16.2 us). coef: the species' table, whose first entry of a
+// point is c0.
+__global__ void invDiagKernel(const double *coef, double shift, size_t ns,
+                              double *inv, float *inv32) {
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (p < ns) inv[p] = (float)invDiag(c0, p, shift);
+  if (p >= ns) return;
+  const double d = coef[8 * p] + shift;
+  const double v = d != 0.0 ? 1.0 / d : 1.0;
+  inv[p] = v;
+  if (inv32) inv32[p] = (float)v;
 }
 } // namespace
 
-void inverseDiagonal32(const double *c0, double shift, size_t ns, float *inv,
-                       cudaStream_t s) {
-  invDiag32Kernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(c0, shift, ns,
-                                                               inv);
+double *inverseJacobiDiagonal(ncgm_ctx *ctx, int species, double shift,
+                              float *inv32, cudaStream_t s) {
+  double *inv = static_cast<double *>(
+      ctx->buf(12 + species, ctx->ns * sizeof(double)));
+  if (!inv) return nullptr;
+  invDiagKernel<<<(unsigned)((ctx->ns + 255) / 256), 256, 0, s>>>(
+      ctx->sp[species].coef64, shift, ctx->ns, inv, inv32);
+  return inv;
 }
 
 int pcgBlocks(size_t N) {
@@ -588,13 +642,13 @@ void pcgRun(const PcgPlan<T> &pl, cudaStream_t s) {
         pl.X64, pl.AX64, reinterpret_cast<const V *>(pl.D0),
         reinterpret_cast<const V *>(pl.AP), reinterpret_cast<V *>(pl.W),
         reinterpret_cast<V *>(pl.R), reinterpret_cast<V *>(pl.Z),
-        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.coef, pl.shift,
+        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.inv, pl.shift,
         pl.partials2, pl.partials, nblk, pl.useNet);
   } else if (pl.AX64) {
     pcgInitCorrKernel<T><<<grid, kThreads, 0, s>>>(
         pl.X64, pl.AX64, reinterpret_cast<V *>(pl.W),
         reinterpret_cast<V *>(pl.R), reinterpret_cast<V *>(pl.Z),
-        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.coef, pl.shift,
+        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.inv, pl.shift,
         pl.partials, nblk);
   } else {
     // T = (A + shift) X
@@ -603,15 +657,15 @@ void pcgRun(const PcgPlan<T> &pl, cudaStream_t s) {
         reinterpret_cast<const V *>(pl.X), pl.ldx,
         reinterpret_cast<const V *>(pl.AP), reinterpret_cast<V *>(pl.W),
         reinterpret_cast<V *>(pl.R), reinterpret_cast<V *>(pl.Z),
-        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.coef, pl.shift,
-        pl.partials, nblk);
+        reinterpret_cast<V *>(pl.P), pl.N, pl.lamShift, pl.inv, pl.partials,
+        nblk);
   }
   if (pl.ndone) cudaMemsetAsync(pl.ndone, 0, sizeof(int), s);
   cudaMemsetAsync(pl.arrive, 0, 2 * sizeof(unsigned) * pl.ncols, s);
   pcgInitFinish<<<pl.ncols, 32, 0, s>>>(pl.st, pl.partials, nblk, pl.tol,
                                         pl.ndone);
-  // Early exit: after the init and after every step a one-thread kernel
-  // writes the count of finished columns into the next slot of mapped
+  // Early exit: after the init (a one-thread kernel) and in the last kernel
+  // of every step a thread writes the count of finished columns into the next slot of mapped
   // pinned host memory (slot 0 after the init, it + 1 after step it); the
   // host marks a slot unwritten (-1) before it launches the step that
   // writes it. Before step `it` the host reads the slot of step it - kLag
@@ -649,15 +703,15 @@ void pcgRun(const PcgPlan<T> &pl, cudaStream_t s) {
     pcgUpdateKernel<T><<<grid, kThreads, 0, s>>>(
         reinterpret_cast<V *>(pl.W), reinterpret_cast<V *>(pl.R),
         reinterpret_cast<V *>(pl.Z), reinterpret_cast<const V *>(pl.P),
-        reinterpret_cast<const V *>(pl.AP), pl.N, pl.st, pl.coef, pl.shift,
-        pl.invd, pl.partials2, nblk, pl.arrive + pl.ncols, pl.live,
+        reinterpret_cast<const V *>(pl.AP), pl.N, pl.st, pl.inv, pl.invd,
+        pl.partials2, nblk, pl.arrive + pl.ncols, pl.live,
         pl.ndone);
     pcgPKernel<T><<<grid, kThreads, 0, s>>>(
         reinterpret_cast<V *>(pl.P), reinterpret_cast<const V *>(pl.Z), pl.N,
-        pl.st);
-    mark();
+        pl.st, pl.ndone, poll ? poll->hostDev : nullptr,
+        poll ? poll->counter : nullptr);
   };
-  // One step is the same five launches with the same arguments every time:
+  // One step is the same four launches with the same arguments every time:
   // after a first direct step (which also settles the stencil's tuned
   // shape), it is captured once into a CUDA graph and replayed, one graph
   // launch per step. NCGM_PCG_GRAPH=0 keeps direct launches.

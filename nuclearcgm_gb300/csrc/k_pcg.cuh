@@ -24,9 +24,9 @@ template <class T> struct PcgPlan {
   size_t ldx = 0;
   void *W = nullptr, *R = nullptr, *Z = nullptr, *P = nullptr, *AP = nullptr;
   const double *lamShift = nullptr; // lambda_k + shift per column (device)
-  const double *coef = nullptr;     // Jacobi diagonal c0 per point (n^3)
-  // FP32 plans: 1 / (c0 + shift) per point in FP32 (n^3), for the step's
-  // preconditioner (null: FP64 division from coef)
+  // inverse Jacobi diagonal 1 / (c0 + shift) per point (n^3), and its FP32
+  // copy for the step's preconditioner of FP32 plans (null: the FP64 one)
+  const double *inv = nullptr;
   const float *invd = nullptr;
   double shift = 0, tol = 0;
   int maxSteps = 0;
@@ -56,12 +56,12 @@ template <class T> struct PcgPlan {
 };
 
 int pcgBlocks(size_t N);
-// The Jacobi diagonal c0 = U + UC + 7.5 f / h^2 of a species' current
-// coefficient table, one double per lattice point, in a context buffer.
-double *jacobiDiagonal(ncgm_ctx *ctx, int species, cudaStream_t s);
-// inv[p] = 1 / (c0[p] + shift) in FP32 (1 where the sum is 0)
-void inverseDiagonal32(const double *c0, double shift, size_t ns, float *inv,
-                       cudaStream_t s);
+// inv[p] = 1 / (c0 + shift) (1 where the sum is 0) for the Jacobi diagonal
+// c0 = U + UC + 7.5 f / h^2 of a species' current coefficient table, one
+// double per lattice point, in a context buffer; inv32: its FP32 copy (may be
+// null)
+double *inverseJacobiDiagonal(ncgm_ctx *ctx, int species, double shift,
+                              float *inv32, cudaStream_t s);
 template <class T> void pcgRun(const PcgPlan<T> &plan, cudaStream_t s);
 
 } // namespace ncgm
