@@ -118,73 +118,6 @@ __device__ inline double2 cconjmul(double2 a, double2 b) { // conj(a) b
   return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
 
-// One CTA. G (m x m, col-major, Hermitian, upper triangle used) ->
-// R upper with G = R^H R, columns whose pivot <= dropTol are dropped (their
-// row/column of R zero). Writes T = R^{-1} (m x m, zero rows/cols for dropped
-// columns) and keep[j] (1 kept, 0 dropped). Work arrays in global memory.
-__global__ void cholDropKernel(const double2 *G, int ldg, int m,
-                               double dropTol, double2 *R, double2 *T,
-                               int *keep) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int e = tid; e < m * m; e += nt) {
-    R[e] = make_double2(0, 0);
-    T[e] = make_double2(0, 0);
-  }
-  __syncthreads();
-  __shared__ double piv;
-  for (int j = 0; j < m; ++j) {
-    // pivot: d = G_jj - sum_{k<j} |R_kj|^2
-    if (tid == 0) {
-      double d = G[(size_t)j * ldg + j].x;
-      for (int k = 0; k < j; ++k) {
-        double2 r = R[(size_t)j * m + k];
-        d -= r.x * r.x + r.y * r.y;
-      }
-      // The Gram pivot carries a rounding floor of ~eps * G_jj, so a column
-      // whose residual is below that floor is dependent to working precision
-      // and is dropped, as MGS drops residual norms below 1e-12.
-      const double floor = fmax(dropTol, 64.0 * 2.220446049250313e-16 *
-                                             G[(size_t)j * ldg + j].x);
-      const int kp = (d > floor) ? 1 : 0;
-      piv = kp ? d : 0.0;
-      keep[j] = kp;
-      if (kp) R[(size_t)j * m + j] = make_double2(sqrt(d), 0.0);
-    }
-    __syncthreads();
-    if (piv > 0.0) {
-      const double rjj = sqrt(piv);
-      // R_ji = (G_ji - sum_{k<j} conj(R_kj) R_ki) / R_jj, i > j
-      for (int i = j + 1 + tid; i < m; i += nt) {
-        double2 s = G[(size_t)i * ldg + j];
-        for (int k = 0; k < j; ++k) {
-          double2 t = cconjmul(R[(size_t)j * m + k], R[(size_t)i * m + k]);
-          s.x -= t.x;
-          s.y -= t.y;
-        }
-        R[(size_t)i * m + j] = make_double2(s.x / rjj, s.y / rjj);
-      }
-    }
-    __syncthreads();
-  }
-  // T = R^{-1} restricted to kept columns: solve R T = I column by column
-  // (upper triangular back substitution), one thread per column of T.
-  for (int c = tid; c < m; c += nt) {
-    if (!keep[c]) continue;
-    for (int i = c; i >= 0; --i) {
-      if (!keep[i]) continue;
-      double2 s = make_double2(i == c ? 1.0 : 0.0, 0.0);
-      for (int k = i + 1; k <= c; ++k) {
-        if (!keep[k]) continue;
-        double2 t = cmul(R[(size_t)k * m + i], T[(size_t)c * m + k]);
-        s.x -= t.x;
-        s.y -= t.y;
-      }
-      double rii = R[(size_t)i * m + i].x;
-      T[(size_t)c * m + i] = make_double2(s.x / rii, s.y / rii);
-    }
-  }
-}
-
 // FP64 cyclic Jacobi sweeps sweep0 .. 59 on the Hermitian A (m x m,
 // column-major), rotations accumulated into Vm (round-robin pairing: every
 // round rotates m/2 disjoint (p,q) pairs at once). Returns 1 on convergence.
@@ -628,12 +561,101 @@ void BlockProducts::vc(const double2 *V, size_t ldv, int m, const double2 *Cm,
     gemmVC(V, ldv, m, Cm, ldc, k, Y, ldy, N, accum ? 1.0 : 0.0, s);
 }
 
+// a / b from the correctly rounded r = 1 / b, rounded as the division is
+// (Markstein 1990: one residual step on a r), for three operations of the FP64
+// pipe instead of a division's ten
+__device__ __forceinline__ double divBy(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
+
+// T = R^{-1} on the kept columns: one warp per column c of T, by columns of R:
+// x_i = s_i / R_ii, then s_k -= R_ki x_i for all k < i at once. Bound by the
+// chain of one FP64 step (64 cycles an operation) per row; the columns of R
+// come four steps ahead by asynchronous copies. One thread per column with a
+// dot product per element ran m^2 / 2 such steps: m = 192 5860 -> 180 us, m = 60
+// about 250 -> 39 us. Dropped rows stay zero. T starts as zero.
+// Without kStaged (columns too long for shared memory) R is read and T's
+// column built where they are.
+constexpr int kInvAhead = 4;
+template <bool kStaged>
+__global__ void __launch_bounds__(32)
+    cholInvKernel(const double2 *R, int m, const int *keep, double2 *T) {
+  extern __shared__ double2 inv[];
+  const int c = blockIdx.x, lane = threadIdx.x;
+  if (!keep[c]) return;
+  // sv: the right-hand side, then T's column
+  double2 *sv = kStaged ? inv : T + (size_t)c * m, *ring = inv + m;
+  double *rd = reinterpret_cast<double *>(ring + (size_t)kInvAhead * m);
+  auto fetch = [&](int i) {
+    if (kStaged && i >= 0) {
+      const unsigned to = static_cast<unsigned>(
+          __cvta_generic_to_shared(ring + (size_t)(i % kInvAhead) * m));
+      const double2 *from = R + (size_t)i * m;
+      for (int k = lane; k <= i; k += 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         to + 16u * (unsigned)k),
+                     "l"(from + k)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int a = 0; a < kInvAhead - 1; ++a) fetch(c - a);
+  for (int i = lane; i <= c; i += 32) {
+    // 0 marks a dropped row
+    if (kStaged) rd[i] = keep[i] ? 1.0 / R[(size_t)i * m + i].x : 0.0;
+    sv[i] = make_double2(i == c ? 1.0 : 0.0, 0.0);
+  }
+  for (int i = c; i >= 0; --i) {
+    fetch(i - kInvAhead + 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kInvAhead - 1) : "memory");
+    __syncwarp();
+    const double2 *col =
+        kStaged ? ring + (size_t)(i % kInvAhead) * m : R + (size_t)i * m;
+    const double rii = col[i].x,
+                 r = kStaged ? rd[i] : (keep[i] ? 1.0 / rii : 0.0);
+    double2 x = make_double2(0.0, 0.0);
+    if (r != 0.0) {
+      const double2 b = sv[i];
+      x = make_double2(divBy(b.x, rii, r), divBy(b.y, rii, r));
+      for (int k = lane; k < i; k += 32) {
+        const double2 a = col[k];
+        double2 v = sv[k];
+        v.x = fma(a.y, x.y, fma(-a.x, x.x, v.x));
+        v.y = fma(-a.y, x.x, fma(-a.x, x.y, v.y));
+        sv[k] = v;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) sv[i] = x;
+  }
+  __syncwarp();
+  if (kStaged)
+    for (int i = lane; i <= c; i += 32) T[(size_t)c * m + i] = sv[i];
+}
+
+// e -> (row, column) of the e-th element of an upper triangle stored by
+// columns
+__device__ __forceinline__ void triangleAt(int e, int &a, int &b) {
+  b = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+  while (b * (b + 1) / 2 > e) --b;
+  while ((b + 1) * (b + 2) / 2 <= e) ++b;
+  a = e - b * (b + 1) / 2;
+}
+
+// The factorisations in shared memory leave T to cholInvKernel from this size
+// on: measured with T, FP64, m = 60: 427 us inside, 163 us with the second
+// launch. Below, T is small, and the serial order of its sums is the one that
+// the fixed points of the small lattices were compared in.
+constexpr int kInvOutside = 48;
+
 // Same factorisation in shared memory, right-looking: at step j the pivot is
 // the updated diagonal A_jj = G_jj - sum_{k<j} |R_kj|^2, row j of R is
 // A_j. / R_jj, and the trailing upper triangle takes the rank-1 update
 // A_ab -= conj(R_ja) R_jb in parallel (one barrier-separated phase per
-// step instead of a serial dot product per element). The drop rule and
-// T = R^{-1} are those of cholDropKernel.
+// step instead of a serial dot product per element). A column whose pivot
+// is not above max(dropTol, 64 eps G_jj) is dropped: keep[j] = 0 and its row of
+// R, its row and its column of T are zero.
 constexpr int kCholSmemMax = 80; // 2 m^2 double2 <= 200 KB
 // The FP32 forms' CholQR factor with the matrix held as double-float in
 // shared memory: the O(m^3) trailing updates and R^-1 run on the FP32 pipe
@@ -682,13 +704,14 @@ __global__ void cholDropDfKernel(const double2 *G, int ldg, int m,
       }
       __syncthreads();
       const int w = m - j - 1;
-      for (int e = tid; e < w * w; e += nt) {
-        const int a = j + 1 + e % w, b = j + 1 + e / w;
-        if (a <= b) {
-          const dfc t = dfcConjMul(A[(size_t)a * m + j], A[(size_t)b * m + j]);
-          dfc &x = A[(size_t)b * m + a];
-          x = dfcSub(x, t);
-        }
+      for (int e = tid; e < w * (w + 1) / 2; e += nt) {
+        int a, b;
+        triangleAt(e, a, b);
+        a += j + 1;
+        b += j + 1;
+        const dfc t = dfcConjMul(A[(size_t)a * m + j], A[(size_t)b * m + j]);
+        dfc &x = A[(size_t)b * m + a];
+        x = dfcSub(x, t);
       }
     } else {
       for (int i = j + tid; i < m; i += nt) A[(size_t)i * m + j] = zero;
@@ -698,7 +721,7 @@ __global__ void cholDropDfKernel(const double2 *G, int ldg, int m,
   }
   // T = R^{-1} on the kept columns, one thread per column; dropped rows and
   // columns hold zeros in R and T, so they add nothing to the sums
-  for (int c = tid; c < m; c += nt) {
+  for (int c = tid; c < m && m < kInvOutside; c += nt) {
     if (!kp[c]) continue;
     for (int i = c; i >= 0; --i) {
       if (!kp[i]) continue;
@@ -732,7 +755,7 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
   double2 *Ts = csm + m * m; // T
   __shared__ int kp[kCholSmemMax];
   __shared__ double gd[kCholSmemMax]; // the Gram diagonal (drop floor)
-  __shared__ double piv;
+  __shared__ double piv, rjjS, rinvS;
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < m * m; e += nt) {
     const double2 g = G[(size_t)(e / m) * ldg + (e % m)];
@@ -749,26 +772,32 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
       const int k = (d > floor) ? 1 : 0;
       kp[j] = k;
       piv = k ? d : 0.0;
+      if (k) { // one thread: eight warps would queue for the FP64 pipe
+        rjjS = sqrt(d);
+        rinvS = 1.0 / rjjS;
+      }
     }
     __syncthreads();
     const double pv = piv;
     if (pv > 0.0) {
-      const double rjj = sqrt(pv);
+      const double rjj = rjjS, rinv = rinvS;
       for (int i = j + 1 + tid; i < m; i += nt) {
         const double2 a = A[(size_t)i * m + j];
-        A[(size_t)i * m + j] = make_double2(a.x / rjj, a.y / rjj);
+        A[(size_t)i * m + j] = make_double2(divBy(a.x, rjj, rinv),
+                                              divBy(a.y, rjj, rinv));
       }
       if (tid == 0) A[(size_t)j * m + j] = make_double2(rjj, 0.0);
       __syncthreads();
       const int w = m - j - 1;
-      for (int e = tid; e < w * w; e += nt) {
-        const int a = j + 1 + e % w, b = j + 1 + e / w;
-        if (a <= b) {
-          const double2 t = cconjmul(A[(size_t)a * m + j], A[(size_t)b * m + j]);
-          double2 &x = A[(size_t)b * m + a];
-          x.x -= t.x;
-          x.y -= t.y;
-        }
+      for (int e = tid; e < w * (w + 1) / 2; e += nt) {
+        int a, b;
+        triangleAt(e, a, b);
+        a += j + 1;
+        b += j + 1;
+        const double2 t = cconjmul(A[(size_t)a * m + j], A[(size_t)b * m + j]);
+        double2 &x = A[(size_t)b * m + a];
+        x.x -= t.x;
+        x.y -= t.y;
       }
     } else {
       for (int i = j + tid; i < m; i += nt) A[(size_t)i * m + j] = make_double2(0, 0);
@@ -776,7 +805,7 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
     __syncthreads();
   }
   // T = R^{-1} on the kept columns, one thread per column of T
-  for (int c = tid; c < m; c += nt) {
+  for (int c = tid; c < m && m < kInvOutside; c += nt) {
     if (!kp[c]) continue;
     for (int i = c; i >= 0; --i) {
       if (!kp[i]) continue;
@@ -802,8 +831,8 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
 
 // Large m (> 80): the same right-looking factorisation in global memory with
 // one launch pair per column (pivot and row scaling in one block, the rank-1
-// update of the trailing triangle over the whole GPU), then T = R^{-1} one
-// thread per column. G's diagonal (drop floor) and the pivots are kept in
+// update of the trailing triangle over the whole GPU), then T = R^{-1}
+// (cholInvKernel). G's diagonal (drop floor) and the pivots are kept in
 // T's first 2m entries until T is computed.
 __global__ void cholCopyKernel(const double2 *G, int ldg, int m, double2 *R,
                                double2 *T) {
@@ -855,22 +884,19 @@ __global__ void cholFinishKernel(double2 *R, int m, double2 *T) {
   if (e % m > e / m) R[e] = make_double2(0, 0); // lower triangle
   T[e] = make_double2(0, 0);
 }
-__global__ void cholInvKernel(const double2 *R, int m, const int *keep,
-                              double2 *T) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m || !keep[c]) return;
-  for (int i = c; i >= 0; --i) {
-    if (!keep[i]) continue;
-    double2 sum = make_double2(i == c ? 1.0 : 0.0, 0.0);
-    for (int k = i + 1; k <= c; ++k) {
-      if (!keep[k]) continue;
-      const double2 t = cmul(R[(size_t)k * m + i], T[(size_t)c * m + k]);
-      sum.x -= t.x;
-      sum.y -= t.y;
-    }
-    const double rii = R[(size_t)i * m + i].x;
-    T[(size_t)c * m + i] = make_double2(sum.x / rii, sum.y / rii);
+static void cholInverse(const double2 *R, int m, const int *keep, double2 *T,
+                        cudaStream_t s) {
+  const size_t smem =
+      (size_t)m * ((1 + kInvAhead) * sizeof(double2) + sizeof(double));
+  if (smem > 200 * 1024) { // m > 2327
+    cholInvKernel<false><<<m, 32, 0, s>>>(R, m, keep, T);
+    return;
   }
+  if (smem > 48 * 1024)
+    cudaFuncSetAttribute(cholInvKernel<true>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+  cholInvKernel<true><<<m, 32, smem, s>>>(R, m, keep, T);
 }
 
 void cholDrop(const double2 *G, int ldg, int m, double dropTol, double2 *R,
@@ -885,33 +911,30 @@ void cholDrop(const double2 *G, int ldg, int m, double dropTol, double2 *R,
         cholUpdateKernel<<<dim3((w + 127) / 128, w), 128, 0, s>>>(R, m, j, T);
     }
     cholFinishKernel<<<gm, 256, 0, s>>>(R, m, T);
-    cholInvKernel<<<(m + 63) / 64, 64, 0, s>>>(R, m, keep, T);
+    cholInverse(R, m, keep, T, s);
     return;
   }
-  if (m <= kCholSmemMax) {
-    static const bool attr = [] {
-      cudaFuncSetAttribute(cholDropSmemKernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           2 * kCholSmemMax * kCholSmemMax * (int)sizeof(double2));
-      return true;
-    }();
-    (void)attr;
-    const size_t smem = 2 * (size_t)m * m * sizeof(double2);
-    static const bool dfAttr = [] {
-      cudaFuncSetAttribute(cholDropDfKernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           2 * kCholSmemMax * kCholSmemMax * (int)sizeof(dfc));
-      return true;
-    }();
-    (void)dfAttr;
-    if (fast)
-      cholDropDfKernel<<<1, 256, 2 * (size_t)m * m * sizeof(dfc), s>>>(
-          G, ldg, m, dropTol, R, T, keep);
-    else
-      cholDropSmemKernel<<<1, 256, smem, s>>>(G, ldg, m, dropTol, R, T, keep);
-    return;
-  }
-  cholDropKernel<<<1, 256, 0, s>>>(G, ldg, m, dropTol, R, T, keep);
+  static const bool attr = [] {
+    cudaFuncSetAttribute(cholDropSmemKernel,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         2 * kCholSmemMax * kCholSmemMax * (int)sizeof(double2));
+    return true;
+  }();
+  (void)attr;
+  const size_t smem = 2 * (size_t)m * m * sizeof(double2);
+  static const bool dfAttr = [] {
+    cudaFuncSetAttribute(cholDropDfKernel,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         2 * kCholSmemMax * kCholSmemMax * (int)sizeof(dfc));
+    return true;
+  }();
+  (void)dfAttr;
+  if (fast)
+    cholDropDfKernel<<<1, 256, 2 * (size_t)m * m * sizeof(dfc), s>>>(
+        G, ldg, m, dropTol, R, T, keep);
+  else
+    cholDropSmemKernel<<<1, 256, smem, s>>>(G, ldg, m, dropTol, R, T, keep);
+  if (m >= kInvOutside) cholInverse(R, m, keep, T, s);
 }
 
 // NCGM_HEIG_FP64=1 keeps the one-CTA FP64 Jacobi for every size
