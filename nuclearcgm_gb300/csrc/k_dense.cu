@@ -262,7 +262,8 @@ __device__ void jacobiFinish(double2 *A, const double2 *Vm, int m,
 // w: eigenvalues ascending; Vm: eigenvectors in the same order.
 __global__ void heigKernel(const double2 *Ain, int lda, int m, double2 *Ag,
                            double2 *Vg, double *w, int *perm, int *status,
-                           int useSmem) {
+                           int useSmem, int onlyIfFailed) {
+  if (onlyIfFailed && *status == 0) return;
   // working copies in shared memory when they fit: useSmem 2 = A and V
   // (m <= 81), 1 = A only (m <= 114), 0 = both in the global work buffers
   extern __shared__ double2 hsm[];
@@ -959,7 +960,8 @@ static bool heigMidOn() {
 }
 
 size_t heigScratchBytes(int m) {
-  return std::max(heigMidScratchBytes(m), heigLargeScratchBytes(m));
+  return std::max({heigMidScratchBytes(m), heigLargeScratchBytes(m),
+                   heigRefinedScratchBytes(m)});
 }
 
 void heig(const double2 *A, int lda, int m, double2 *work, double2 *V,
@@ -1013,14 +1015,23 @@ void heig(const double2 *A, int lda, int m, double2 *work, double2 *V,
         heigLarge(A, lda, m, V, w, perm, status, scr, s);
       }))
     return;
+  // The refined double-float method in FP64: m = 60 5100 -> 1250 us, m = 48
+  // 6050 -> 1060 us with the copies of a whole call. Below 48 the Jacobi stays:
+  // it is cheaper there (860 us for m = 8 and 24 together), and the fixed
+  // points of the small lattices were compared in its roundings.
+  const bool refined =
+      !heigFp64Only() && heigRefinedTakes(m) &&
+      withScratch(heigRefinedScratchBytes(m), [&](void *scr) {
+        heigRefined(A, lda, m, V, w, perm, status, scr, s);
+      });
   const size_t mat = (size_t)m * m * sizeof(double2);
   const int sm = 2 * mat <= kMaxDyn ? 2 : (mat <= kMaxDyn ? 1 : 0);
   const size_t smem = sm == 2 ? 2 * mat : (sm == 1 ? mat : 0);
   // a round updates m x m/2 elements between barriers: small problems run
   // with fewer warps, so each of the ~4 barriers per round is cheaper
   const int threads = m <= 32 ? 128 : (m <= 48 ? 256 : 512);
-  heigKernel<<<1, threads, smem, s>>>(A, lda, m, work, V, w, perm, status,
-                                      sm);
+  heigKernel<<<1, threads, smem, s>>>(A, lda, m, work, V, w, perm, status, sm,
+                                      refined ? 1 : 0);
 }
 
 } // namespace ncgm

@@ -83,11 +83,18 @@ void heigMid(const double2 *A, int lda, int m, double2 *V, double *w,
              int *perm, int *status, void *scratch, cudaStream_t s);
 size_t heigMidScratchBytes(int m);
 int heigMidMax();
+// FP64 solver for the sizes that heigRefinedTakes: heigMid and one step of FP64
+// refinement (k_heig_refine.cu). *status = 1: it gave up, solve again.
+bool heigRefinedTakes(int m);
+size_t heigRefinedScratchBytes(int m);
+void heigRefined(const double2 *A, int lda, int m, double2 *V, double *w,
+                 int *perm, int *status, void *scratch, cudaStream_t s);
 // Hermitian eigensolver (lower triangle): w ascending, V eigenvectors (m x m).
 // fast (the FP32 precision forms): for m <= heigMidMax(), the one-CTA
 // double-float Householder method (heigMid; with NCGM_HEIG_MID=0 the
-// double-float Jacobi up to m = 80); otherwise the FP64 Jacobi up to m = 80
-// and the multi-kernel Householder method above it. Degenerate eigenvectors
+// double-float Jacobi up to m = 80); otherwise the FP64 Jacobi below
+// m = 48, the refined method up to m = 80 and the multi-kernel Householder
+// method above it. Degenerate eigenvectors
 // may come out rotated within their eigenspace between the methods.
 // scratch (optional, heigScratchBytes(m) bytes): the Householder methods'
 // workspace; without it they take stream-ordered allocations per call.
