@@ -7,8 +7,7 @@
 // is also tridiagonalisation based):
 //  1. Householder tridiagonalisation of the full Hermitian matrix, one step
 //     per column: the reflector (one block), the matrix-vector product
-//     p = tau A22 v split over row blocks and column chunks, w = p - tau/2
-//     (p^H v) v, and the rank-2 update A22 -= v w^H + w v^H over the whole
+//     p = tau A22 v with a warp per row, w = p - tau/2 (p^H v) v, and the rank-2 update A22 -= v w^H + w v^H over the whole
 //     grid. Reflectors H = I - tau v v^H with real beta (the LAPACK
 //     convention), so the tridiagonal matrix is real.
 //  2. Eigenvalues of the real tridiagonal by multisection on Sturm counts,
@@ -34,7 +33,6 @@ namespace ncgm {
 namespace {
 
 constexpr int kT = 256;
-constexpr int kJC = 32; // column chunks of the matrix-vector product
 
 __device__ __forceinline__ double2 cmulD(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -42,16 +40,56 @@ __device__ __forceinline__ double2 cmulD(double2 a, double2 b) {
 __device__ __forceinline__ double2 cconjmulD(double2 a, double2 b) {
   return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
-__device__ double blockSumD(double v, double *sh) {
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+// sums of K values over the block in all threads: the tree v_t += v_{t+s}, s =
+// blockDim / 2 .. 1, the levels above a warp through shared memory (sh: K x
+// blockDim values), the last five by shuffles
+template <int K> __device__ void blockSumsD(double (&v)[K], double *sh) {
+  const int t = threadIdx.x, nt = blockDim.x;
+  for (int s = nt / 2; s >= 32; s >>= 1) {
+    if (t >= s && t < 2 * s)
+#pragma unroll
+      for (int k = 0; k < K; ++k) sh[k * nt + t] = v[k];
     __syncthreads();
+    if (t < s)
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] += sh[k * nt + t + s];
   }
-  const double r = sh[0];
+  if (t < 32) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        v[k] += __shfl_down_sync(0xffffffffu, v[k], s);
+    if (t == 0)
+#pragma unroll
+      for (int k = 0; k < K; ++k) sh[k * nt] = v[k];
+  }
   __syncthreads();
-  return r;
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = sh[k * nt];
+  __syncthreads();
+}
+__device__ double blockSumD(double v, double *sh) {
+  double x[1] = {v};
+  blockSumsD(x, sh);
+  return x[0];
+}
+
+// True in the block of the grid that arrives last, which then sees what all
+// others wrote (read it with __ldcg: lines may be stale in the SM's L1). It
+// resets the counter for the next launch.
+__device__ bool lastBlock(unsigned *counter) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned all = gridDim.x * gridDim.y;
+    last = atomicAdd(counter, 1u) == all - 1;
+    if (last) *counter = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
 }
 
 // full Hermitian copy from the lower triangle of Ain
@@ -69,35 +107,51 @@ __global__ void fullCopyKernel(const double2 *Ain, int lda, int m,
   A[e] = v;
 }
 
-// step k: reflector of x = A[k+1:, k] into Vr[:, k], tau[k], d[k], e[k]
-__global__ void hhVectorKernel(const double2 *A, int m, int k, double2 *Vr,
-                               double2 *tau, double *d, double *e) {
-  __shared__ double sh[kT];
-  __shared__ double2 sc;   // 1 / (alpha - beta)
+// step k: reflector of x = A[k+1:, k] into Vr[:, k], tau[k], d[k], e[k] (one
+// block of kT threads)
+__device__ void hhVector(const double2 *A, int m, int k, double2 *Vr,
+                         double2 *tau, double *d, double *e, double *sh) {
+  __shared__ double2 sc; // 1 / (alpha - beta)
   __shared__ int skip;
   const int L = m - k - 1;
   const double2 *x = A + (size_t)k * m + k + 1;
   double loc = 0;
-  for (int i = 1 + threadIdx.x; i < L; i += blockDim.x)
-    loc += x[i].x * x[i].x + x[i].y * x[i].y;
+  for (int i = 1 + threadIdx.x; i < L; i += blockDim.x) {
+    const double2 v = __ldcg(x + i);
+    loc += v.x * v.x + v.y * v.y;
+  }
   const double xn2 = blockSumD(loc, sh);
-  if (threadIdx.x == 0) {
-    const double2 al = x[0];
-    d[k] = A[(size_t)k * m + k].x;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const double2 al = __ldcg(x);
+    if (lane == 0) d[k] = __ldcg(A + (size_t)k * m + k).x;
     if (xn2 == 0.0 && al.y == 0.0) {
-      tau[k] = make_double2(0.0, 0.0);
-      e[k] = al.x;
-      skip = 1;
+      if (lane == 0) {
+        tau[k] = make_double2(0.0, 0.0);
+        e[k] = al.x;
+        skip = 1;
+      }
     } else {
       const double beta =
           -(al.x >= 0.0 ? 1.0 : -1.0) * sqrt(al.x * al.x + al.y * al.y + xn2);
-      tau[k] = make_double2((beta - al.x) / beta, -al.y / beta);
-      e[k] = beta;
-      // 1 / (alpha - beta)
+      // tau = ((beta - alpha_r) / beta, -alpha_i / beta) and 1 / (alpha -
+      // beta): four divisions, one per lane
       const double2 den = make_double2(al.x - beta, al.y);
       const double dd = den.x * den.x + den.y * den.y;
-      sc = make_double2(den.x / dd, -den.y / dd);
-      skip = 0;
+      const double num = lane == 0   ? beta - al.x
+                         : lane == 1 ? -al.y
+                         : lane == 2 ? den.x
+                                     : -den.y;
+      const double q = num / (lane < 2 ? beta : dd);
+      const double q1 = __shfl_sync(0xffffffffu, q, 1),
+                   q2 = __shfl_sync(0xffffffffu, q, 2),
+                   q3 = __shfl_sync(0xffffffffu, q, 3);
+      if (lane == 0) {
+        tau[k] = make_double2(q, q1);
+        e[k] = beta;
+        sc = make_double2(q2, q3);
+        skip = 0;
+      }
     }
   }
   __syncthreads();
@@ -105,56 +159,59 @@ __global__ void hhVectorKernel(const double2 *A, int m, int k, double2 *Vr,
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     double2 r = make_double2(0.0, 0.0);
     if (!skip && i > k) r = (i == k + 1) ? make_double2(1.0, 0.0)
-                                        : cmulD(x[i - k - 1], sc);
+                                        : cmulD(__ldcg(x + i - k - 1), sc);
     v[i] = r;
   }
 }
-
-// partial products P[c][i] = sum_{j in chunk c} A22[i][j] v_j (rows k+1..)
-__global__ void hhMatvecKernel(const double2 *A, int m, int k,
-                               const double2 *Vr, double2 *P) {
-  const int L = m - k - 1;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  if (i >= L) return;
-  const int per = (L + kJC - 1) / kJC;
-  const int j0 = c * per, j1 = min(L, j0 + per);
-  const double2 *v = Vr + (size_t)k * m + k + 1;
-  double2 s = make_double2(0.0, 0.0);
-  for (int j = j0; j < j1; ++j) {
-    const double2 a = A[(size_t)(k + 1 + j) * m + (k + 1 + i)];
-    const double2 t = cmulD(a, v[j]);
-    s.x += t.x;
-    s.y += t.y;
-  }
-  P[(size_t)c * m + i] = s;
+__global__ void __launch_bounds__(kT)
+    hhFirstKernel(const double2 *A, int m, double2 *Vr, double2 *tau, double *d,
+                  double *e) {
+  __shared__ double sh[kT];
+  hhVector(A, m, 0, Vr, tau, d, e, sh);
 }
 
-// w = p - tau/2 (p^H v) v with p = tau sum_c P[c] (one block)
-__global__ void hhWKernel(int m, int k, const double2 *P, const double2 *Vr,
-                          const double2 *tau, double2 *Wv) {
-  __shared__ double sh[kT];
-  const int L = m - k - 1;
-  const double2 t = tau[k];
+// p = tau A22 v, one warp per row: row i is the conjugate of column i, which is
+// contiguous. The last block to finish then forms w = p - tau/2 (p^H v) v. A
+// step is two launches of this kind (four separate ones took 19 us and 9 us of
+// gaps between them at m = 160, these 15 and 6). A split of the columns over
+// blocks left 32 partial sums per row to the one block: 5 k cycles of its FP64
+// pipe.
+__global__ void __launch_bounds__(kT)
+    hhMatvecKernel(const double2 *A, int m, int k, const double2 *Vr,
+                   const double2 *tau, double2 *P, double2 *Wv,
+                   unsigned *counter) {
+  __shared__ double sh[2 * kT];
+  const int L = m - k - 1, lane = threadIdx.x % 32;
+  const int row = blockIdx.x * (kT / 32) + threadIdx.x / 32;
   const double2 *v = Vr + (size_t)k * m + k + 1;
-  double re = 0, im = 0;
-  for (int i = threadIdx.x; i < L; i += blockDim.x) {
-    double2 p = make_double2(0.0, 0.0);
-    for (int c = 0; c < kJC; ++c) {
-      p.x += P[(size_t)c * m + i].x;
-      p.y += P[(size_t)c * m + i].y;
+  const double2 t = tau[k];
+  if (row < L) {
+    const double2 *col = A + (size_t)(k + 1 + row) * m + k + 1;
+    double2 s = make_double2(0.0, 0.0);
+    for (int j = lane; j < L; j += 32) {
+      const double2 q = cconjmulD(col[j], v[j]);
+      s.x += q.x;
+      s.y += q.y;
     }
-    p = cmulD(t, p);
+    for (int o = 16; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) P[row] = cmulD(t, s);
+  }
+  if (!lastBlock(counter)) return;
+  double dot[2] = {0.0, 0.0};
+  for (int i = threadIdx.x; i < L; i += blockDim.x) {
+    const double2 p = __ldcg(P + i);
     Wv[i] = p;
     const double2 pv = cconjmulD(p, v[i]); // conj(p) v
-    re += pv.x;
-    im += pv.y;
+    dot[0] += pv.x;
+    dot[1] += pv.y;
   }
-  re = blockSumD(re, sh);
-  im = blockSumD(im, sh);
+  blockSumsD(dot, sh);
   // alpha2 = -1/2 tau (p^H v)
   const double2 a2 = cmulD(make_double2(-0.5 * t.x, -0.5 * t.y),
-                           make_double2(re, im));
+                           make_double2(dot[0], dot[1]));
   for (int i = threadIdx.x; i < L; i += blockDim.x) {
     const double2 av = cmulD(a2, v[i]);
     Wv[i].x += av.x;
@@ -162,21 +219,25 @@ __global__ void hhWKernel(int m, int k, const double2 *P, const double2 *Vr,
   }
 }
 
-// A22[i][j] -= v_i conj(w_j) + w_i conj(v_j)
-__global__ void hhUpdateKernel(double2 *A, int m, int k, const double2 *Vr,
-                               const double2 *Wv, const double2 *tau) {
+// A22[i][j] -= v_i conj(w_j) + w_i conj(v_j), two columns per block; the last
+// block to finish makes the next column's reflector
+__global__ void __launch_bounds__(kT)
+    hhUpdateKernel(double2 *A, int m, int k, double2 *Vr, const double2 *Wv,
+                   double2 *tau, double *d, double *e, unsigned *counter) {
+  __shared__ double sh[kT];
   const double2 t = tau[k];
-  if (t.x == 0.0 && t.y == 0.0) return;
   const int L = m - k - 1;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y;
-  if (i >= L || j >= L) return;
-  const double2 *v = Vr + (size_t)k * m + k + 1;
-  const double2 a = cconjmulD(Wv[j], v[i]); // v_i conj(w_j)
-  const double2 b = cconjmulD(v[j], Wv[i]); // w_i conj(v_j)
-  double2 &x = A[(size_t)(k + 1 + j) * m + (k + 1 + i)];
-  x.x -= a.x + b.x;
-  x.y -= a.y + b.y;
+  const int i = blockIdx.x * (kT / 2) + threadIdx.x % (kT / 2);
+  const int j = blockIdx.y * 2 + threadIdx.x / (kT / 2);
+  if (i < L && j < L && !(t.x == 0.0 && t.y == 0.0)) {
+    const double2 *v = Vr + (size_t)k * m + k + 1;
+    const double2 a = cconjmulD(Wv[j], v[i]); // v_i conj(w_j)
+    const double2 b = cconjmulD(v[j], Wv[i]); // w_i conj(v_j)
+    double2 &x = A[(size_t)(k + 1 + j) * m + (k + 1 + i)];
+    x.x -= a.x + b.x;
+    x.y -= a.y + b.y;
+  }
+  if (lastBlock(counter)) hhVector(A, m, k + 1, Vr, tau, d, e, sh);
 }
 
 __global__ void lastDiagKernel(const double2 *A, int m, double *d) {
@@ -198,41 +259,113 @@ __device__ int sturmCount(const double *d, const double *e, int m, double x,
   return c;
 }
 
-// eigenvalue j (ascending) by multisection from the Gershgorin bounds, one
-// warp per eigenvalue: each step the 32 lanes count the eigenvalues below
-// 32 equally spaced points of the bracket (Sturm counts), which shrinks it
-// 33-fold, so about 11 steps reach the 2.3e-16 relative tolerance where
-// bisection takes ~55
-__global__ void multisectKernel(const double *d, const double *e, int m,
-                                double *w) {
-  const int j = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+// Multisection of [lo, hi] for eigenvalue j with the Sturm counts in
+// double-float arithmetic, down to a width of 2 tol: a quotient costs a few
+// dependent FP32 operations where an FP64 division takes ~600 cycles on GB300.
+// dd, ee: the diagonal and the squared off-diagonal in double-float.
+constexpr int kDfSturmMax = 512;
+__device__ void sectionDf(const dfl *dd, const dfl *ee, int m, int j,
+                          float pivmin, double tol, double &lo, double &hi) {
   const int lane = threadIdx.x % 32;
-  if (j >= m) return;
-  double lo = 1e300, hi = -1e300, emax = 0;
-  for (int i = lane; i < m; i += 32) {
+  for (int it = 0; it < 64; ++it) {
+    if (hi - lo <= 2.0 * tol) break;
+    const double step = (hi - lo) / 33.0;
+    const double x = lo + (lane + 1) * step;
+    bool below = false;
+    if (x > lo && x < hi) {
+      const dfl xd = dfFrom(x);
+      dfl q = dfSub(dd[0], xd);
+      int c = q.hi < 0.f ? 1 : 0;
+      for (int i = 1; i < m; ++i) {
+        if (fabsf(q.hi) < pivmin) q = {-pivmin, 0.f};
+        q = dfSub(dfSub(dd[i], xd), dfDiv(ee[i - 1], q));
+        if (q.hi < 0.f) ++c;
+      }
+      below = c <= j;
+    }
+    // the bracket is [x_k, x_{k+1}] for the last lane k whose point has at
+    // most j eigenvalues below it (the counts grow with the lane)
+    const unsigned mask = __ballot_sync(0xffffffffu, below);
+    const int k = mask ? 31 - __clz(mask) : -1;
+    const double nlo = k >= 0 ? lo + (k + 1) * step : lo;
+    const double nhi = k < 31 ? lo + (k + 2) * step : hi;
+    if (nlo == lo && nhi == hi) break; // no representable progress
+    lo = nlo;
+    hi = fmin(nhi, hi);
+  }
+}
+
+// Gershgorin bounds and the largest off-diagonal of the tridiagonal, by one
+// warp; its double-float form into dd, ee when it fits
+__device__ void sturmBounds(const double *d, const double *e, int m, dfl *dd,
+                            dfl *ee, double &lo, double &hi, double &emax) {
+  lo = 1e300;
+  hi = -1e300;
+  emax = 0;
+  for (int i = threadIdx.x % 32; i < m; i += 32) {
     double r = 0;
     if (i > 0) r += fabs(e[i - 1]);
     if (i + 1 < m) r += fabs(e[i]);
     lo = fmin(lo, d[i] - r);
     hi = fmax(hi, d[i] + r);
     if (i + 1 < m) emax = fmax(emax, fabs(e[i]));
+    if (m <= kDfSturmMax) {
+      dd[i] = dfFrom(d[i]);
+      if (i + 1 < m) {
+        const dfl ei = dfFrom(e[i]);
+        ee[i] = dfMul(ei, ei);
+      }
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
   }
+  __syncwarp();
+}
+
+// Eigenvalue j (ascending) by multisection from the Gershgorin bounds, one
+// warp per eigenvalue: each step the 32 lanes count the eigenvalues below
+// 32 equally spaced points of the bracket (Sturm counts), which shrinks it
+// 33-fold. Bound by the chain of FP64 divisions of a count (~600 cycles each):
+// the double-float counts make the first digits, and FP64 takes over from a
+// bracket of 1e-12 of the scale (their resolution with a margin) after a step
+// whose first and last point confirm it; if they do not, or the matrix does
+// not fit the double-float form, FP64 does all of it. m = 160: 940 -> 415 us.
+__global__ void __launch_bounds__(32)
+    multisectKernel(const double *d, const double *e, int m, double *w) {
+  __shared__ dfl dd[kDfSturmMax], ee[kDfSturmMax];
+  const int j = blockIdx.x, lane = threadIdx.x;
+  if (j >= m) return;
+  double lo, hi, emax;
+  sturmBounds(d, e, m, dd, ee, lo, hi, emax);
   const double scale = fmax(fabs(lo), fabs(hi));
   const double pivmin = fmax(1e-300, 2.3e-308 * fmax(1.0, emax * emax));
   const double tol = 2.3e-16 * scale;
+  if (m <= kDfSturmMax) {
+    double a = lo, b = hi;
+    sectionDf(dd, ee, m, j, (float)fmax(1e-30, 5.7e-14 * fmax(1.0, emax * emax)),
+              1.2e-13 * scale, a, b);
+    a = fmax(lo, a - 4e-13 * scale);
+    b = fmin(hi, b + 4e-13 * scale);
+    const double step = (b - a) / 31.0;
+    const double x = lane == 31 ? b : a + lane * step;
+    const unsigned mask = __ballot_sync(
+        0xffffffffu, sturmCount(d, e, m, x, pivmin) <= j);
+    // at most j eigenvalues below the first point, more below the last
+    if ((mask & 1u) && !(mask >> 31)) {
+      const int k = 31 - __clz(mask);
+      lo = a + k * step;
+      hi = k == 30 ? b : a + (k + 1) * step;
+    }
+  }
   for (int it = 0; it < 64; ++it) {
     if (hi - lo <= 2.0 * tol) break;
     const double step = (hi - lo) / 33.0;
     const double x = lo + (lane + 1) * step;
     const bool below =
         x > lo && x < hi && sturmCount(d, e, m, x, pivmin) <= j;
-    // the bracket is [x_k, x_{k+1}] for the last lane k whose point has at
-    // most j eigenvalues below it (the counts grow with the lane)
     const unsigned mask = __ballot_sync(0xffffffffu, below);
     const int k = mask ? 31 - __clz(mask) : -1;
     const double nlo = k >= 0 ? lo + (k + 1) * step : lo;
@@ -254,27 +387,36 @@ __device__ __forceinline__ double hashUniform(uint64_t x) {
 
 // inverse iteration for eigenvalue j: three solves of (T - w_j) z = b with
 // one LU factorisation with partial pivoting of the tridiagonal; column j of
-// Z. The factors live in column j of the scratch arrays F (5 x m x m): the
-// reciprocal pivots, the two upper diagonals of U, the multipliers and the
-// row swaps. Divisions (slow on the FP64 pipe) are made once per row in the
-// factorisation; the solves multiply.
-__global__ void invIterKernel(const double *d, const double *e, int m,
-                              const double *w, double *Z, double *F) {
+// Z. The factors are the reciprocal pivots, the two upper diagonals of U, the
+// multipliers and the row swaps, in shared memory (kSmem) or in column j of the
+// scratch arrays F (5 x m x m). One lane runs the recurrences, bound by their
+// FP64 chain: divisions (slow on the FP64 pipe) are made once per row in the
+// factorisation, the solves multiply, and the warp fills and scales the
+// vector. With the factors in global memory m = 160 took 325 us, in shared
+// memory 250.
+template <bool kSmem>
+__global__ void __launch_bounds__(32)
+    invIterKernel(const double *d, const double *e, int m, const double *w,
+                  double *Z, double *F) {
+  extern __shared__ double lu[];
   // one eigenvalue per block (its FP64 chain on an SM of its own)
-  const int j = blockIdx.x;
-  if (j >= m || threadIdx.x != 0) return;
-  const size_t mm = (size_t)m * m;
-  double *rb = F + (size_t)j * m, *c = F + mm + (size_t)j * m,
-         *u2 = F + 2 * mm + (size_t)j * m, *l = F + 3 * mm + (size_t)j * m,
-         *sw = F + 4 * mm + (size_t)j * m;
-  double *z = Z + (size_t)j * m;
+  const int j = blockIdx.x, lane = threadIdx.x;
+  if (j >= m) return;
+  const size_t st = kSmem ? (size_t)m : (size_t)m * m;
+  double *rb = kSmem ? lu : F + (size_t)j * m;
+  double *c = rb + st, *u2 = rb + 2 * st, *l = rb + 3 * st, *sw = rb + 4 * st;
+  double *z = kSmem ? lu + 5 * m : Z + (size_t)j * m;
   double scale = 0;
-  for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(d[i]));
-  for (int i = 0; i + 1 < m; ++i) scale = fmax(scale, fabs(e[i]));
+  for (int i = lane; i < m; i += 32) {
+    scale = fmax(scale, fabs(d[i]));
+    if (i + 1 < m) scale = fmax(scale, fabs(e[i]));
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
   const double eps = 2.3e-16 * fmax(scale, 1e-300);
   const double lam = w[j];
   // factorisation: row i of U is (b0, c0, u0) after elimination
-  {
+  if (lane == 0) {
     double b0 = d[0] - lam, c0 = m > 1 ? e[0] : 0.0, u0 = 0.0;
     for (int i = 0; i + 1 < m; ++i) {
       double a1 = e[i], b1 = d[i + 1] - lam, c1 = (i + 2 < m) ? e[i + 1] : 0.0;
@@ -302,96 +444,70 @@ __global__ void invIterKernel(const double *d, const double *e, int m,
     if (b0 == 0.0) b0 = eps;
     rb[m - 1] = 1.0 / b0;
   }
-  for (int i = 0; i < m; ++i)
+  for (int i = lane; i < m; i += 32)
     z[i] = hashUniform(((uint64_t)j << 32) ^ (uint64_t)i);
+  __syncwarp();
   for (int rep = 0; rep < 3; ++rep) {
-    // forward: the recorded swaps and multipliers on the right-hand side
-    double y0 = z[0];
-    for (int i = 0; i + 1 < m; ++i) {
-      double y1 = z[i + 1];
-      if (sw[i] != 0.0) {
-        const double t = y0;
-        y0 = y1;
-        y1 = t;
+    double inv = 0;
+    if (lane == 0) {
+      // forward: the recorded swaps and multipliers on the right-hand side
+      double y0 = z[0];
+      for (int i = 0; i + 1 < m; ++i) {
+        double y1 = z[i + 1];
+        if (sw[i] != 0.0) {
+          const double t = y0;
+          y0 = y1;
+          y1 = t;
+        }
+        z[i] = y0;
+        y0 = y1 - l[i] * y0;
       }
-      z[i] = y0;
-      y0 = y1 - l[i] * y0;
+      z[m - 1] = y0;
+      // back substitution
+      double nrm = 0, z1 = 0, z2 = 0;
+      for (int i = m - 1; i >= 0; --i) {
+        double sacc = z[i];
+        if (i + 1 < m) sacc -= c[i] * z1;
+        if (i + 2 < m) sacc -= u2[i] * z2;
+        z2 = z1;
+        z1 = sacc * rb[i];
+        z[i] = z1;
+        nrm += z1 * z1;
+      }
+      inv = 1.0 / sqrt(nrm);
     }
-    z[m - 1] = y0;
-    // back substitution
-    double nrm = 0;
-    for (int i = m - 1; i >= 0; --i) {
-      double sacc = z[i];
-      if (i + 1 < m) sacc -= c[i] * z[i + 1];
-      if (i + 2 < m) sacc -= u2[i] * z[i + 2];
-      z[i] = sacc * rb[i];
-      nrm += z[i] * z[i];
-    }
-    const double inv = 1.0 / sqrt(nrm);
-    for (int i = 0; i < m; ++i) z[i] *= inv;
+    inv = __shfl_sync(0xffffffffu, inv, 0);
+    __syncwarp();
+    for (int i = lane; i < m; i += 32) z[i] *= inv;
+    __syncwarp();
   }
+  if (kSmem)
+    for (int i = lane; i < m; i += 32) Z[(size_t)j * m + i] = z[i];
 }
 
-// The same multisection with the Sturm counts in double-float arithmetic
-// (heigMid): a quotient costs a few dependent FP32 operations where an FP64
-// division takes ~600 cycles on GB300. The bracket stops at 2^-44 of the
-// spectrum's scale (the double-float resolution), so the eigenvalues are good
-// to about 1e-13 relative. d, e2: the diagonal and the squared off-diagonal
-// in double-float (dfl), staged in shared memory.
-constexpr int kDfSturmMax = 512;
+// shared memory up to the default limit of 48 KB (m <= 1024)
+void inverseIteration(const double *d, const double *e, int m, const double *w,
+                      double *Z, double *F, cudaStream_t s) {
+  if (m <= 1024)
+    invIterKernel<true><<<m, 32, 6 * (size_t)m * sizeof(double), s>>>(
+        d, e, m, w, Z, F);
+  else
+    invIterKernel<false><<<m, 32, 0, s>>>(d, e, m, w, Z, F);
+}
+
+// The same multisection by the double-float counts alone (heigMid). The bracket
+// stops at 2^-44 of the spectrum's scale (the double-float resolution), so the
+// eigenvalues are good to about 1e-13 relative.
 __global__ void __launch_bounds__(32)
     multisectDfKernel(const double *d, const double *e, int m, double *w) {
   __shared__ dfl dd[kDfSturmMax], ee[kDfSturmMax];
-  const int j = blockIdx.x, lane = threadIdx.x;
+  const int j = blockIdx.x;
   if (j >= m) return;
-  double lo = 1e300, hi = -1e300, emax = 0;
-  for (int i = lane; i < m; i += 32) {
-    double r = 0;
-    if (i > 0) r += fabs(e[i - 1]);
-    if (i + 1 < m) r += fabs(e[i]);
-    lo = fmin(lo, d[i] - r);
-    hi = fmax(hi, d[i] + r);
-    dd[i] = dfFrom(d[i]);
-    if (i + 1 < m) {
-      emax = fmax(emax, fabs(e[i]));
-      const dfl ei = dfFrom(e[i]);
-      ee[i] = dfMul(ei, ei);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-  }
-  __syncwarp();
-  const double scale = fmax(fabs(lo), fabs(hi));
-  const float pivmin = (float)fmax(1e-30, 5.7e-14 * fmax(1.0, emax * emax));
-  const double tol = 5.7e-14 * scale;
-  for (int it = 0; it < 64; ++it) {
-    if (hi - lo <= 2.0 * tol) break;
-    const double step = (hi - lo) / 33.0;
-    const double x = lo + (lane + 1) * step;
-    bool below = false;
-    if (x > lo && x < hi) {
-      const dfl xd = dfFrom(x);
-      dfl q = dfSub(dd[0], xd);
-      int c = q.hi < 0.f ? 1 : 0;
-      for (int i = 1; i < m; ++i) {
-        if (fabsf(q.hi) < pivmin) q = {-pivmin, 0.f};
-        q = dfSub(dfSub(dd[i], xd), dfDiv(ee[i - 1], q));
-        if (q.hi < 0.f) ++c;
-      }
-      below = c <= j;
-    }
-    const unsigned mask = __ballot_sync(0xffffffffu, below);
-    const int k = mask ? 31 - __clz(mask) : -1;
-    const double nlo = k >= 0 ? lo + (k + 1) * step : lo;
-    const double nhi = k < 31 ? lo + (k + 2) * step : hi;
-    if (nlo == lo && nhi == hi) break;
-    lo = nlo;
-    hi = fmin(nhi, hi);
-  }
-  if (lane == 0) w[j] = 0.5 * (lo + hi);
+  double lo, hi, emax;
+  sturmBounds(d, e, m, dd, ee, lo, hi, emax);
+  sectionDf(dd, ee, m, j, (float)fmax(1e-30, 5.7e-14 * fmax(1.0, emax * emax)),
+            5.7e-14 * fmax(fabs(lo), fabs(hi)), lo, hi);
+  if (threadIdx.x == 0) w[j] = 0.5 * (lo + hi);
 }
 
 // modified Gram-Schmidt inside each cluster of equal eigenvalues (one block
@@ -542,25 +658,30 @@ __global__ void __launch_bounds__(kMidT, 1)
 }
 
 // sum over the block with two barriers: warp shuffles, then the warps'
-// partial sums (red: 32 doubles per value)
-__device__ __forceinline__ double2 blockSum2(double a, double b, double *red) {
+// partial sums (red: 32 doubles per value). Only the first n threads hold
+// values other than zero: the other warps stay off the FP64 pipe (all 16 took
+// 2.5 k cycles a sum).
+__device__ __forceinline__ double2 blockSum2(double a, double b, int n,
+                                             double *red) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  if (lane == 0) {
-    red[warp] = a;
-    red[32 + warp] = b;
+  const int nw = min((int)blockDim.x / 32, max(1, (n + 31) / 32));
+  if (warp < nw) {
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      red[warp] = a;
+      red[32 + warp] = b;
+    }
   }
   __syncthreads();
-  // one warp sums the warps' partials (FP64 work stays off the other 15
-  // warps: the FP64 pipe retires 2 operations per clock per SM)
+  // one warp sums the warps' partials (the levels above them would add zeros)
   if (warp == 0) {
-    const int nw = blockDim.x / 32;
     double ra = lane < nw ? red[lane] : 0.0;
     double rb = lane < nw ? red[32 + lane] : 0.0;
     for (int o = 16; o > 0; o >>= 1) {
+      if (o >= nw && o > 1) continue;
       ra += __shfl_xor_sync(0xffffffffu, ra, o);
       rb += __shfl_xor_sync(0xffffffffu, rb, o);
     }
@@ -609,7 +730,7 @@ __global__ void __launch_bounds__(kMidT, 1)
       const double2 xi = dfcTo(x[i]);
       loc += xi.x * xi.x + xi.y * xi.y;
     }
-    const double xn2 = blockSum2(loc, 0.0, red).x;
+    const double xn2 = blockSum2(loc, 0.0, L, red).x;
     if (tid == 0) {
       // the reflector in double-float: an FP64 square root or quotient takes
       // ~650 cycles on GB300's FP64 pipe
@@ -678,7 +799,7 @@ __global__ void __launch_bounds__(kMidT, 1)
       re += pv.x;
       im += pv.y;
     }
-    const double2 pv = blockSum2(re, im, red);
+    const double2 pv = blockSum2(re, im, L, red);
     const double2 a2 = cmulD(make_double2(-0.5 * t.x, -0.5 * t.y), pv);
     for (int i = tid; i < L; i += nt) {
       const double2 av = cmulD(a2, v64[i]);
@@ -787,11 +908,12 @@ __global__ void finishKernel(int m, int *perm, int *status) {
 size_t heigLargeScratchBytes(int m) {
   const size_t mm = (size_t)m * m;
   return 2 * mm * sizeof(double2)                // A, Vr
-         + (size_t)kJC * m * sizeof(double2)     // P
+         + (size_t)m * sizeof(double2)           // P
          + (size_t)m * sizeof(double2)           // Wv
          + (size_t)m * sizeof(double2)           // tau
          + 2 * (size_t)m * sizeof(double)        // d, e
-         + 6 * mm * sizeof(double) + 1024;       // Z, F (5)
+         + 6 * mm * sizeof(double)               // Z, F (5)
+         + 10 * 256;                             // counters, alignment
 }
 
 // w ascending, V eigenvectors (m x m, column-major); scratch holds
@@ -807,27 +929,29 @@ void heigLarge(const double2 *Ain, int lda, int m, double2 *V, double *w,
   };
   double2 *A = reinterpret_cast<double2 *>(take(mm * sizeof(double2)));
   double2 *Vr = reinterpret_cast<double2 *>(take(mm * sizeof(double2)));
-  double2 *P = reinterpret_cast<double2 *>(take((size_t)kJC * m * sizeof(double2)));
+  double2 *P = reinterpret_cast<double2 *>(take(m * sizeof(double2)));
   double2 *Wv = reinterpret_cast<double2 *>(take(m * sizeof(double2)));
   double2 *tau = reinterpret_cast<double2 *>(take(m * sizeof(double2)));
   double *d = reinterpret_cast<double *>(take(m * sizeof(double)));
   double *e = reinterpret_cast<double *>(take(m * sizeof(double)));
   double *Z = reinterpret_cast<double *>(take(mm * sizeof(double)));
   double *F = reinterpret_cast<double *>(take(5 * mm * sizeof(double)));
+  unsigned *counter = reinterpret_cast<unsigned *>(take(2 * sizeof(unsigned)));
   const unsigned gm = (unsigned)((mm + kT - 1) / kT);
   fullCopyKernel<<<gm, kT, 0, s>>>(Ain, lda, m, A);
-  for (int k = 0; k + 1 < m; ++k) {
+  cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned), s);
+  hhFirstKernel<<<1, kT, 0, s>>>(A, m, Vr, tau, d, e);
+  // the last reflector (L = 1) only makes e[m-2] real
+  for (int k = 0; k + 2 < m; ++k) {
     const int L = m - k - 1;
-    hhVectorKernel<<<1, kT, 0, s>>>(A, m, k, Vr, tau, d, e);
-    if (L < 2) continue; // the last reflector only makes e[m-2] real
-    hhMatvecKernel<<<dim3((L + 127) / 128, kJC), 128, 0, s>>>(A, m, k, Vr, P);
-    hhWKernel<<<1, kT, 0, s>>>(m, k, P, Vr, tau, Wv);
-    hhUpdateKernel<<<dim3((L + 127) / 128, L), 128, 0, s>>>(A, m, k, Vr, Wv,
-                                                            tau);
+    hhMatvecKernel<<<(L + kT / 32 - 1) / (kT / 32), kT, 0, s>>>(
+        A, m, k, Vr, tau, P, Wv, counter);
+    hhUpdateKernel<<<dim3((L + kT / 2 - 1) / (kT / 2), (L + 1) / 2), kT, 0,
+                     s>>>(A, m, k, Vr, Wv, tau, d, e, counter + 1);
   }
   lastDiagKernel<<<1, 32, 0, s>>>(A, m, d);
   multisectKernel<<<m, 32, 0, s>>>(d, e, m, w);
-  invIterKernel<<<m, 32, 0, s>>>(d, e, m, w, Z, F);
+  inverseIteration(d, e, m, w, Z, F, s);
   clusterMgsKernel<<<m, kT, 0, s>>>(w, m, Z);
   btColumnsKernel<<<(m + kBtWarps - 1) / kBtWarps, 32 * kBtWarps,
                     kBtWarps * (size_t)m * sizeof(double2), s>>>(Z, m, Vr, tau,
@@ -894,7 +1018,7 @@ void heigMid(const double2 *Ain, int lda, int m, double2 *V, double *w,
     multisectKernel<<<m, 32, 0, s>>>(d, e, m, w);
   else
     multisectDfKernel<<<m, 32, 0, s>>>(d, e, m, w);
-  invIterKernel<<<m, 32, 0, s>>>(d, e, m, w, Z, F);
+  inverseIteration(d, e, m, w, Z, F, s);
   clusterMgsKernel<<<m, kT, 0, s>>>(w, m, Z);
   if (heigMidFp64())
     btColumnsKernel<<<(m + kBtWarps - 1) / kBtWarps, 32 * kBtWarps,
