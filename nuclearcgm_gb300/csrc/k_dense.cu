@@ -574,7 +574,7 @@ __device__ __forceinline__ double divBy(double a, double b, double r) {
 // x_i = s_i / R_ii, then s_k -= R_ki x_i for all k < i at once. Bound by the
 // chain of one FP64 step (64 cycles an operation) per row; the columns of R
 // come four steps ahead by asynchronous copies. One thread per column with a
-// dot product per element ran m^2 / 2 such steps: m = 192 5860 -> 180 us, m = 60
+// dot product per element ran m^2 / 2 such steps: m = 192 5860 -> 190 us, m = 60
 // about 250 -> 39 us. Dropped rows stay zero. T starts as zero.
 // Without kStaged (columns too long for shared memory) R is read and T's
 // column built where they are.
@@ -619,12 +619,22 @@ __global__ void __launch_bounds__(32)
     if (r != 0.0) {
       const double2 b = sv[i];
       x = make_double2(divBy(b.x, rii, r), divBy(b.y, rii, r));
-      for (int k = lane; k < i; k += 32) {
-        const double2 a = col[k];
-        double2 v = sv[k];
-        v.x = fma(a.y, x.y, fma(-a.x, x.x, v.x));
-        v.y = fma(-a.y, x.x, fma(-a.x, x.y, v.y));
-        sv[k] = v;
+      // three rows of a lane at a time: their chains overlap
+      for (int k = lane; k < i; k += 96) {
+        double2 v[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + 32 * u < i) v[u] = sv[k + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + 32 * u < i) {
+            const double2 a = col[k + 32 * u];
+            v[u].x = fma(a.y, x.y, fma(-a.x, x.x, v[u].x));
+            v[u].y = fma(-a.y, x.x, fma(-a.x, x.y, v[u].y));
+          }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (k + 32 * u < i) sv[k + 32 * u] = v[u];
       }
     }
     __syncwarp();
@@ -831,10 +841,12 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
 }
 
 // Large m (> 80): the same right-looking factorisation in global memory with
-// one launch pair per column (pivot and row scaling in one block, the rank-1
-// update of the trailing triangle over the whole GPU), then T = R^{-1}
-// (cholInvKernel). G's diagonal (drop floor) and the pivots are kept in
-// T's first 2m entries until T is computed.
+// one launch per column: the rank-1 update of the trailing triangle over the
+// whole GPU, whose last block to finish takes the next pivot and scales its
+// row (m = 192: 5.1 us a column; a pivot launch of its own took 4.4 us beside
+// the update's 2.2 and a gap), then T = R^{-1} (cholInvKernel). G's diagonal (drop floor), the pivots
+// and the arrival counter are kept in T's first 2m + 1 entries until T is
+// computed.
 __global__ void cholCopyKernel(const double2 *G, int ldg, int m, double2 *R,
                                double2 *T) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -844,24 +856,28 @@ __global__ void cholCopyKernel(const double2 *G, int ldg, int m, double2 *R,
   R[e] = g;
   if (row == col) T[row] = make_double2(g.x, 0.0);
 }
-__global__ void cholPivotKernel(double2 *R, int m, int j, double dropTol,
-                                double2 *T, int *keep) {
-  __shared__ double piv;
+// pivot j and its row (one block). Other blocks of the same launch may have
+// written R: it is read past L1.
+__device__ void cholPivot(double2 *R, int m, int j, double dropTol, double2 *T,
+                          int *keep) {
+  __shared__ double rjjS, rinvS;
   if (threadIdx.x == 0) {
-    const double d = R[(size_t)j * m + j].x;
+    const double d = __ldcg(R + (size_t)j * m + j).x;
     const double floor =
         fmax(dropTol, 64.0 * 2.220446049250313e-16 * T[j].x);
     const int k = (d > floor) ? 1 : 0;
     keep[j] = k;
-    piv = k ? d : 0.0;
-    T[m + j] = make_double2(piv, 0.0);
+    T[m + j] = make_double2(k ? d : 0.0, 0.0);
+    rjjS = k ? sqrt(d) : 0.0;
+    rinvS = k ? 1.0 / rjjS : 0.0;
   }
   __syncthreads();
-  if (piv > 0.0) {
-    const double rjj = sqrt(piv);
+  const double rjj = rjjS, rinv = rinvS;
+  if (rjj > 0.0) {
     for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) {
-      const double2 a = R[(size_t)i * m + j];
-      R[(size_t)i * m + j] = make_double2(a.x / rjj, a.y / rjj);
+      const double2 a = __ldcg(R + (size_t)i * m + j);
+      R[(size_t)i * m + j] =
+          make_double2(divBy(a.x, rjj, rinv), divBy(a.y, rjj, rinv));
     }
     if (threadIdx.x == 0) R[(size_t)j * m + j] = make_double2(rjj, 0.0);
   } else {
@@ -869,15 +885,33 @@ __global__ void cholPivotKernel(double2 *R, int m, int j, double dropTol,
       R[(size_t)i * m + j] = make_double2(0, 0);
   }
 }
-__global__ void cholUpdateKernel(double2 *R, int m, int j, const double2 *T) {
-  if (T[m + j].x <= 0.0) return;
+__global__ void cholFirstKernel(double2 *R, int m, double dropTol, double2 *T,
+                                int *keep) {
+  if (threadIdx.x == 0) T[2 * m] = make_double2(0.0, 0.0); // no arrivals yet
+  cholPivot(R, m, 0, dropTol, T, keep);
+}
+__global__ void cholUpdateKernel(double2 *R, int m, int j, double dropTol,
+                                 double2 *T, int *keep) {
   const int a = j + 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int b = j + 1 + blockIdx.y;
-  if (a >= m || a > b) return;
-  const double2 t = cconjmul(R[(size_t)a * m + j], R[(size_t)b * m + j]);
-  double2 &x = R[(size_t)b * m + a];
-  x.x -= t.x;
-  x.y -= t.y;
+  if (T[m + j].x > 0.0 && a < m && a <= b) {
+    const double2 t = cconjmul(R[(size_t)a * m + j], R[(size_t)b * m + j]);
+    double2 &x = R[(size_t)b * m + a];
+    x.x -= t.x;
+    x.y -= t.y;
+  }
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned *counter = reinterpret_cast<unsigned *>(T + 2 * m);
+    last = atomicAdd(counter, 1u) == gridDim.x * gridDim.y - 1;
+    if (last) *counter = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  cholPivot(R, m, j + 1, dropTol, T, keep);
 }
 __global__ void cholFinishKernel(double2 *R, int m, double2 *T) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -905,11 +939,11 @@ void cholDrop(const double2 *G, int ldg, int m, double dropTol, double2 *R,
   if (m > kCholSmemMax) {
     const unsigned gm = (unsigned)(((size_t)m * m + 255) / 256);
     cholCopyKernel<<<gm, 256, 0, s>>>(G, ldg, m, R, T);
-    for (int j = 0; j < m; ++j) {
-      cholPivotKernel<<<1, 128, 0, s>>>(R, m, j, dropTol, T, keep);
+    cholFirstKernel<<<1, 128, 0, s>>>(R, m, dropTol, T, keep);
+    for (int j = 0; j + 1 < m; ++j) {
       const int w = m - j - 1;
-      if (w > 0)
-        cholUpdateKernel<<<dim3((w + 127) / 128, w), 128, 0, s>>>(R, m, j, T);
+      cholUpdateKernel<<<dim3((w + 127) / 128, w), 128, 0, s>>>(
+          R, m, j, dropTol, T, keep);
     }
     cholFinishKernel<<<gm, 256, 0, s>>>(R, m, T);
     cholInverse(R, m, keep, T, s);
