@@ -406,10 +406,11 @@ int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C, int k,
  * lower triangle read; m <= 1024): w ascending, V the eigenvectors in the
  * same order. This is the projected eigenproblem of the GCG's Rayleigh-Ritz
  * step (the reference's SelfAdjointEigenSolver on the lower triangle,
- * src/solver/solver.cpp:766-777) and of the HFB step. m <= 80: one-CTA
- * Jacobi in shared memory (NCGM_FP64: FP64 rotations; NCGM_FP32 and
- * NCGM_FP32_TC: double-float rotations); m > 80: Householder
- * tridiagonalisation, bisection and inverse iteration over the whole GPU.
+ * src/solver/solver.cpp:766-777) and of the HFB step. NCGM_FP64: one-CTA
+ * Jacobi below m = 48, a double-float stage with FP64 refinement up to 80;
+ * NCGM_FP32 and NCGM_FP32_TC: one-CTA double-float Householder method up to
+ * 112; above these sizes Householder tridiagonalisation, multisection and
+ * inverse iteration over the whole GPU.
  * Host or device pointers. */
 int ncgm_heig(ncgm_ctx *ctx, const double *A, int m, double *w, double *V,
               int precision);
