@@ -683,6 +683,7 @@ __global__ void cholDropDfKernel(const double2 *G, int ldg, int m,
   __shared__ int kp[kCholSmemMax];
   __shared__ double gd[kCholSmemMax]; // the Gram diagonal (drop floor)
   __shared__ dfl rinv[kCholSmemMax];
+  __shared__ dfl rjj;
   __shared__ int pivOk;
   const int tid = threadIdx.x, nt = blockDim.x;
   const dfc zero = {{0.f, 0.f}, {0.f, 0.f}};
@@ -700,19 +701,19 @@ __global__ void cholDropDfKernel(const double2 *G, int ldg, int m,
           fmax(dropTol, 64.0 * 2.220446049250313e-16 * gd[j]);
       pivOk = (d > floor) ? 1 : 0;
       kp[j] = pivOk;
+      if (pivOk) { // one thread: it overwrites the pivot below
+        rjj = dfSqrt(A[(size_t)j * m + j].re);
+        rinv[j] = dfDiv(dfl{1.f, 0.f}, rjj);
+      }
     }
     __syncthreads();
     if (pivOk) {
-      const dfl sq = dfSqrt(A[(size_t)j * m + j].re);
-      const dfl inv = dfDiv(dfl{1.f, 0.f}, sq);
+      const dfl inv = rinv[j];
       for (int i = j + 1 + tid; i < m; i += nt) {
         dfc &a = A[(size_t)i * m + j];
         a = {dfMul(a.re, inv), dfMul(a.im, inv)};
       }
-      if (tid == 0) {
-        A[(size_t)j * m + j] = {sq, {0.f, 0.f}};
-        rinv[j] = inv;
-      }
+      if (tid == 0) A[(size_t)j * m + j] = {rjj, {0.f, 0.f}};
       __syncthreads();
       const int w = m - j - 1;
       for (int e = tid; e < w * (w + 1) / 2; e += nt) {
