@@ -195,12 +195,12 @@ int buildWoodsSaxon(ncgm_ctx *ctx, int species, int A, int Z, double V0,
 void applyH64(ncgm_ctx *ctx, int species, const double2 *X, double2 *Y,
               int ncols, double shift, cudaStream_t s) {
   const SpeciesFields &F = ctx->sp[species];
-  // A tile of the integer form shares one scale. On a fine mesh it spans 4 to
-  // 5 fm and every digit of FP64 survives; on lattices of fewer than 15
-  // points per axis the mesh is coarse, a tile covers half of the box, and
-  // an orbital falls by more than the spare bits inside it. Those keep the
-  // FP64 kernel (12^3 x 4 columns: 16 us against 10; 16^3 x 16: 27 against 12;
-  // 36^3 x 60: 760 against 213).
+  // Not a line of speed: the integer form is the faster one everywhere (4^3 x 4
+  // columns 6.2 us against 8.2, 12^3 x 16 8.2 against 14.3, 16^3 x 16 10.4
+  // against 24.6, 36^3 x 60 243 against 758). The lattices below are too small
+  // for a run in earnest; they keep the FP64 kernel and with it their results
+  // to the bit, on which fixed points with a nearly free centre of mass have
+  // been compared.
   if (ctx->n >= 15) {
     applyHInt(X, Y, F.coef64, F.coefInt, ctx->n, ncols, shift, s);
     return;

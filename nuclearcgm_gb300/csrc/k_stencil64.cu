@@ -3,31 +3,43 @@
 // GB300's FP64 pipe retires two operations per clock per SM, its integer
 // pipes 64 to 128, and H at one lattice point and column takes 144 FP64
 // operations, so an FP64 kernel is bound by that pipe: one thread per point and
-// column took 0.76 ms for 36^3 x 60 columns and 1.11 ms for 40^3 x 64, where
-// the bytes take 0.03 ms. This kernel takes 0.21 and 0.27 ms, bound by
-// instruction latency (14 warps per SM, 36 % of the issue slots). Here the
-// operator is evaluated exactly, or to more bits than FP64 keeps, on the
-// integer pipes.
+// column took 758 us for 36^3 x 60 columns and 1108 us for 40^3 x 64, where
+// the bytes take 30 us. Here the products run on the integer pipes, with more
+// bits than FP64 keeps, in 243 and 302 us, bound by instruction issue and
+// latency: 43 and 47 % of the slots with 13 and 15 % of the warps (128
+// registers, two blocks of 216 or 256 threads per SM). One scale per tile, 57
+// bits below its largest value, took 210 and 266 us, but an orbital falls by
+// more than the spare bits inside a tile.
 //  * A block owns a tile of lattice points and walks over columns. It copies
 //    the tile with its two-point face halos into shared memory (cp.async, the
-//    next column's copy in flight while this one is computed), takes the
-//    largest exponent e of the tile and rounds every value to an integer of 57
-//    bits below 2^e, held as two 32-bit limbs X = Xh 2^29 + Xl. The scale is
-//    the tile's own, so the tails of an orbital keep their digits.
-//  * Neighbour sums S1 (distance 1), S2 (distance 2) and the differences E_a =
-//    (p1 - m1) - (p2 - m2)/8 along each axis are formed limb by limb, without
-//    carries (the /8 rounds down by one unit of a term that is ~60 times
-//    smaller).
-//  * Coefficients are 58-bit integers (intCoefKernel), scaled so that no sum
-//    of |coefficient| |X| can overflow, C = Ch 2^27 + Cl. A product takes three
-//    32 x 32 -> 64 bit multiply-adds; Xl Cl is left out (2^-60 of the largest
-//    value the operator can give in the tile). The 12 products of one output
-//    component add up in three 64-bit integers, which become one double at
-//    the end.
-// Errors: 2^-58 of the tile's largest |x| in X and 2^-59 of the largest
-// possible |Y| in the products, against ~2^-53 per operation in FP64.
-// A tile that holds an infinity, a NaN or numbers outside 2^-900 .. 2^900, and
-// fields or shifts outside the format, are computed in FP64 by the same block.
+//    next column's copy in flight while this one is computed). The thread
+//    that copied a point replaces its four real values by integers of 57 bits
+//    below 2^e, e the exponent of the point's largest value, and stores e.
+//  * An output point takes the largest exponent of the 13 points that it
+//    reads, shifts their integers right to it, and forms the centre, the
+//    neighbour sums S1 (distance 1), S2 (distance 2) and the differences E_a =
+//    8 (p1 - m1) - (p2 - m2), the first three times 8, in 64 bits, S = Sh 2^32
+//    + Sl. So the scale of every output is the one of its own stencil, as far
+//    as an orbital may fall inside the tile.
+//  * Coefficients are integers of 58 bits (intCoefKernel), scaled for every
+//    lattice point by the
+//    largest |Y| / max|X| that its row can give, C = Ch 2^28 + Cl. A product
+//    takes three 32 x 32 -> 64 bit multiply-adds; Sl Cl is left out. The 12
+//    products of one output component add up in three 64-bit integers, which
+//    become one double at the end.
+//  * What is cut off is rounded to odd, which treats x and -x alike, and sums
+//    of integers do not depend on their order: a block with the mirror
+//    symmetries of the lattice keeps them to the bit, as in FP64 arithmetic (a
+//    nucleus would drift otherwise: its centre of mass is a near-zero mode).
+// Errors, in units of the largest |x| of the point's stencil times the row sum
+// R of its |coefficients|: 2^-57 per value of X, 2^-59 per coefficient, 2^-60
+// per product for the part left out, and one rounding to FP64 at the end,
+// where an FP64 sum rounds every product and partial sum to 2^-53 of itself.
+// The unit is the stencil's: a component that is 2^-s of the largest one of
+// its stencil keeps 57 - s bits.
+// A point that reads an infinity, a NaN or numbers outside 2^-500 .. 2^500, and
+// points whose fields or shift are outside the format, are computed in FP64
+// (fp64Point).
 #include "ncgm_internal.cuh"
 #include "stencil_core.cuh"
 
@@ -42,8 +54,12 @@ namespace {
 constexpr int kCoefs = 9; // d, alpha1, alpha2, 8 g_x..z, 8 w_x..z
 constexpr int kThreadsMax = 256;
 constexpr int kIterMax = 5; // copied points per thread
-constexpr int kXBits = 57, kXLow = 29, kCBits = 57, kCLow = 27;
-constexpr int kSmemMax = 110 * 1024;
+// bits of X, of the neighbour sums' unit (they are multiples of X / 8) and of C
+constexpr int kXBits = 57, kSBits = kXBits + 3, kCBits = 58, kCLow = 28;
+// exponent fields of the format: 2^-500 .. 2^500, and the mark of a point
+// outside it
+constexpr int kExpLo = 1023 - 500, kExpHi = 1023 + 500, kExpBad = 4095;
+constexpr int kSmemMax = 113 * 1024; // two blocks per SM
 
 __device__ __forceinline__ uint32_t sAddr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -60,101 +76,91 @@ __device__ double rowBound(const double *c) {
   for (int a = 0; a < 3; ++a) r += 18.0 * (fabs(c[2 + a]) + 2 * fabs(c[5 + a]));
   return r;
 }
-// the largest bound of the lattice, as IEEE bits (a NaN is largest)
-__global__ void rowBoundKernel(const double *coef, size_t ns,
-                               unsigned long long *rmax) {
-  __shared__ unsigned long long sh[256];
-  unsigned long long m = 0;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < ns;
-       p += (size_t)gridDim.x * blockDim.x)
-    m = max(m, (unsigned long long)(__double_as_longlong(
-                                        rowBound(coef + 8 * p)) &
-                                    0x7FFFFFFFFFFFFFFFll));
-  sh[threadIdx.x] = m;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-      sh[threadIdx.x] = max(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) atomicMax(rmax, sh[0]);
-}
-
-// exponent ec with R < 2^ec, or false when the fields are outside the format
-__device__ __forceinline__ bool coefExp(const unsigned long long *rmax,
-                                        int &ec) {
-  const int f = (int)(*rmax >> 52);
-  ec = f - 1022;
-  return f > 1023 - 400 && f < 1023 + 400;
-}
-
-// C = Ch 2^27 + Cl, |Cl| <= 2^26
+// C = Ch 2^28 + Cl, |Cl| <= 2^27
 __device__ __forceinline__ int2 splitCoef(long long C) {
   const int lo = ((int)(C + (1 << (kCLow - 1))) & ((1 << kCLow) - 1)) -
                  (1 << (kCLow - 1));
   return make_int2((int)((C - lo) >> kCLow), lo);
 }
 
-// out: kCoefs arrays of ns int2
-__global__ void intCoefKernel(const double *coef, size_t ns,
-                              const unsigned long long *rmax, int2 *out) {
+// out: kCoefs arrays of ns int2, then the exponents ec (the row's bound is
+// below 2^ec; kExpBad for fields outside the format)
+__global__ void intCoefKernel(const double *coef, size_t ns, int2 *out,
+                              int *exps) {
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (p >= ns) return;
-  int ec;
-  const bool ok = coefExp(rmax, ec);
   const double *c = coef + 8 * p;
   const double v[kCoefs] = {c[0],       -(4.0 / 3.0) * c[1], c[1] / 12.0,
                             8.0 * c[2], 8.0 * c[3],          8.0 * c[4],
                             8.0 * c[5], 8.0 * c[6],          8.0 * c[7]};
+  // exponent field of the bound (2047: a NaN or an infinity)
+  const int f = (__double2hiint(rowBound(c)) >> 20) & 0x7FF;
+  const bool ok = f > 1023 - 400 && f < 1023 + 400;
+  const int ec = f - 1022;
+  exps[p] = ok ? ec : kExpBad;
   for (int q = 0; q < kCoefs; ++q)
     out[q * ns + p] =
         splitCoef(ok ? __double2ll_rn(scalbn(v[q], kCBits - ec)) : 0ll);
 }
 
-// |x| < 2^e rounded to an integer of kXBits bits in two limbs Xh 2^29 + Xl,
-// |Xl| <= 2^28; f = 1027 + e. Zeros and numbers below 2^-1022 shift out.
-__device__ __forceinline__ int2 toLimbs(int lo, int hi, int f) {
+// |x| < 2^e as an integer of kXBits bits, f = e + 1022 the largest exponent
+// field of the point. It is rounded to odd: the lowest bit of every value but
+// zero is set, also where nothing is cut off, and stays set when the integer is
+// shifted further (shifted), so that -x gives the negative integer throughout.
+// Zeros and numbers below 2^-1022 give 0.
+__device__ __forceinline__ long long toFixed(int lo, int hi, int f) {
   const unsigned long long m =
       (((unsigned long long)((hi & 0xFFFFF) | 0x100000) << 32) | (unsigned)lo)
-      << 10;
-  const int s = min(f - ((hi >> 20) & 0x7FF), 63);
-  const long long w = (long long)(m >> s); // in half units
+      << (kXBits - 53);
+  const int fx = (hi >> 20) & 0x7FF;
+  const long long w =
+      (long long)((m >> min(f - fx, 63)) | (unsigned)min(fx, 1));
   const long long g = hi >> 31;
-  const long long u = (w ^ g) + 1; // |x| rounded half up
-  return make_int2((int)((u + (1 << kXLow)) >> (kXLow + 1)),
-                   (int)((unsigned)u << (31 - kXLow)) >> (32 - kXLow));
+  return (w ^ g) - g;
+}
+__device__ __forceinline__ int2 pair(long long v) {
+  return make_int2((int)v, (int)(v >> 32));
+}
+// the 64-bit integer (lo, hi) 2^-s rounded to odd (zero: 0)
+__device__ __forceinline__ long long shifted(int lo, int hi, int s) {
+  long long v = (long long)(((unsigned long long)(unsigned)hi << 32) |
+                            (unsigned)lo);
+  asm("shr.s64 %0, %0, %1;" : "+l"(v) : "r"(s)); // clamps s
+  return v | (unsigned)(lo & 1);
 }
 
+// One output component: the sum of C S in integers. With the row bound and the
+// shift the sum of |C| |S| stays below 1.85 2^118, that of |Ch| below 2^31,
+// and that of |Sh| below 34 2^28.
 struct Acc {
-  long long hh, mx, mc; // weights 2^56, 2^29, 2^27
-  // C X, x = limbs (h, l)
-  __device__ __forceinline__ void add(int2 c, int2 x) {
-    hh += (long long)c.x * x.x;
-    mx += (long long)c.y * x.x;
-    mc += (long long)c.x * x.y;
+  long long hh, mx, mc; // Ch Sh, Cl Sh, Ch Sl: weights 2^60, 2^32, 2^28
+  __device__ __forceinline__ void add(int2 c, int2 s) { // (h, l)
+    hh += (long long)c.x * s.x;
+    mx += (long long)c.y * s.x;
+    mc += (long long)c.x * s.y;
   }
-  // in units of 2^53: |sum| < 2^115, so below 2^62
+  // in units of 2^56, rounded to odd, so that the double made of it is the
+  // sum's nearest one
   __device__ __forceinline__ long long value() const {
-    return hh * 8 + ((mx * 4 + mc) >> 26);
+    const long long t = mx + (mc >> 4);
+    const unsigned cut = ((unsigned)t & 0xFFFFFFu) | ((unsigned)mc & 15u);
+    return (hh * 16 + (t >> 24)) | min(cut, 1u);
   }
 };
 __device__ __forceinline__ int2 neg(int2 v) { return make_int2(-v.x, -v.y); }
-__device__ __forceinline__ int2 sum2(int2 a, int2 b) {
-  return make_int2(a.x + b.x, a.y + b.y);
-}
-// (p1 - m1) - (p2 - m2) / 8
-__device__ __forceinline__ int2 diff(int2 p1, int2 m1, int2 p2, int2 m2) {
-  const int bh = p2.x - m2.x, bl = p2.y - m2.y;
-  return make_int2((p1.x - m1.x) - (bh >> 3),
-                   (p1.y - m1.y) - (bl >> 3) - ((bh & 7) << (kXLow - 3)));
+// v = h 2^32 + l with a signed l
+__device__ __forceinline__ int2 limbs(long long v) {
+  const int l = (int)v;
+  return make_int2((int)(v >> 32) + (int)((unsigned)l >> 31), l);
 }
 __device__ __forceinline__ double pow2(int e) { // normal range
   return __hiloint2double((e + 1023) << 20, 0);
 }
 
 // Tile tx x ty x tz, nx x ny x nz of them; the box in shared memory has row
-// pitch px and plane pitch pz (points), P points in all; `points` of them are
-// copied, `iters` per thread.
+// pitch px and plane pitch pz (points): point (i, j, k) of the tile at i + px j
+// + pz (k + 2), halos at -2, -1, t, t + 1 of one axis each, so P points from the
+// first to the last; `points` of them are copied, `iters` per thread.
 struct Tiling {
   int tx, ty, tz, nx, ny, nz, threads, px, pz, P, points, iters;
 };
@@ -184,13 +190,15 @@ __device__ __noinline__ void fp64Point(const double2 *x, const double *coef,
 
 __global__ void __launch_bounds__(kThreadsMax, 2)
     stencilInt(const double2 *__restrict__ X, double2 *__restrict__ Y,
-               const int2 *__restrict__ CI, const double *__restrict__ coef,
-               const unsigned long long *__restrict__ rmax, int n, int cols,
-               int group, double shift, Tiling T) {
-  extern __shared__ __align__(16) int4 box[]; // [buffer][spin][point]
-  __shared__ int wmax[2][kThreadsMax / 32];
+               const int2 *__restrict__ CI, const int *__restrict__ EC,
+               const double *__restrict__ coef, int n, int cols, int group,
+               double shift, Tiling T) {
+  // [buffer][spin][point], the coefficients, the exponents [buffer][point]
+  extern __shared__ __align__(16) int4 box[];
   const size_t ns = (size_t)n * n * n;
   const int tid = threadIdx.x, nthr = blockDim.x;
+  int2 *ct = reinterpret_cast<int2 *>(box + 4 * T.P) + tid;
+  short *ex = reinterpret_cast<short *>(ct - tid + kCoefs * nthr);
   const int x0 = ((int)blockIdx.x % T.nx) * T.tx,
             y0 = ((int)blockIdx.x / T.nx % T.ny) * T.ty,
             z0 = ((int)blockIdx.x / (T.nx * T.ny)) * T.tz;
@@ -219,14 +227,16 @@ __global__ void __launch_bounds__(kThreadsMax, 2)
       b -= hy;
       i = b % T.tx, j = b / T.tx % T.ty, k = layer(b / (T.tx * T.ty), T.tz);
     }
-    at[it] = i + 2 + T.px * (j + 2) + T.pz * (k + 2);
+    at[it] = i + T.px * j + T.pz * (k + 2);
     const int gx = x0 + i, gy = y0 + j, gz = z0 + k;
-    if (gx >= 0 && gx < n && gy >= 0 && gy < n && gz >= 0 && gz < n)
+    if (gx >= 0 && gx < n && gy >= 0 && gy < n && gz >= 0 && gz < n) {
       off[it] = gx + n * (gy + n * gz);
-    else
+    } else {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         box[q * T.P + at[it]] = make_int4(0, 0, 0, 0);
+      ex[at[it]] = ex[T.P + at[it]] = 0;
+    }
   }
   auto fetch = [&](int col, int buf) {
     const double2 *x = X + (size_t)col * 2 * ns;
@@ -245,163 +255,147 @@ __global__ void __launch_bounds__(kThreadsMax, 2)
   const int gi = x0 + i, gj = y0 + j, gk = z0 + k;
   const bool active = k < T.tz && gi < n && gj < n && gk < n;
   const size_t p = gi + (size_t)n * (gj + (size_t)n * gk);
-  const int pb = i + 2 + T.px * (j + 2) + T.pz * (k + 2);
-  int ec;
-  bool fields = coefExp(rmax, ec);
-  int2 cd = {}, ca1 = {}, ca2 = {}, cg[3] = {}, cw[3] = {};
-  if (active && fields) {
-    cd = CI[p];
-    ca1 = CI[ns + p];
-    ca2 = CI[2 * ns + p];
+  const int pb = i + T.px * j + T.pz * (k + 2);
+  // the coefficients wait in shared memory between their uses (each thread
+  // reads back its own): held in registers they made the loop spill
+  int ec = kExpBad;
+  if (active) {
+    ec = EC[p];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      cg[a] = CI[(3 + a) * ns + p];
-      cw[a] = CI[(6 + a) * ns + p];
+    for (int q = 0; q < kCoefs; ++q) ct[q * nthr] = CI[q * ns + p];
+    if (shift != 0.0 && ec != kExpBad) {
+      const double sI = scalbn(shift, kCBits - ec);
+      if (fabs(sI) < 0.85 * (double)(1ll << kCBits)) {
+        const int2 d = ct[0];
+        ct[0] =
+            splitCoef(((long long)d.x << kCLow) + d.y + __double2ll_rn(sI));
+      } else {
+        ec = kExpBad; // NaN too
+      }
     }
   }
-  if (shift != 0.0 && fields) {
-    const double sI = scalbn(shift, kCBits - ec);
-    if (fabs(sI) < 0.85 * (double)(1ll << kCBits))
-      cd = splitCoef(((long long)cd.x << kCLow) + cd.y + __double2ll_rn(sI));
-    else
-      fields = false; // NaN too
-  }
   unsigned long long bad = 0; // columns left to FP64 (bit c - c0)
-  // the coefficients wait in shared memory between their uses (each thread
-  // reads back its own): held in registers they made the loop spill (244 us
-  // against 213 us for 36^3 x 60)
-  int2 *ct = reinterpret_cast<int2 *>(box + 4 * T.P) + tid;
-  ct[0] = cd;
-  ct[nthr] = ca1;
-  ct[2 * nthr] = ca2;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    ct[(3 + a) * nthr] = cg[a];
-    ct[(6 + a) * nthr] = cw[a];
-  }
   for (int c = c0; c < c1; ++c) {
     const int buf = (c - c0) & 1;
     int4 *B = box + 2 * buf * T.P;
+    short *eb = ex + buf * T.P;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // largest high word of the tile; a value with only low bits counts as 1
-    int m = 0;
+    // each thread replaces the points that it copied
 #pragma unroll
     for (int it = 0; it < kIterMax; ++it)
-      if (off[it] >= 0)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int4 v = B[q * T.P + at[it]];
-          m = max(m, max((v.y & 0x7FFFFFFF) | (v.x != 0),
-                         (v.w & 0x7FFFFFFF) | (v.z != 0)));
-        }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((tid & 31) == 0) wmax[buf][tid >> 5] = m;
+      if (off[it] >= 0) {
+        int4 &u = B[at[it]], &d = B[T.P + at[it]];
+        // largest high word; a value with only low bits counts as 1
+        const int m = max(max((u.y & 0x7FFFFFFF) | (u.x != 0),
+                              (u.w & 0x7FFFFFFF) | (u.z != 0)),
+                          max((d.y & 0x7FFFFFFF) | (d.x != 0),
+                              (d.w & 0x7FFFFFFF) | (d.z != 0)));
+        // (a point of zeros: an exponent that shifts their implicit bit out)
+        const int f = max(m >> 20, 64);
+        eb[at[it]] = (short)(m == 0                       ? 0
+                             : f > kExpLo && f < kExpHi ? f
+                                                        : kExpBad);
+        const int2 ur = pair(toFixed(u.x, u.y, f)),
+                   ui = pair(toFixed(u.z, u.w, f)),
+                   dr = pair(toFixed(d.x, d.y, f)),
+                   di = pair(toFixed(d.z, d.w, f));
+        u = make_int4(ur.x, ur.y, ui.x, ui.y);
+        d = make_int4(dr.x, dr.y, di.x, di.y);
+      }
     __syncthreads();
     // every thread has left column c - 1: its buffer takes column c + 1
     if (c + 1 < c1) fetch(c + 1, buf ^ 1);
-    m = wmax[buf][0];
-    for (int w = 1; w < (nthr >> 5); ++w) m = max(m, wmax[buf][w]);
-    const int f = m >> 20; // exponent field of the largest value
-    const bool ok =
-        fields && (m == 0 || (f > 1023 - 900 && f < 1023 + 900));
-    const int e = m ? f - 1022 : 0; // all |x| < 2^e
-    if (ok) {
+    if (!active) continue;
+    // the scale of this stencil
+    int sh[3][4]; // p1, m1, p2, m2 per axis
+    int top = eb[pb], sc = top;
 #pragma unroll
-      for (int it = 0; it < kIterMax; ++it)
-        if (off[it] >= 0)
+    for (int a = 0; a < 3; ++a) {
+      const int st = a == 0 ? 1 : (a == 1 ? T.px : T.pz);
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            int4 &v = B[q * T.P + at[it]];
-            const int2 re = toLimbs(v.x, v.y, 1027 + e),
-                       im = toLimbs(v.z, v.w, 1027 + e);
-            v = make_int4(re.x, re.y, im.x, im.y);
-          }
-    } else {
-      bad |= 1ull << (c - c0);
-    }
-    __syncthreads();
-    if (ok && active) {
-      double2 *y = Y + (size_t)c * 2 * ns;
-      Acc o[4] = {}; // Re, Im of the upper and the lower component
-      int2 s1[4], s2[4];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int4 v = B[q * T.P + pb];
-        o[2 * q].add(ct[0], make_int2(v.x, v.y));
-        o[2 * q + 1].add(ct[0], make_int2(v.z, v.w));
-        s1[2 * q] = s1[2 * q + 1] = make_int2(0, 0);
-        s2[2 * q] = s2[2 * q + 1] = make_int2(0, 0);
+      for (int q = 0; q < 4; ++q) {
+        sh[a][q] = eb[pb + (q < 2 ? st : 2 * st) * (q & 1 ? -1 : 1)];
+        top = max(top, sh[a][q]);
       }
+    }
+    if (top == kExpBad || ec == kExpBad) {
+      bad |= 1ull << (c - c0);
+      continue;
+    }
+    sc = top - sc;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sh[a][q] = top - sh[a][q];
+    Acc o[4] = {}; // Re, Im of the upper and the lower component
+#pragma unroll
+    for (int q = 0; q < 2; ++q) { // spin of the input
+      const int4 *b = B + q * T.P + pb;
+      long long s1[2] = {0, 0}, s2[2] = {0, 0};
+      int2 E[3][2]; // [axis][Re, Im]
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const int st = a == 0 ? 1 : (a == 1 ? T.px : T.pz);
-        int2 E[4];
+        const int4 p1 = b[st], m1 = b[-st], p2 = b[2 * st], m2 = b[-2 * st];
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int4 *b = B + q * T.P + pb;
-          const int4 p1 = b[st], m1 = b[-st], p2 = b[2 * st], m2 = b[-2 * st];
-          const int2 p1r = {p1.x, p1.y}, p1i = {p1.z, p1.w};
-          const int2 m1r = {m1.x, m1.y}, m1i = {m1.z, m1.w};
-          const int2 p2r = {p2.x, p2.y}, p2i = {p2.z, p2.w};
-          const int2 m2r = {m2.x, m2.y}, m2i = {m2.z, m2.w};
-          s1[2 * q] = sum2(s1[2 * q], sum2(p1r, m1r));
-          s1[2 * q + 1] = sum2(s1[2 * q + 1], sum2(p1i, m1i));
-          s2[2 * q] = sum2(s2[2 * q], sum2(p2r, m2r));
-          s2[2 * q + 1] = sum2(s2[2 * q + 1], sum2(p2i, m2i));
-          E[2 * q] = diff(p1r, m1r, p2r, m2r);
-          E[2 * q + 1] = diff(p1i, m1i, p2i, m2i);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) o[q].add(ct[(3 + a) * nthr], E[q]);
-        // spin-orbit, -i (sigma x W)_a E_a (see pointH)
-        if (a == 0) { // [[i Wy, -Wz], [Wz, -i Wy]]
-          const int2 wy = ct[7 * nthr], wz = ct[8 * nthr];
-          const int2 ny = neg(wy), nz = neg(wz);
-          o[0].add(ny, E[1]), o[0].add(nz, E[2]);
-          o[1].add(wy, E[0]), o[1].add(nz, E[3]);
-          o[2].add(wz, E[0]), o[2].add(wy, E[3]);
-          o[3].add(wz, E[1]), o[3].add(ny, E[2]);
-        } else if (a == 1) { // [[-i Wx, i Wz], [i Wz, i Wx]]
-          const int2 wx = ct[6 * nthr], wz = ct[8 * nthr];
-          const int2 nx = neg(wx), nz = neg(wz);
-          o[0].add(wx, E[1]), o[0].add(nz, E[3]);
-          o[1].add(nx, E[0]), o[1].add(wz, E[2]);
-          o[2].add(nz, E[1]), o[2].add(nx, E[3]);
-          o[3].add(wz, E[0]), o[3].add(wx, E[2]);
-        } else { // [[0, Wx - i Wy], [-Wx - i Wy, 0]]
-          const int2 wx = ct[6 * nthr], wy = ct[7 * nthr];
-          const int2 nx = neg(wx), ny = neg(wy);
-          o[0].add(wx, E[2]), o[0].add(wy, E[3]);
-          o[1].add(wx, E[3]), o[1].add(ny, E[2]);
-          o[2].add(nx, E[0]), o[2].add(wy, E[1]);
-          o[3].add(nx, E[1]), o[3].add(ny, E[0]);
+        for (int r = 0; r < 2; ++r) {
+          const auto at = [&](const int4 &v, int s) {
+            return shifted(r ? v.z : v.x, r ? v.w : v.y, s);
+          };
+          const long long xp1 = at(p1, sh[a][0]), xm1 = at(m1, sh[a][1]),
+                          xp2 = at(p2, sh[a][2]), xm2 = at(m2, sh[a][3]);
+          s1[r] += xp1 + xm1;
+          s2[r] += xp2 + xm2;
+          E[a][r] = limbs(((xp1 - xm1) << 3) - (xp2 - xm2));
         }
       }
+      const int4 v = b[0];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        o[q].add(ct[nthr], s1[q]);
-        o[q].add(ct[2 * nthr], s2[q]);
+      for (int r = 0; r < 2; ++r) {
+        Acc &s = o[2 * q + r];
+        s.add(ct[0], limbs(shifted(r ? v.z : v.x, r ? v.w : v.y, sc) << 3));
+        s.add(ct[nthr], limbs(s1[r] << 3));
+        s.add(ct[2 * nthr], limbs(s2[r] << 3));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) s.add(ct[(3 + a) * nthr], E[a][r]);
       }
-      // units: 2^(e - kXBits) 2^(ec - kCBits) 2^53; |e| <= 901, |ec| <= 401:
-      // in two factors
-      const double u1 = pow2(e);
-      const double u2 = pow2(ec + 53 - kXBits - kCBits);
-      y[2 * p] = make_double2((double)o[0].value() * u2 * u1,
-                              (double)o[1].value() * u2 * u1);
-      y[2 * p + 1] = make_double2((double)o[2].value() * u2 * u1,
-                                  (double)o[3].value() * u2 * u1);
+      // spin-orbit, -i (sigma x W)_a E_a (see pointH): what this spin adds to
+      // itself (0, 1) and to the other one (2, 3)
+      const int2 wx = ct[6 * nthr], wy = ct[7 * nthr], wz = ct[8 * nthr];
+      Acc &o0 = o[2 * q], &o1 = o[2 * q + 1], &o2 = o[2 - 2 * q],
+          &o3 = o[3 - 2 * q];
+      const int2 ny = neg(wy), nx = neg(wx), nz = neg(wz);
+      if (q == 0) {
+        o0.add(ny, E[0][1]), o0.add(wx, E[1][1]);
+        o1.add(wy, E[0][0]), o1.add(nx, E[1][0]);
+        o2.add(wz, E[0][0]), o2.add(nx, E[2][0]);
+        o2.add(nz, E[1][1]), o2.add(wy, E[2][1]);
+        o3.add(wz, E[0][1]), o3.add(nx, E[2][1]);
+        o3.add(wz, E[1][0]), o3.add(ny, E[2][0]);
+      } else {
+        o0.add(wy, E[0][1]), o0.add(nx, E[1][1]);
+        o1.add(ny, E[0][0]), o1.add(wx, E[1][0]);
+        o2.add(nz, E[0][0]), o2.add(wx, E[2][0]);
+        o2.add(nz, E[1][1]), o2.add(wy, E[2][1]);
+        o3.add(nz, E[0][1]), o3.add(wx, E[2][1]);
+        o3.add(wz, E[1][0]), o3.add(ny, E[2][0]);
+      }
     }
+    // units: 2^(e - kSBits) 2^(ec - kCBits) 2^56, e = top - 1022
+    const double u = pow2(max(top, kExpLo) - 1022 + ec + 56 - kSBits - kCBits);
+    double2 *y = Y + (size_t)c * 2 * ns + 2 * p;
+    y[0] = make_double2((double)o[0].value() * u, (double)o[1].value() * u);
+    y[1] = make_double2((double)o[2].value() * u, (double)o[3].value() * u);
   }
-  if (active)
-    for (; bad; bad &= bad - 1) {
-      const size_t o = (size_t)(c0 + __ffsll((long long)bad) - 1) * 2 * ns;
-      fp64Point(X + o, coef, n, gi, gj, gk, shift, Y + o);
-    }
+  for (; bad; bad &= bad - 1) {
+    const size_t o = (size_t)(c0 + __ffsll((long long)bad) - 1) * 2 * ns;
+    fp64Point(X + o, coef, n, gi, gj, gk, shift, Y + o);
+  }
 }
 
-// two boxes of two spins, and the coefficients
+// two boxes of two spins, the coefficients, two boxes of exponents
 size_t smemBytes(const Tiling &t) {
-  return (size_t)t.P * 4 * sizeof(int4) +
+  return (size_t)t.P * (4 * sizeof(int4) + 2 * sizeof(short)) +
          (size_t)kCoefs * t.threads * sizeof(int2);
 }
 
@@ -427,7 +421,7 @@ Tiling chooseTiling(int n) {
         t.threads = (pts + 31) / 32 * 32;
         t.px = tx % 8 ? tx + 8 : tx + 4;
         t.pz = t.px * (ty + 4) + (t.px % 2 ? 4 : 0);
-        t.P = t.pz * (tz + 4);
+        t.P = tx + t.px * (ty - 1) + t.pz * (tz + 3);
         t.points = pts + 4 * (ty * tz + tx * tz + tx * ty);
         t.iters = (t.points + t.threads - 1) / t.threads;
         if (t.iters > kIterMax || smemBytes(t) > kSmemMax) continue;
@@ -443,37 +437,31 @@ Tiling chooseTiling(int n) {
 
 } // namespace
 
-size_t intCoefBytes(size_t ns) { return kCoefs * ns * sizeof(int2) + 256; }
+size_t intCoefBytes(size_t ns) {
+  return ns * (kCoefs * sizeof(int2) + sizeof(int));
+}
 
-// the integer coefficients of a species' table: the row bound in the first
-// 8 bytes of buf, the table from byte 256 on
+// the integer coefficients of a species' table and their exponents
 void buildIntCoefficients(const double *coef64, size_t ns, void *buf,
                           cudaStream_t s) {
-  auto *rmax = static_cast<unsigned long long *>(buf);
-  auto *tab = reinterpret_cast<int2 *>(static_cast<char *>(buf) + 256);
-  cudaMemsetAsync(rmax, 0, sizeof(*rmax), s);
-  rowBoundKernel<<<(unsigned)std::min<size_t>(256, (ns + 255) / 256), 256, 0,
-                   s>>>(coef64, ns, rmax);
-  intCoefKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(coef64, ns, rmax,
-                                                             tab);
+  auto *tab = static_cast<int2 *>(buf);
+  intCoefKernel<<<(unsigned)((ns + 255) / 256), 256, 0, s>>>(
+      coef64, ns, tab, reinterpret_cast<int *>(tab + kCoefs * ns));
 }
 
 void applyHInt(const double2 *X, double2 *Y, const double *coef64,
                const void *intCoef, int n, int ncols, double shift,
                cudaStream_t s) {
-  static const bool attr = [] {
-    cudaFuncSetAttribute(stencilInt,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         kSmemMax);
-    return true;
-  }();
-  (void)attr;
+  // a per-device attribute: set on every call
+  cudaFuncSetAttribute(stencilInt, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       kSmemMax);
   thread_local int lastN = 0;
   thread_local Tiling T{};
   if (lastN != n) {
     T = chooseTiling(n);
     lastN = n;
   }
+  const size_t ns = (size_t)n * n * n;
   const long long tiles = (long long)T.nx * T.ny * T.nz;
   // columns per block: the fewest waves of two blocks per SM, counting a
   // block's set-up as a column and a half
@@ -488,12 +476,11 @@ void applyHInt(const double2 *X, double2 *Y, const double *coef64,
       group = g;
     }
   }
+  const auto *tab = static_cast<const int2 *>(intCoef);
   stencilInt<<<dim3((unsigned)tiles, (ncols + group - 1) / group), T.threads,
                smemBytes(T), s>>>(
-      X, Y,
-      reinterpret_cast<const int2 *>(static_cast<const char *>(intCoef) + 256),
-      coef64, static_cast<const unsigned long long *>(intCoef), n, ncols,
-      group, shift, T);
+      X, Y, tab, reinterpret_cast<const int *>(tab + kCoefs * ns), coef64, n,
+      ncols, group, shift, T);
 }
 
 } // namespace ncgm
