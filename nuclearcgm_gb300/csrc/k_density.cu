@@ -54,10 +54,30 @@ __device__ __forceinline__ double d2(const double *v, size_t base,
 
 // First-derivative weights a_1 .. a_4 of f(+k) - f(-k) for the central rules
 // of order 2, 4, 6 and 8 (rows 1 .. 4) and the two-point rule of a box face
-// (row 0, where the missing neighbour is the point itself), over h
-struct DerivWeights {
-  double a[5][4];
+// (row 0, where the missing neighbour is the point itself), times 840 / 1024:
+// exact in FP64. The factor 1024 / (840 h) of a derivative is left to the
+// densities: one rounding each, where weights over h would put the rounding of
+// every weight on all points alike.
+__constant__ double kDerivWeights[5][4] = {
+    {840. / 1024, 0, 0, 0},
+    {420. / 1024, 0, 0, 0},
+    {560. / 1024, -70. / 1024, 0, 0},
+    {630. / 1024, -126. / 1024, 14. / 1024, 0},
+    {672. / 1024, -168. / 1024, 32. / 1024, -3. / 1024}};
+
+// c = 1024 / (840 h) and c^2 with what their rounding cut off
+struct DerivScale {
+  double one, oneLo, two, twoLo;
 };
+DerivScale derivScale(double h) {
+  const double d = 840.0 * h, dLo = std::fma(840.0, h, -d);
+  DerivScale s;
+  s.one = 1024.0 / d;
+  s.oneLo = (std::fma(-s.one, d, 1024.0) - s.one * dLo) / d;
+  s.two = s.one * s.one;
+  s.twoLo = std::fma(s.one, s.one, -s.two) + 2.0 * s.one * s.oneLo;
+  return s;
+}
 
 // NaN test on the bits (a comparison would take a slot of the FP64 pipe)
 __device__ __forceinline__ bool nanBits(double x) {
@@ -65,36 +85,38 @@ __device__ __forceinline__ bool nanBits(double x) {
          0x7FF0000000000000ll;
 }
 
-// s + Im(a^H sigma_nu b) of two spinors
+// Im(a^H sigma_nu b) of two spinors
 template <int nu>
-__device__ __forceinline__ double spinIm(double s, double2 a0, double2 a1,
-                                         double2 b0, double2 b1) {
+__device__ __forceinline__ double spinIm(double2 a0, double2 a1, double2 b0,
+                                         double2 b1) {
   if (nu == 0)
-    return fma(a0.x, b1.y,
-               fma(-a0.y, b1.x, fma(a1.x, b0.y, fma(-a1.y, b0.x, s))));
+    return fma(a0.x, b1.y, fma(-a0.y, b1.x, fma(a1.x, b0.y, -a1.y * b0.x)));
   if (nu == 1)
-    return fma(-a0.x, b1.x,
-               fma(-a0.y, b1.y, fma(a1.x, b0.x, fma(a1.y, b0.y, s))));
-  return fma(a0.x, b0.y,
-             fma(-a0.y, b0.x, fma(-a1.x, b1.y, fma(a1.y, b1.x, s))));
+    return fma(-a0.x, b1.x, fma(-a0.y, b1.y, fma(a1.x, b0.x, a1.y * b0.y)));
+  return fma(a0.x, b0.y, fma(-a0.y, b0.x, fma(-a1.x, b1.y, a1.y * b1.x)));
+}
+__device__ __forceinline__ double norm2(double2 a, double s) {
+  return fma(a.x, a.x, fma(a.y, a.y, s));
 }
 
 // One thread per point, a loop over the columns. Bound by the FP64 pipe (two
-// operations per clock per SM): 160 of its operations per point and column, 96
-// for the six spinor derivatives (differences first, weights that already
-// hold 1/h) and 64 for the densities. Every point runs the same instructions:
-// rules of lower order next to the faces are zero weights, their neighbours
-// are not read. The form it replaces branched on the rule (a warp spans all of
-// them along x) and divided each derivative by its denominator: 36^3 x 20
-// columns 1110 -> 303 us. 64 threads per block: 36^3 points are then 4.8
-// blocks per SM, so the last wave costs little.
+// operations per clock per SM): 172 of its operations per point and column, 96
+// for the six spinor derivatives (differences first) and 76 for the densities,
+// which add one column's contribution at a time to the running sums: rounding
+// those once per column and not once per product halves the error (36^3 x 20
+// columns, tau: 5.3e-16 -> 1.6e-16, 12 operations and 12 % more time). Every point runs the
+// same instructions: rules of lower order next to the faces are zero weights,
+// their neighbours are not read. The form it replaces branched on the rule (a
+// warp spans all of them along x) and divided each derivative by its
+// denominator: 36^3 x 20 columns 1110 -> 339 us, 87 % of the pipe. 64 threads per block: 36^3
+// points are then 4.8 blocks per SM, so the last wave costs little.
 __global__ void __launch_bounds__(64)
     densityKernel(const double2 *__restrict__ Phi, size_t ldphi, int M, int n,
-                  DerivWeights wt, double *rho, double *tau, double *J9,
+                  DerivScale f, double *rho, double *tau, double *J9,
                   double *divJ) {
   __shared__ double ws[5][4];
   if (threadIdx.x < 20) ws[threadIdx.x / 4][threadIdx.x % 4] =
-      wt.a[threadIdx.x / 4][threadIdx.x % 4];
+      kDerivWeights[threadIdx.x / 4][threadIdx.x % 4];
   __syncthreads();
   const size_t ns = (size_t)n * n * n;
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -146,28 +168,32 @@ __global__ void __launch_bounds__(64)
       }
     }
     // density: sum_s |psi_s|^2
-    r = fma(u.x, u.x, fma(u.y, u.y, fma(d.x, d.x, fma(d.y, d.y, r))));
-    
+    r += norm2(u, norm2(d, 0.0));
+    double t0 = 0.0, t1 = 0.0;
 #pragma unroll
     for (int mu = 0; mu < 3; ++mu) {
       const double2 g0 = g[mu][0], g1 = g[mu][1];
       // kinetic density
-      t = fma(g0.x, g0.x, fma(g0.y, g0.y, fma(g1.x, g1.x, fma(g1.y, g1.y, t))));
+      t0 = norm2(g0, t0);
+      t1 = norm2(g1, t1);
       // spin-orbit density J_{mu nu} = Im(psi^H sigma_nu d_mu psi)
-      J[3 * mu] = spinIm<0>(J[3 * mu], u, d, g0, g1);
-      J[3 * mu + 1] = spinIm<1>(J[3 * mu + 1], u, d, g0, g1);
-      J[3 * mu + 2] = spinIm<2>(J[3 * mu + 2], u, d, g0, g1);
+      J[3 * mu] += spinIm<0>(u, d, g0, g1);
+      J[3 * mu + 1] += spinIm<1>(u, d, g0, g1);
+      J[3 * mu + 2] += spinIm<2>(u, d, g0, g1);
     }
+    t += t0 + t1;
     // div J: -sum eps_{mu nu la} Im(d_nu psi^H sigma_la d_mu psi); the two
     // orders of a pair are equal, so the three cyclic ones count twice
-    dj = spinIm<2>(dj, g[1][0], g[1][1], g[0][0], g[0][1]);
-    dj = spinIm<0>(dj, g[2][0], g[2][1], g[1][0], g[1][1]);
-    dj = spinIm<1>(dj, g[0][0], g[0][1], g[2][0], g[2][1]);
+    dj += spinIm<2>(g[1][0], g[1][1], g[0][0], g[0][1]) +
+          spinIm<0>(g[2][0], g[2][1], g[1][0], g[1][1]) +
+          spinIm<1>(g[0][0], g[0][1], g[2][0], g[2][1]);
   }
   rho[p] = r;
-  tau[p] = t;
-  for (int q = 0; q < 9; ++q) J9[q * ns + p] = J[q];
-  divJ[p] = -2.0 * dj;
+  tau[p] = fma(t, f.two, t * f.twoLo);
+  for (int q = 0; q < 9; ++q)
+    J9[q * ns + p] = fma(J[q], f.one, J[q] * f.oneLo);
+  dj *= -2.0;
+  divJ[p] = fma(dj, f.two, dj * f.twoLo);
 }
 
 __global__ void gradLapKernel(const double *v, int n, double h, double *g3,
@@ -404,17 +430,8 @@ void densities(const double2 *Phi, size_t ld, int M, int n, double h,
                double *rho, double *tau, double *J9, double *divJ,
                cudaStream_t s) {
   const size_t ns = (size_t)n * n * n;
-  static constexpr double rule[5][4] = {{1, 0, 0, 0},
-                                        {1, 0, 0, 0},
-                                        {8, -1, 0, 0},
-                                        {45, -9, 1, 0},
-                                        {672, -168, 32, -3}};
-  static constexpr double den[5] = {1, 2, 12, 60, 840};
-  DerivWeights w;
-  for (int o = 0; o < 5; ++o)
-    for (int k = 0; k < 4; ++k) w.a[o][k] = rule[o][k] / (den[o] * h);
   densityKernel<<<(unsigned)((ns + 63) / 64), 64, 0, s>>>(
-      Phi, ld, M, n, w, rho, tau, J9, divJ);
+      Phi, ld, M, n, derivScale(h), rho, tau, J9, divJ);
 }
 
 void gradLap(const double *v, int n, double h, double *g3, double *lap,
