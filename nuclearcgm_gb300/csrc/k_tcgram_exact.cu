@@ -6,41 +6,51 @@
 // 2p, column 2c = Re A_c, 2c + 1 = Im A_c) and T (N x 2q, same for B). Every
 // column c of S and T is scaled by a power of two 2^-e_c that brings its
 // entries into [-1, 1] (e_c from the column's max-abs, exact), and each
-// scaled value is written as a sum of kDig signed 7-bit integer digits,
-//   x 2^-e = sum_t a_t 2^(-7t),  |a_1| <= 128, |a_t| <= 64 (t > 1),
-// all exactly representable in BF16. A product of two digits is an integer
-// below 2^14; the MMAs of one "level" l = t + u (pairs with the same scale
-// 2^(-7l)) accumulate in FP32 tensor memory over 256 rows, so every partial
-// sum is an integer below 2^24 and the FP32 accumulation is exact. After each
-// 256-row block the levels are combined exactly in 64-bit integers (held in
-// registers over at most 16 blocks); the chunks' integers are added in 128
-// bits and rounded to FP64 once.
-// Levels above kDig + 1 are dropped: the truncation error is ~2^(-7 kDig) of
-// the column max per element. 6 digits (the tensor-core precision form) give
-// ~2e-13 relative; 8 digits hold all 53 bits of every entry above 2^-4 of its
-// column's maximum, and the product is then as accurate as an FP64 sum or
-// better: against 113-bit sums, 2 36^3 rows, 60 columns of orbitals and
-// corrections 1000 times smaller, the Gram is off by 2.4e-17 rms (1.3e-16 at
-// most) of |a||b| where the FP64 kernel is off by 1.5e-16 (9.8e-16), and V C
-// by 1.2e-16 of |y| where it is off by 3.0e-16.
+// scaled value is rounded to an integer and written as a sum of kDig signed
+// digits (Fmt),
+//   x 2^(kBits-e) = sum_t a_t 2^(kBase (kDig-1-t)),  t = 0 .. kDig-1,
+// all exactly representable in BF16: 6 digits of 7 bits (42 bits, the
+// tensor-core precision form) or 8 digits of 8 bits (62 bits, the FP64 form).
+// A product of two digits is an integer of at most 2^14; the MMAs of one
+// "level" l = t + u (pairs with the same scale) accumulate in FP32 tensor
+// memory over 256 (6 digits) or 128 rows (8), so every partial sum is an
+// integer of at most 2^24 and the FP32 accumulation is exact. After each such
+// block the levels are combined exactly in integers (64 bits, and 32 more for
+// the low part with 8 digits, held in registers over at most 4096 rows); the
+// chunks' integers are added in 128 bits and rounded to FP64 once. Levels from
+// kDig on are left out.
+//
+// Errors: 6 digits give ~2e-13 of the column maxima. 8 digits hold a value to
+// 2^-63 of its column's largest entry (V of Y = V C: of its row's largest, the
+// columns scaled), nine bits below FP64's own 53: values down to 2^-9 of it
+// keep all their bits, smaller ones lose what FP64 would keep of them. What is
+// left out is about 2^-59 of the maxima per V C element. With the one rounding
+// that is less than an FP64 sum loses. Against 113-bit sums, 2 36^3 rows (FP64
+// kernel; 8 digits of 7 bits): Gram of orbitals x and x + 1e-10 d 4.3e-17 rms
+// of |a||b| (3.1e-16; 3.2e-16), its pairs of parallel columns 7.4e-17 at most
+// (6.5e-16; 1.6e-15: the products left out have one sign there); V C, m = 60,
+// 4.7e-17 of |Y| for a random C (2.7e-16; 1.0e-16) and 4.8e-17 for a nearly
+// triangular one (6.9e-17; 1.6e-16).
 //
 // What bounds it: GB300's FP64 pipe retires two operations per clock per SM,
 // so the FP64 kernels take 4.25 ms (Gram) and 3.66 ms (V C) at 2 36^3 x 60,
-// m = k = 60; the 36 digit products run on the tensor cores in 0.28 and
-// 0.45 ms. The digit images (16 bytes per real value) go through L2.
+// m = k = 60; the 36 digit products take 0.23 and 0.30 ms, of which the MMA
+// kernels 0.13 and 0.21 (tensor pipe 37 and 23 % active): the copies of 96 KB
+// a slab from L2 through two stages and the folds. Digitising takes 0.07 and
+// 0.06 ms (DRAM 51 and 57 %).
 //
 // Two passes per product:
 //  1. A digitising kernel writes each operand's digits once, as the exact
 //     K-major core-matrix image of the 128 x 32 BF16 tiles that the MMAs
-//     read (48 KB per tile, kDig planes). It runs at full occupancy, so the
-//     integer work of the splitting hides the memory latency.
-//  2. The MMA kernel streams those tiles into shared memory with 16-byte
-//     cp.async copies through a three-stage ring: the copies of slab s + 2
-//     are in flight while the tensor cores work on slab s. One thread issues
-//     the MMAs (tile M = 128, N = 64, instruction K = 16, two per slab per
-//     digit pair) and commits them to the stage's mbarrier; after every 8
-//     slabs all warps fold the level accumulators (tcgen05.ld) into their
-//     64-bit sums. Every wait is bounded.
+//     read (48 or 64 KB per tile, kDig planes). It runs at full occupancy, so
+//     the integer work of the splitting hides the memory latency.
+//  2. The MMA kernel streams those tiles into shared memory with bulk copies
+//     through a ring of three (6 digits) or two stages: the copies of the next
+//     slabs are in flight while the tensor cores work on this one. One thread
+//     issues copies and MMAs (tile M = 128, N = 64 per digit plane, instruction
+//     K = 16, two per slab and run of digit planes) and commits them to the
+//     stage's mbarrier; after every kFold slabs all warps fold the level
+//     accumulators (tcgen05.ld) into their integer sums. Every wait is bounded.
 #include "ncgm_internal.cuh"
 
 #include <cuda_bf16.h>
@@ -56,19 +66,24 @@ namespace {
 
 constexpr int kM = 128, kN = 64;         // D tile
 constexpr int kSlab = 32;                // K rows per stage (2 MMAs of K 16)
-constexpr int kFold = 8;                 // slabs per exact accumulation block
-constexpr int kMaxFolds = 16;            // fold blocks per 64-bit sum
+constexpr int kBlkRows = 256;            // row chunks are multiples of this
+constexpr int kMaxBlks = 16;             // and at most so many of them
 constexpr int kThr = 256;
 constexpr int kABytes = kM * kSlab * 2;  // one digit plane of A: 8 KB
 constexpr int kBBytes = kN * kSlab * 2;  // one digit plane of B: 4 KB
 constexpr uint32_t kLBO = 128, kSBO = 512;       // 8 rows x 16 B cores; K 32
 constexpr uint32_t kTmemCols = 512; // kDig levels x kN = 384 or 512
 
-// sizes of a digit format of kDig digits per value: 6 (42 bits, the
-// tensor-core precision form) or 8 (56 bits, the FP64 form)
+// A digit format of kDig digits per value: 6 of 7 bits (42 bits, the
+// tensor-core precision form) or 8 of 8 bits (62 bits, the FP64 form). The
+// level sums of kFold slabs stay integers of at most 2^24 (FP32 exact).
 template <int kDig> struct Fmt {
   static_assert(kDig == 6 || kDig == 8, "digit formats");
-  static constexpr int kBits = 7 * kDig;
+  static constexpr int kBase = kDig == 6 ? 7 : 8;
+  static constexpr int kBits = kDig == 6 ? 42 : 62;
+  static constexpr int kFold = kDig == 6 ? 8 : 4; // slabs per exact block
+  // the sum of all levels, in units of the last one: 2^(eA + eB + kUnit)
+  static constexpr int kUnit = kBase * (kDig - 1) - 2 * kBits;
   // a digitised 128 x 32 tile: 48 / 64 KB; one stage (A tile and the 64
   // columns of B): 72 / 96 KB, so 3 / 2 stages fit the 227 KB of an SM
   static constexpr int kTile = kDig * kABytes;
@@ -127,30 +142,31 @@ __device__ __forceinline__ bool waitSpin(uint64_t *bar, uint32_t phase) {
 }
 
 // digits of a scaled value: w = round(x 2^(kBits-e)), |w| <= 2^kBits, written
-// as sum_t a_t 2^(kBits-7t) with |a_1| <= 128 and |a_t| <= 64, by integer
-// rounding divisions (exact; the digits are integers, exact in BF16). One
-// 64-bit rounding split w = h 2^S + l (S = kBits / 2, |l| <= 2^(S-1)) leaves
-// 32-bit work: half of the digits from each part, and 32-bit
-// integer-to-float conversions (the 64-bit conversion runs on the slow FP64
-// pipe).
+// as sum_t a_t 2^(kBase (kDig-1-t)) by integer rounding divisions (exact; the
+// digits are integers, exact in BF16): |a_t| <= 2^(kBase-1), and |a_1| <= 128
+// (6 digits) or 64 (8). One 64-bit rounding split w = h 2^S + l (S = kBase
+// kDig / 2, |l| <= 2^(S-1)) leaves 32-bit work: half of the digits from each
+// part, and 32-bit integer-to-float conversions (the 64-bit conversion runs
+// on the slow FP64 pipe).
 template <int kDig>
 __device__ __forceinline__ void digits(long long w, float (&d)[kDig]) {
-  constexpr int H = kDig / 2, S = 7 * H;
+  constexpr int H = kDig / 2, B = Fmt<kDig>::kBase, S = B * H;
   const long long hh = (w + (1ll << (S - 1))) >> S;
-  int l = (int)(w - (hh << S));
-  int h = (int)hh;
+  unsigned l = (unsigned)(w - (hh << S));
+  unsigned h = (unsigned)hh;
 #pragma unroll
   for (int t = 0; t < H - 1; ++t) {
-    const int sh = 7 * (H - 1 - t);
-    const int a = (h + (1 << (sh - 1))) >> sh;
+    const int sh = B * (H - 1 - t);
+    // (x >> (sh - 1)) + 1 >> 1: no overflow next to 2^31
+    const int a = (((int)h >> (sh - 1)) + 1) >> 1;
     d[t] = (float)a;
-    h -= a << sh;
-    const int b = (l + (1 << (sh - 1))) >> sh;
+    h -= (unsigned)a << sh;
+    const int b = (((int)l >> (sh - 1)) + 1) >> 1;
     d[H + t] = (float)b;
-    l -= b << sh;
+    l -= (unsigned)b << sh;
   }
-  d[H - 1] = (float)h;
-  d[kDig - 1] = (float)l;
+  d[H - 1] = (float)(int)h;
+  d[kDig - 1] = (float)(int)l;
 }
 
 // w = round(x 2^(kBits - e)) for |x| < 2^e, from the bits of x with integer
@@ -222,6 +238,7 @@ __global__ void colMaxKernel(const double2 *X, size_t ld, int p, size_t N,
 }
 // exponent field of 2^900 and 2^-900 (bias 1023)
 constexpr int kExpHi = 1023 + 900, kExpLo = 1023 - 900;
+constexpr int kExpZero = -4000; // scale of a column of zeros
 __device__ __forceinline__ bool expOutside(double x) {
   const int f = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
   return f > kExpHi || (f < kExpLo && x != 0.0);
@@ -231,7 +248,9 @@ __global__ void colExpKernel(int cols, double *sc, int *exq, int *flag) {
   if (c >= cols) return;
   const double m = sc[c]; // the bit pattern written by colMaxKernel
   if (flag && expOutside(m)) *flag = 1;
-  int e = 0;
+  // a column of zeros: far below all others, so that its coefficients do not
+  // count in the scale of C
+  int e = kExpZero;
   if (m > 0) frexp(m, &e); // m < 2^e
   sc[c] = ldexp(1.0, e);   // column scale: entries / sc in (-1, 1)
   exq[c] = e;
@@ -271,17 +290,12 @@ __device__ __forceinline__ uint4 packRow(const float (*d)[kDig], int t) {
 // Thread (complex column cc of the tile, 8-row group kq) loads 8 consecutive
 // entries (4 lanes read 512 contiguous bytes) and writes one 16-byte core
 // row per digit for Re (tile row 2 cc) and Im (2 cc + 1). Rows past N and
-// columns past p are zero digits. sq (8 digits, the Gram of a block with
-// itself): the products of level 8, the first one that the MMAs leave out,
-// of every real column with itself. Between different columns those products
-// have random signs; in a column's square the term a_4^2 does not, and left
-// out it would put 2e-15 on the diagonal of a block of narrow peaks.
+// columns past p are zero digits.
 template <int kDig>
 __global__ void __launch_bounds__(256)
     digitizeGramKernel(const double2 *__restrict__ X, size_t ld, int p,
                        size_t N, const int *__restrict__ ex, int nslab,
-                       unsigned char *__restrict__ img, const int *flag,
-                       unsigned long long *__restrict__ sq) {
+                       unsigned char *__restrict__ img, const int *flag) {
   constexpr int kTile = Fmt<kDig>::kTile;
   if (flag && *flag) return;
   const int s = blockIdx.x, mt = blockIdx.y;
@@ -307,20 +321,6 @@ __global__ void __launch_bounds__(256)
     for (int t = 0; t < kDig; ++t)
       *reinterpret_cast<uint4 *>(base + (size_t)t * kABytes + o) =
           packRow<kDig>(d, t);
-    if (kDig == 8 && sq) {
-      // level 8 of the column's square, in integers below 2^18
-      float m = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        m += d[i][4] * d[i][4] +
-             2.f * (d[i][1] * d[i][7] + d[i][2] * d[i][6] +
-                    d[i][3] * d[i][5]);
-      int k = __float2int_rn(m);
-      k += __shfl_xor_sync(0xffffffffu, k, 1);
-      k += __shfl_xor_sync(0xffffffffu, k, 2);
-      if (kq == 0 && c < p)
-        atomicAdd(sq + 2 * c + part, (unsigned long long)(long long)k);
-    }
   }
 }
 
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256)
 // The same image with 8 digits and a power-of-two scale per lattice row on
 // top of the column scales (eR[r]: the row's entries, column-scaled, lie
 // below 2^eR), so that a row far from the nucleus, where every orbital is
-// small, keeps its own 56 bits as FP64 would. One block per 128-row tile:
+// small, keeps 62 bits of its own. One block per 128-row tile:
 // the threads first take the row maxima over all columns (reading the tile
 // from memory), then digitise slab by slab (reading it from L1 / L2).
 __global__ void __launch_bounds__(256)
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(256)
                         size_t N, const int *__restrict__ ex, int nslab,
                         unsigned char *__restrict__ img,
                         int *__restrict__ eR, const int *flag) {
-  constexpr int kDig = 8, kTile = Fmt<kDig>::kTile;
+  constexpr int kDig = 8, kTile = Fmt<kDig>::kTile, kBits = Fmt<kDig>::kBits;
   __shared__ int emax[2][kM];
   if (*flag) return;
   const int mt = blockIdx.x;
@@ -422,10 +422,10 @@ __global__ void __launch_bounds__(256)
       for (int i = 0; i < 4; ++i) {
         const bool in = c0 + i < m;
         digits<kDig>(
-            scaledInt<56>(v[i].x, em + (in ? ex[2 * (c0 + i)] : 0)),
+            scaledInt<kBits>(v[i].x, em + (in ? ex[2 * (c0 + i)] : 0)),
             d[2 * i]);
         digits<kDig>(
-            scaledInt<56>(v[i].y, em + (in ? ex[2 * (c0 + i) + 1] : 0)),
+            scaledInt<kBits>(v[i].y, em + (in ? ex[2 * (c0 + i) + 1] : 0)),
             d[2 * i + 1]);
       }
       const uint32_t o = off16(row, 8 * kq);
@@ -459,9 +459,10 @@ __device__ __forceinline__ void mmaIssue(uint32_t td, uint64_t ad,
 // one MMA with A digit t writes the levels t + u0 .. t + u1 into their
 // adjacent 64-column blocks of tensor memory: per 16 K and with 6 digits, A
 // digit 0 takes B digits 0-3 and 4-5, digit 1 takes 0-3 and 4, digits 2 .. 5
-// take 0 .. 5 - t (8 MMAs instead of 21; with 8 digits 12 instead of 36). aBase / bBase: shared addresses of digit
-// plane 0 of A and B. first: the slab opens a fold block (A digit 0 writes
-// every level first and overwrites). Descriptors are the plane-0
+// take 0 .. 5 - t (8 MMAs instead of 21; with 8 digits 12 instead of 36).
+// aBase / bBase: shared addresses of digit plane 0 of A and B. first: the slab
+// opens a fold block (A digit 0 writes every level first and overwrites).
+// Descriptors are the plane-0
 // descriptor plus a constant: the start-address field holds address / 16
 // and shared addresses stay below 256 KB, so the addition never carries.
 template <int kDig>
@@ -492,7 +493,7 @@ __device__ __forceinline__ void issueSlab(uint32_t taddr, uint32_t aBase,
 // 64-bit sums of TMEM lane row (lw 32 + lane), columns cBeg .. cBeg + 31:
 // sum_l L_l 2^(7 (kDig-1-l)) = (L0 2^7 + L1) 2^28 + (L2 2^7 + L3) 2^14 +
 // (L4 2^7 + L5), each pair in 32 bits (|L_l| < 2^23), the sum below 2^58.1,
-// so kMaxFolds = 16 blocks stay below 2^63. Two levels per load wait.
+// so 16 blocks of 256 rows stay below 2^63. Two levels per load wait.
 __device__ __forceinline__ void tmemLoad16(uint32_t ta, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, "
@@ -522,11 +523,12 @@ template <int kDig> struct Sums {
   __device__ double value(int j, int e) const;
   __device__ void storeLo(int *, int) const {}
 };
-// 8 digits: hi 2^14 + lo with |lo| <= 2^13. A fold adds (L0 2^7 + L1) 2^28 +
-// (L2 2^7 + L3) 2^14 + (L4 2^7 + L5) to hi and L6 2^7 + L7 to lo, whose
-// multiples of 2^14 carry into hi: every level is kept, exactly. |L_l| <=
-// 256 (2 2^13 + 6 2^12) < 2^23.4, so a pair stays below 2^30.5 in 32 bits and
-// hi below 2^58.1 per fold.
+// 8 digits: hi 2^20 + lo with |lo| <= 2^19. A fold adds (L0 2^8 + L1) 2^48 +
+// (L2 2^8 + L3) 2^32 + (L4 2^8 + L5) 2^16 + L6 2^8 + L7: every level is kept,
+// exactly. With |a_1| <= 64 and |a_t| <= 128 for the others, the products of
+// 128 rows give |L0| <= 2^19, |L1| <= 2^21, |L2| <= 2^22, |L3| < 2^23 (the
+// first two pairs fit 32 bits) and at most 7 2^21 < 2^24 for the last, so a
+// fold is below 2^75.2 and hi below 2^61.2 after 64 folds (8192 rows).
 template <> struct Sums<8> {
   long long hi[32];
   int lo[32];
@@ -657,7 +659,8 @@ __device__ __forceinline__ void Sums<8>::fold(uint32_t taddr, int lw,
   for (int h = 0; h < 4; ++h) {
     const uint32_t ta =
         taddr + ((uint32_t)(lw * 32) << 16) + (uint32_t)(cBeg + 8 * h);
-    int pr[4][8];
+    int pr[2][8];
+    long long low[2][8];
 #pragma unroll
     for (int pl = 0; pl < 4; ++pl) {
       uint32_t a[8], b[8];
@@ -665,30 +668,32 @@ __device__ __forceinline__ void Sums<8>::fold(uint32_t taddr, int lw,
       tmemLoad8(ta + (uint32_t)((2 * pl + 1) * kN), b);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        pr[pl][j] = __float2int_rn(__uint_as_float(a[j])) * 128 +
-                    __float2int_rn(__uint_as_float(b[j]));
+      for (int j = 0; j < 8; ++j) {
+        const int u = __float2int_rn(__uint_as_float(a[j])),
+                  v = __float2int_rn(__uint_as_float(b[j]));
+        if (pl < 2)
+          pr[pl][j] = u * 256 + v;
+        else
+          low[pl - 2][j] = (long long)u * 256 + v;
+      }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int t = lo[8 * h + j] + pr[3][j];
-      const int c = (t + (1 << 13)) >> 14;
-      lo[8 * h + j] = t - (c << 14);
-      hi[8 * h + j] += ((long long)pr[0][j] << 28) +
-                       ((long long)pr[1][j] << 14) + (long long)pr[2][j] +
-                       (long long)c;
+      const long long t = (low[0][j] << 16) + low[1][j] + lo[8 * h + j];
+      const long long c = (t + (1 << 19)) >> 20;
+      lo[8 * h + j] = (int)(t - (c << 20));
+      hi[8 * h + j] +=
+          ((long long)pr[0][j] << 28) + ((long long)pr[1][j] << 12) + c;
     }
   }
 }
-// rounded from all bits while hi 2^14 + lo fits 62 bits; a larger hi keeps
-// 6 bits of lo, then none: below half a unit in the last place of a double
+// rounded from the leading 62 bits of hi 2^20 + lo (all of them while hi is
+// below 2^42)
 __device__ __forceinline__ double Sums<8>::value(int j, int e) const {
-  const long long h = hi[j], a = h < 0 ? -h : h;
-  const bool some = a >= 1ll << 47, none = a >= 1ll << 55;
-  const int sh = none ? 0 : (some ? 6 : 14);
-  return scaledDoubleInt(
-      (h << sh) + (long long)(none ? 0 : (some ? lo[j] >> 8 : lo[j])),
-      e + 14 - sh);
+  const long long h = hi[j];
+  const int sh = min(max(__clzll(h ^ (h >> 63)) - 2, 0), 20);
+  return scaledDoubleInt((h << sh) + (long long)(lo[j] >> (20 - sh)),
+                         e + 20 - sh);
 }
 
 __device__ __forceinline__ void tmemAlloc(uint32_t *slot) {
@@ -831,6 +836,7 @@ __global__ void __launch_bounds__(kThr, 1)
                     int self, const int *flag, int *err) {
   constexpr int kTile = Fmt<kDig>::kTile, kBuf = Fmt<kDig>::kBuf,
                 kStages = Fmt<kDig>::kStages;
+  constexpr int kFold = Fmt<kDig>::kFold;
   extern __shared__ __align__(1024) unsigned char sm[];
   const int mt = blockIdx.x, nt = blockIdx.y, chunk = blockIdx.z;
   if (self && tileBelow(mt, nt)) return;
@@ -922,19 +928,18 @@ __global__ void __launch_bounds__(kThr, 1)
 }
 
 // Chunk partials: the exact sums as 64-bit integers (partHi) and, with 8
-// digits, their low parts (partLo; value = hi 2^14 + lo). They are added in
+// digits, their low parts (partLo; value = hi 2^20 + lo). They are added in
 // 128-bit integers and rounded once, so the result does not depend on the
 // chunking and the FP64 pipe (two operations per clock) stays out of it. The
-// real and the imaginary part each join two such sums. One warp per output element: lane l takes the chunks l,
-// l + 32, ... self: elements below the diagonal are the conjugates of those
-// above it.
+// real and the imaginary part each join two such sums. One warp per output
+// element: lane l takes the chunks l, l + 32, ... self: elements below the
+// diagonal are the conjugates of those above it.
 template <int kDig>
 __global__ void exactGramReduce(const long long *__restrict__ partHi,
                                 const int *__restrict__ partLo, int chunks,
                                 int p, int q, const int *__restrict__ eA,
                                 const int *__restrict__ eB,
                                 double2 *__restrict__ C, int ldc, int self,
-                                const long long *__restrict__ sq,
                                 const int *flag) {
   const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -955,7 +960,7 @@ __global__ void exactGramReduce(const long long *__restrict__ partHi,
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const size_t o = (size_t)ch * step + off[x];
-      t[x] += kDig == 8 ? ((__int128)partHi[o] << 14) + partLo[o]
+      t[x] += kDig == 8 ? ((__int128)partHi[o] << 20) + partLo[o]
                         : (__int128)partHi[o];
     }
 #pragma unroll
@@ -969,18 +974,11 @@ __global__ void exactGramReduce(const long long *__restrict__ partHi,
       t[x] += ((__int128)hi << 64) | (__int128)(unsigned __int128)lo;
     }
   if (lane != 0) return;
-  int unit = 7 * (kDig + 1);
-  if (kDig == 8 && self && i == j) { // with level 8 of the squares
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-      t[x] = (t[x] << 7) + (x < 2 ? sq[2 * i + x] : 0ll);
-    unit += 7;
-  }
   double v[4];
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
     const int ei = 2 * i + (x & 1), ej = 2 * j + (x == 1 || x == 2 ? 1 : 0);
-    v[x] = scaledDouble128(t[x], eA[ei] + eB[ej] - unit);
+    v[x] = scaledDouble128(t[x], eA[ei] + eB[ej] + Fmt<kDig>::kUnit);
   }
   const double re = v[0] + v[1], im = v[2] - v[3];
   if (mirror)
@@ -1052,8 +1050,9 @@ __global__ void plainVCKernel(const double2 *__restrict__ V, size_t ldv, int m,
 // of two 2^-eA (colMaxKernel); the scales move into B, whose columns are
 // scaled again by 2^-eB, and the digits of that B are precomputed once
 // (vcPrepKernel) in the shared-memory image the MMAs read. The reduction
-// (K = 2m <= 512) is a few 32-row slabs; every 8 slabs the level sums fold
-// into FP64. Each CTA owns 128 rows of Y and 64 of its 2k real columns.
+// (K = 2m <= 8192) is a few 32-row slabs; every kFold slabs the level sums fold
+// into the integer sums. Each CTA owns 128 rows of Y and 64 of its 2k real
+// columns.
 
 // digits of B = diag(2^eA) B0 2^-eB, laid out per (column tile, slab, digit)
 // as the K-major core-matrix image of one 64 x 32 BF16 plane
@@ -1137,6 +1136,7 @@ __global__ void __launch_bounds__(kThr, 1)
                   const int *flag, int *err) {
   constexpr int kTile = Fmt<kDig>::kTile, kBuf = Fmt<kDig>::kBuf,
                 kStages = Fmt<kDig>::kStages;
+  constexpr int kFold = Fmt<kDig>::kFold;
   extern __shared__ __align__(1024) unsigned char sm[];
   if (flag && *flag) return;
   Pipe<kDig> P(sm);
@@ -1202,12 +1202,12 @@ __global__ void __launch_bounds__(kThr, 1)
       P.foldDone();
       if (s == nslab - 1) {
         // Y[j][r] = (sum[2j] 2^eB[2j], sum[2j+1] 2^eB[2j+1]) 2^eR[r]
-        // 2^(-7 (kDig+1))
+        // 2^kUnit
         const int tile = (int)blockIdx.x + (i / nslab) * G;
         const int mt = tile / ntiles, nt = tile % ntiles;
         const size_t r = (size_t)mt * kM + lw * 32 + lane;
         if (r < N) {
-          const int ew = -7 * (kDig + 1) + (kDig == 8 ? eR[r] : 0);
+          const int ew = Fmt<kDig>::kUnit + (kDig == 8 ? eR[r] : 0);
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const int jr = nt * kN + cBeg + j;
@@ -1232,8 +1232,8 @@ __global__ void __launch_bounds__(kThr, 1)
   P.release(warp, taddr);
 }
 
-// rows per chunk of the Gram grid: a multiple of one fold block and at most
-// kMaxFolds blocks (the 64-bit sums), chosen to minimise the waves of one
+// rows per chunk of the Gram grid: a multiple of kBlkRows and at most kMaxBlks
+// of them (the 64-bit sums), chosen to minimise the waves of one
 // CTA per SM times the rows of a chunk (plus a fixed cost per CTA)
 int chunkRows(size_t N, int p, int q, bool self) {
   const int mts = (2 * p + kM - 1) / kM, nts = (2 * q + kN - 1) / kN;
@@ -1241,11 +1241,11 @@ int chunkRows(size_t N, int p, int q, bool self) {
   if (self)
     for (int mt = 0; mt < mts; ++mt)
       for (int nt = 0; nt < nts; ++nt) tiles -= tileBelow(mt, nt) ? 1 : 0;
-  const size_t blk = (size_t)kSlab * kFold;
+  const size_t blk = kBlkRows;
   const size_t sms = (size_t)smCount();
   size_t best = blk;
   double bestCost = 1e300;
-  for (size_t rows = blk; rows <= kMaxFolds * blk; rows += blk) {
+  for (size_t rows = blk; rows <= kMaxBlks * blk; rows += blk) {
     const size_t chunks = (N + rows - 1) / rows;
     const size_t waves = (chunks * tiles + sms - 1) / sms;
     const double cost = (double)waves * (double)(std::min(rows, N) + 2 * kSlab);
@@ -1262,8 +1262,7 @@ size_t gramImageBytes(size_t N, int p, int digits) {
   const size_t nslab = (N + kSlab - 1) / kSlab;
   return nslab * (size_t)((2 * p + kM - 1) / kM) * digits * kABytes;
 }
-// column scales (doubles) and exponents (ints) of both operands, the flag,
-// the level-8 squares
+// column scales (doubles) and exponents (ints) of both operands, the flag
 size_t gramHeaderBytes(int p, int q) {
   return ((sizeof(double) * (4 * (size_t)(p + q) + 8)) + 255) & ~(size_t)255;
 }
@@ -1288,10 +1287,6 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
   int *eB = eA + 2 * (size_t)p;
   // the FP64 form hands operands outside the digit format to plainGramKernel
   int *flag = kDig == 8 ? eB + 2 * (size_t)q : nullptr;
-  // 2p sums behind the flag (zeroed with the header)
-  auto *sq = kDig == 8 && self ? reinterpret_cast<unsigned long long *>(
-                                     scratch + 3 * (size_t)(p + q) + 1)
-                               : nullptr;
   const size_t head = gramHeaderBytes(p, q);
   unsigned char *imgA = reinterpret_cast<unsigned char *>(scratch) + head;
   unsigned char *imgB = imgA + gramImageBytes(N, p, kDig);
@@ -1303,14 +1298,14 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
   if (!self) colMax(B, ldb, q, N, scB, eB, flag, s);
   digitizeGramKernel<kDig>
       <<<dim3(nslab, (2 * p + kM - 1) / kM), 256, 0, s>>>(
-          A, lda, p, N, eA, nslab, imgA, flag, sq);
+          A, lda, p, N, eA, nslab, imgA, flag);
   if (self) {
     imgB = imgA;
     eB = eA;
   } else {
     digitizeGramKernel<kDig>
         <<<dim3(nslab, (2 * q + kM - 1) / kM), 256, 0, s>>>(
-            B, ldb, q, N, eB, nslab, imgB, flag, nullptr);
+            B, ldb, q, N, eB, nslab, imgB, flag);
   }
   const int rows = chunkRows(N, p, q, self);
   const int spc = rows / kSlab;
@@ -1323,7 +1318,7 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
   exactGramReduce<kDig>
       <<<(unsigned)(((size_t)p * q * 32 + 255) / 256), 256, 0, s>>>(
           partHi, partLo, chunks, p, q, eA, eB, C, ldc, self ? 1 : 0,
-          reinterpret_cast<const long long *>(sq), flag);
+          flag);
   if (flag)
     plainGramKernel<<<2 * smCount(), 256, 0, s>>>(A, lda, p, B, ldb, q, N, C,
                                                   ldc, flag);
@@ -1444,7 +1439,7 @@ size_t exactVCScratchBytes(size_t N, int m, int k, int digits) {
 }
 
 // Y = V C (accum: Y += V C) to ~1e-12 relative of the column maxima (6
-// digits) or FP64's accuracy (8 digits; see above)
+// digits) or better than the FP64 kernel's sums (8 digits; see above)
 void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *Cm,
                  int ldc, int k, double2 *Y, size_t ldy, size_t N,
                  void *scratch, cudaStream_t s, bool accum, int digits) {
