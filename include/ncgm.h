@@ -101,6 +101,11 @@ int ncgm_destroy(ncgm_ctx *ctx);
 const char *ncgm_last_error(void);
 /* Device sync; returns the first pending error. */
 int ncgm_sync(ncgm_ctx *ctx);
+/* Fault injection from the host: sets the context's error word as a tensor-
+ * core kernel does whose bounded wait ran out. The context's next call that
+ * runs such kernels (ncgm_gcg, ncgm_gram, ncgm_vc) returns NCGM_ERR_TIMEOUT
+ * and clears it; other contexts do not see it. */
+int ncgm_set_digit_error(ncgm_ctx *ctx);
 
 /* ---- Hamiltonian -------------------------------------------------------- */
 

@@ -115,6 +115,7 @@ SIGNATURES = {
     "ncgm_destroy": ([_vp], _i),
     "ncgm_last_error": ([], C.c_char_p),
     "ncgm_sync": ([_vp], _i),
+    "ncgm_set_digit_error": ([_vp], _i),
     "ncgm_set_fields": ([_vp, _i, _vp, _vp, _vp, _vp, _vp], _i),
     "ncgm_set_woods_saxon": ([_vp, _i, _i, _i, _d, _d, _d, _d, _d, _d, _d,
                               _i], _i),

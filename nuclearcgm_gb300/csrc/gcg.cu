@@ -138,16 +138,6 @@ double msSince(std::chrono::steady_clock::time_point t0) {
 
 } // namespace
 
-int takeExactErr() {
-  int flag = 0, zero = 0;
-  if (cudaMemcpy(&flag, exactGramErrWord(), sizeof(int),
-                 cudaMemcpyDeviceToHost) != cudaSuccess)
-    return 1;
-  if (flag)
-    cudaMemcpy(exactGramErrWord(), &zero, sizeof(int), cudaMemcpyHostToDevice);
-  return flag;
-}
-
 // Orthonormalise the k columns of V (N x k, ld N) into Q with MGS-equivalent
 // dropping (pivot <= 1e-24). Returns kept column count; Q gets them compacted.
 static int cholQR2(ncgm_ctx *ctx, const double2 *V, int k, double2 *Q,
@@ -243,6 +233,8 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
       prod.gramScr = nullptr;
       prod.vcScr = nullptr;
     }
+    prod.err = digitErrWord(ctx);
+    if (!prod.err) return NCGM_ERR_NOMEM;
   }
   // the projected eigensolver's workspace (Householder methods)
   const size_t heigScrB = heigScratchBytes(mx);
@@ -609,7 +601,7 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   for (int k = 0; k < nev; ++k) lamOut[k] = finalL[order[k]];
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
-  if (prod.gramScr && takeExactErr()) {
+  if (takeDigitErr(ctx)) {
     setError("ncgm_gcg: tensor-core kernel wait timed out");
     return NCGM_ERR_TIMEOUT;
   }
@@ -725,7 +717,6 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
                        : static_cast<double2 *>(
                              ctx->buf(28, (size_t)p * q * sizeof(double2)));
   if (!dC) return NCGM_ERR_NOMEM;
-  bool digits = false;
   if (precision == NCGM_FP32) {
     float *part = static_cast<float *>(
         ctx->buf(29, sizeof(float) * tcGramPartialFloats(N, p, q) + 256));
@@ -746,7 +737,8 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
           ctx->buf(29, sizeof(double2) * (size_t)prod.maxChunks * p * q));
       if (!prod.partials) return NCGM_ERR_NOMEM;
     }
-    digits = prod.gramScr != nullptr;
+    prod.err = digitErrWord(ctx);
+    if (!prod.err) return NCGM_ERR_NOMEM;
     prod.gram(dA, N, p, dB, N, q, N, dC, p, s);
   }
   if (!devOut)
@@ -754,8 +746,7 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
                               cudaMemcpyDeviceToHost, s));
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
-  int flag = 0;
-  if (digits) flag = takeExactErr();
+  int flag = takeDigitErr(ctx);
   if (precision == NCGM_FP32)
     NCGM_CUDA(cudaMemcpy(&flag, tcGramErrWord(), sizeof(int),
                          cudaMemcpyDeviceToHost));
@@ -797,6 +788,8 @@ extern "C" int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C,
   if (prod.digits == 6 || digitsPayVC(N, m, k)) {
     prod.vcScr = ctx->buf(29, exactVCScratchBytes(N, m, k, prod.digits));
     if (!prod.vcScr && prod.digits == 6) return NCGM_ERR_NOMEM;
+    prod.err = digitErrWord(ctx);
+    if (!prod.err) return NCGM_ERR_NOMEM;
   }
   prod.vc(dV, N, m, dC, m, k, dY, N, N, s);
   if (!devOut)
@@ -804,7 +797,7 @@ extern "C" int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C,
                               cudaMemcpyDeviceToHost, s));
   NCGM_CUDA(cudaStreamSynchronize(s));
   NCGM_CUDA(cudaGetLastError());
-  if (prod.vcScr && takeExactErr()) {
+  if (takeDigitErr(ctx)) {
     setError("ncgm_vc: tensor-core kernel wait timed out");
     return NCGM_ERR_TIMEOUT;
   }

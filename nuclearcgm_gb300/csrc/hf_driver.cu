@@ -284,8 +284,12 @@ struct Run {
     digitTried = true;
     BlockProducts p;
     p.digits = digits();
-    p.gramScr = static_cast<double *>(digitScr);
-    p.vcScr = digitScr;
+    // without the error word as without scratch
+    p.err = digitScr ? digitErrWord(ctx) : nullptr;
+    if (p.err) {
+      p.gramScr = static_cast<double *>(digitScr);
+      p.vcScr = digitScr;
+    }
     return p;
   }
 
@@ -301,7 +305,8 @@ struct Run {
     if (digits() == 6 || digitsPayGram(ns, M, M)) {
       // both bounds hold for every window size nS <= M
       w.gemmExact = alloc<char>(digitBytes(ns));
-      if (!w.gemmExact) {
+      if (!w.gemmExact || !digitErrWord(ctx)) {
+        w.gemmExact = nullptr;
         if (digits() == 6) return nullptr;
         cudaGetLastError();
       }
@@ -348,6 +353,7 @@ struct Run {
     g.digits = digits();
     g.gramScr = static_cast<double *>(hw.gemmExact);
     g.vcScr = hw.gemmExact;
+    g.err = ctx->digitErr;
     g.partials = hw.gemmParts;
     g.maxChunks = HfbWork::kChunks;
     return g;
@@ -400,6 +406,14 @@ int sync(Run &R) {
     return NCGM_ERR_CUDA;
   }
   return NCGM_OK;
+}
+
+// the digit products on the run's own context; both species' eigensolver
+// calls check theirs
+int checkDigits(Run &R, const char *who) {
+  if (!takeDigitErr(R.ctx)) return NCGM_OK;
+  setError(std::string(who) + ": tensor-core kernel wait timed out");
+  return NCGM_ERR_TIMEOUT;
 }
 
 // gram of columns (N rows): C = A^H B into host matrix (p x q)
@@ -1505,6 +1519,7 @@ int hfRun(const ncgm_hf_config &cfg, ncgm_hf_result &res, double *spe_n,
     double nE = 0, nH = 0;
     NCGM_TRY(energies(R, nE, nH));
     NCGM_TRY(phaseSync(R, "energies", it));
+    NCGM_TRY(checkDigits(R, "hf"));
     bool cconv = true;
     for (auto &c : R.cons)
       if (c.error() != 0.0) cconv = cconv && (c.error() < cfg.constraints_tol);
@@ -1557,6 +1572,7 @@ int hfRun(const ncgm_hf_config &cfg, ncgm_hf_result &res, double *spe_n,
     NCGM_CUDA(cudaMemcpyAsync(rho_p, R.rho[1], sizeof(double) * R.ns,
                               cudaMemcpyDeviceToHost, R.s));
   NCGM_TRY(sync(R));
+  NCGM_TRY(checkDigits(R, "hf"));
   res.wall_s = now() - tStart;
   return NCGM_OK;
 }
@@ -1879,11 +1895,7 @@ extern "C" int ncgm_state_update(ncgm_state *st, const double *Xn,
     }
     NCGM_TRY(updateQuantities(R, iter));
     NCGM_TRY(sync(R));
-    if ((R.digitScr || R.hw.gemmExact) && takeExactErr()) {
-      setError("ncgm_state_update: tensor-core kernel wait timed out");
-      return NCGM_ERR_TIMEOUT;
-    }
-    return NCGM_OK;
+    return checkDigits(R, "ncgm_state_update");
   } catch (const std::exception &e) {
     setError(e.what());
     return NCGM_ERR_ARG;

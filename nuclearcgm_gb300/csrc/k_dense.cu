@@ -548,7 +548,7 @@ void BlockProducts::gram(const double2 *A, size_t lda, int p, const double2 *B,
                          size_t ldb, int q, size_t N, double2 *C, int ldc,
                          cudaStream_t s) const {
   if (gramScr && (digits == 6 || digitsPayGram(N, p, q)))
-    gramTCExact(A, lda, p, B, ldb, q, N, C, ldc, gramScr, s, digits);
+    gramTCExact(A, lda, p, B, ldb, q, N, C, ldc, gramScr, s, digits, err);
   else
     ncgm::gram(A, lda, p, B, ldb, q, N, C, ldc, partials, maxChunks, s);
 }
@@ -557,7 +557,8 @@ void BlockProducts::vc(const double2 *V, size_t ldv, int m, const double2 *Cm,
                        int ldc, int k, double2 *Y, size_t ldy, size_t N,
                        cudaStream_t s, bool accum) const {
   if (vcScr && (digits == 6 || digitsPayVC(N, m, k)))
-    gemmVCExact(V, ldv, m, Cm, ldc, k, Y, ldy, N, vcScr, s, accum, digits);
+    gemmVCExact(V, ldv, m, Cm, ldc, k, Y, ldy, N, vcScr, s, accum, digits,
+                err);
   else
     gemmVC(V, ldv, m, Cm, ldc, k, Y, ldy, N, accum ? 1.0 : 0.0, s);
 }

@@ -24,24 +24,20 @@ int *tcGramErrWord();
 // exact FP32 level sums, exact integer combination (k_tcgram_exact.cu).
 // scratch: exactGramScratchDoubles(N, p, q, digits) doubles, 16-byte aligned.
 // 8 digits: operands with infinities, NaNs or extreme magnitudes take a plain
-// FP64 sum on the device.
+// FP64 sum on the device. err (device): set to 1 when a bounded wait gives up.
 void gramTCExact(const double2 *A, size_t lda, int p, const double2 *B,
                  size_t ldb, int q, size_t N, double2 *C, int ldc,
-                 double *scratch, cudaStream_t s, int digits = 6);
-size_t exactGramScratchDoubles(size_t N, int p, int q, int digits = 6);
-int *exactGramErrWord();
-// reads and clears the error word of the exact-digit kernels (non-zero: a
-// bounded wait of one of them gave up)
-int takeExactErr();
+                 double *scratch, cudaStream_t s, int digits, int *err);
+size_t exactGramScratchDoubles(size_t N, int p, int q, int digits);
 // Y = V C on the tensor cores with the exact digit products of gramTCExact
 // (6 digits: ~1e-12 relative of the column maxima; 8: FP64 accuracy;
 // k_tcgram_exact.cu). scratch: exactVCScratchBytes(N, m, k, digits) bytes,
 // 16-byte aligned.
 void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *C,
                  int ldc, int k, double2 *Y, size_t ldy, size_t N,
-                 void *scratch, cudaStream_t s, bool accum = false,
-                 int digits = 6);
-size_t exactVCScratchBytes(size_t N, int m, int k, int digits = 6);
+                 void *scratch, cudaStream_t s, bool accum, int digits,
+                 int *err);
+size_t exactVCScratchBytes(size_t N, int m, int k, int digits);
 // Y = V C + beta Y (V: N x m with m <= 1600, C: m x k; C is staged in
 // shared memory in blocks of columns).
 void gemmVC(const double2 *V, size_t ldv, int m, const double2 *C, int ldc,
@@ -58,6 +54,7 @@ struct BlockProducts {
   int digits = 8;
   double *gramScr = nullptr; // exactGramScratchDoubles
   void *vcScr = nullptr;     // exactVCScratchBytes (may be the same memory)
+  int *err = nullptr;        // the context's error word (with scratch)
   double2 *partials = nullptr; // plain Gram: maxChunks p q
   int maxChunks = 1;
   // C = A^H B

@@ -60,7 +60,6 @@
 namespace ncgm {
 
 int smCount();
-int *exactGramErrWord();
 
 namespace {
 
@@ -1273,7 +1272,7 @@ size_t vcHeaderBytes(int m, int k) {
 template <int kDig>
 void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
                 size_t ldb, int q, size_t N, double2 *C, int ldc,
-                double *scratch, cudaStream_t s) {
+                double *scratch, cudaStream_t s, int *err) {
   static const bool attr = [] {
     cudaFuncSetAttribute(exactGramKernel<kDig>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1313,8 +1312,7 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
   dim3 grid((2 * p + kM - 1) / kM, (2 * q + kN - 1) / kN, chunks);
   int *partLo = reinterpret_cast<int *>(partHi + (size_t)chunks * 4 * p * q);
   exactGramKernel<kDig><<<grid, kThr, Fmt<kDig>::kSmem, s>>>(
-      imgA, imgB, p, q, nslab, spc, partHi, partLo, self ? 1 : 0, flag,
-      exactGramErrWord());
+      imgA, imgB, p, q, nslab, spc, partHi, partLo, self ? 1 : 0, flag, err);
   exactGramReduce<kDig>
       <<<(unsigned)(((size_t)p * q * 32 + 255) / 256), 256, 0, s>>>(
           partHi, partLo, chunks, p, q, eA, eB, C, ldc, self ? 1 : 0,
@@ -1327,7 +1325,7 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
 template <int kDig>
 void vcDigits(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
               int k, double2 *Y, size_t ldy, size_t N, void *scratch,
-              cudaStream_t s, bool accum) {
+              cudaStream_t s, bool accum, int *err) {
   static const bool attr = [] {
     cudaFuncSetAttribute(exactVCKernel<kDig>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1366,7 +1364,7 @@ void vcDigits(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
   const int G = std::min(tiles, smCount());
   exactVCKernel<kDig><<<G, kThr, Fmt<kDig>::kSmem, s>>>(
       imgV, dig, eB, eR, k, nslab, ntile, tiles, Y, ldy, N, accum ? 1 : 0,
-      flag, exactGramErrWord());
+      flag, err);
   if (flag)
     plainVCKernel<<<2 * smCount(), 256, 0, s>>>(V, ldv, m, Cm, ldc, k, Y, ldy,
                                                 N, accum ? 1 : 0, flag);
@@ -1405,26 +1403,16 @@ size_t exactGramScratchDoubles(size_t N, int p, int q, int digits) {
   return (bytes + sizeof(double) - 1) / sizeof(double);
 }
 
-int *exactGramErrWord() {
-  static int *d = [] {
-    int *x = nullptr;
-    if (cudaMalloc(&x, sizeof(int)) == cudaSuccess)
-      cudaMemset(x, 0, sizeof(int));
-    return x;
-  }();
-  return d;
-}
-
 // C = A^H B on the tensor cores with 6 digits (~1e-13 relative) or 8 (at
 // least FP64's accuracy; see the file comment); scratch holds
 // exactGramScratchDoubles(N, p, q, digits) doubles (256-byte aligned). A Gram
 // of a block with itself (A == B, same ld and width) digitises it once.
 void gramTCExact(const double2 *A, size_t lda, int p, const double2 *B,
                  size_t ldb, int q, size_t N, double2 *C, int ldc,
-                 double *scratch, cudaStream_t s, int digits) {
+                 double *scratch, cudaStream_t s, int digits, int *err) {
   if (p == 0 || q == 0 || N == 0) return;
   (digits == 8 ? gramDigits<8> : gramDigits<6>)(A, lda, p, B, ldb, q, N, C,
-                                                ldc, scratch, s);
+                                                ldc, scratch, s, err);
 }
 
 // scratch of gemmVCExact in bytes: A column scales / exponents (2m), B
@@ -1442,7 +1430,8 @@ size_t exactVCScratchBytes(size_t N, int m, int k, int digits) {
 // digits) or better than the FP64 kernel's sums (8 digits; see above)
 void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *Cm,
                  int ldc, int k, double2 *Y, size_t ldy, size_t N,
-                 void *scratch, cudaStream_t s, bool accum, int digits) {
+                 void *scratch, cudaStream_t s, bool accum, int digits,
+                 int *err) {
   if (k == 0 || N == 0) return;
   if (m == 0) {
     if (accum) return;
@@ -1451,7 +1440,7 @@ void gemmVCExact(const double2 *V, size_t ldv, int m, const double2 *Cm,
     return;
   }
   (digits == 8 ? vcDigits<8> : vcDigits<6>)(V, ldv, m, Cm, ldc, k, Y, ldy, N,
-                                            scratch, s, accum);
+                                            scratch, s, accum, err);
 }
 
 } // namespace ncgm

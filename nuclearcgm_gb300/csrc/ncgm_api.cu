@@ -29,6 +29,38 @@ bool isDevicePtr(const void *p) {
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+int *digitErrWord(ncgm_ctx *ctx) {
+  if (!ctx->digitErr) {
+    int *d = nullptr;
+    if (cudaMalloc(&d, sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      setError("device allocation of the error word failed");
+      return nullptr;
+    }
+    // complete before any stream uses the word
+    const int zero = 0;
+    if (cudaMemcpy(d, &zero, sizeof(int), cudaMemcpyHostToDevice) !=
+        cudaSuccess) {
+      cudaFree(d);
+      return nullptr;
+    }
+    ctx->digitErr = d;
+  }
+  return ctx->digitErr;
+}
+
+int takeDigitErr(ncgm_ctx *ctx) {
+  if (!ctx->digitErr) return 0;
+  int flag = 0;
+  if (cudaMemcpyAsync(&flag, ctx->digitErr, sizeof(int),
+                      cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+      cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+    return 1;
+  if (flag)
+    cudaMemsetAsync(ctx->digitErr, 0, sizeof(int), ctx->stream);
+  return flag;
+}
+
 } // namespace ncgm
 
 void *ncgm_ctx::buf(int slot, size_t bytes) {
@@ -142,6 +174,7 @@ int ncgm_destroy(ncgm_ctx *ctx) {
     if (s.coef32s) cudaFree(s.coef32s);
     if (s.coefInt) cudaFree(s.coefInt);
   }
+  if (ctx->digitErr) cudaFree(ctx->digitErr);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   for (auto e : ctx->xev) cudaEventDestroy(e);
@@ -341,6 +374,20 @@ int ncgm_apply_h_device(ncgm_ctx *ctx, int species, const void *X, void *Y,
   NCGM_CUDA(cudaGetLastError());
   return NCGM_OK;
   NCGM_GUARD_END
+}
+
+int ncgm_set_digit_error(ncgm_ctx *ctx) {
+  if (!ctx) {
+    setError("ncgm_set_digit_error: null context");
+    return NCGM_ERR_ARG;
+  }
+  int *w = digitErrWord(ctx);
+  if (!w) return NCGM_ERR_NOMEM;
+  const int one = 1;
+  NCGM_CUDA(cudaMemcpyAsync(w, &one, sizeof(int), cudaMemcpyHostToDevice,
+                            ctx->stream));
+  NCGM_CUDA(cudaStreamSynchronize(ctx->stream));
+  return NCGM_OK;
 }
 
 int ncgm_set_stream(ncgm_ctx *ctx, void *stream) {

@@ -66,6 +66,9 @@ struct ncgm_ctx {
   std::vector<std::pair<void *, size_t>> bufs;
   void *buf(int slot, size_t bytes);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // set by a digit kernel (k_tcgram_exact.cu) of this context whose bounded
+  // wait gave up; allocated on first use
+  int *digitErr = nullptr;
   ncgm_lp *lp = nullptr; // learned preconditioner (not owned)
   // host-buffer applies: copy-in / copy-out streams and their events,
   // created on first use
@@ -96,6 +99,11 @@ void applyHInt(const double2 *X, double2 *Y, const double *coef64,
                cudaStream_t s);
 void applyH32(ncgm_ctx *ctx, int species, const float2 *X, float2 *Y,
               int ncols, float shift, cudaStream_t s);
+// The context's error word of the digit kernels (null: no memory).
+int *digitErrWord(ncgm_ctx *ctx);
+// Waits for the context's stream; non-zero when one of its digit kernels gave
+// up since the last call (the word is cleared), or the device fails.
+int takeDigitErr(ncgm_ctx *ctx);
 // Non-zero when a stencil's bounded wait gave up since the last reset.
 int stencilErrorFlag();
 
