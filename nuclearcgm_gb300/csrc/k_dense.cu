@@ -925,14 +925,16 @@ static void cholInverse(const double2 *R, int m, const int *keep, double2 *T,
                         cudaStream_t s) {
   const size_t smem =
       (size_t)m * ((1 + kInvAhead) * sizeof(double2) + sizeof(double));
-  if (smem > 200 * 1024) { // m > 2327
+  constexpr size_t kMaxSmem = 200 * 1024;
+  if (smem > kMaxSmem) { // m > 2327
     cholInvKernel<false><<<m, 32, 0, s>>>(R, m, keep, T);
     return;
   }
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(cholInvKernel<true>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+  // a per-device attribute, set to the same value on every call: another
+  // thread may launch with another size in between
+  cudaFuncSetAttribute(cholInvKernel<true>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)kMaxSmem);
   cholInvKernel<true><<<m, 32, smem, s>>>(R, m, keep, T);
 }
 
@@ -951,26 +953,13 @@ void cholDrop(const double2 *G, int ldg, int m, double dropTol, double2 *R,
     cholInverse(R, m, keep, T, s);
     return;
   }
-  static const bool attr = [] {
-    cudaFuncSetAttribute(cholDropSmemKernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2 * kCholSmemMax * kCholSmemMax * (int)sizeof(double2));
-    return true;
-  }();
-  (void)attr;
-  const size_t smem = 2 * (size_t)m * m * sizeof(double2);
-  static const bool dfAttr = [] {
-    cudaFuncSetAttribute(cholDropDfKernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2 * kCholSmemMax * kCholSmemMax * (int)sizeof(dfc));
-    return true;
-  }();
-  (void)dfAttr;
-  if (fast)
-    cholDropDfKernel<<<1, 256, 2 * (size_t)m * m * sizeof(dfc), s>>>(
-        G, ldg, m, dropTol, R, T, keep);
-  else
-    cholDropSmemKernel<<<1, 256, smem, s>>>(G, ldg, m, dropTol, R, T, keep);
+  static_assert(sizeof(dfc) == sizeof(double2), "one shared-memory size");
+  const auto kernel = fast ? cholDropDfKernel : cholDropSmemKernel;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       2 * kCholSmemMax * kCholSmemMax * (int)sizeof(double2));
+  kernel<<<1, 256, 2 * (size_t)m * m * sizeof(double2), s>>>(G, ldg, m,
+                                                             dropTol, R, T,
+                                                             keep);
   if (m >= kInvOutside) cholInverse(R, m, keep, T, s);
 }
 

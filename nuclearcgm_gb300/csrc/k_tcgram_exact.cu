@@ -1273,13 +1273,10 @@ template <int kDig>
 void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
                 size_t ldb, int q, size_t N, double2 *C, int ldc,
                 double *scratch, cudaStream_t s, int *err) {
-  static const bool attr = [] {
-    cudaFuncSetAttribute(exactGramKernel<kDig>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         Fmt<kDig>::kSmem);
-    return true;
-  }();
-  (void)attr;
+  // a per-device attribute: set on every call
+  cudaFuncSetAttribute(exactGramKernel<kDig>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       Fmt<kDig>::kSmem);
   const bool self = A == B && lda == ldb && p == q;
   double *scA = scratch, *scB = scA + 2 * (size_t)p;
   int *eA = reinterpret_cast<int *>(scB + 2 * (size_t)q);
@@ -1326,13 +1323,10 @@ template <int kDig>
 void vcDigits(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
               int k, double2 *Y, size_t ldy, size_t N, void *scratch,
               cudaStream_t s, bool accum, int *err) {
-  static const bool attr = [] {
-    cudaFuncSetAttribute(exactVCKernel<kDig>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         Fmt<kDig>::kSmem);
-    return true;
-  }();
-  (void)attr;
+  // a per-device attribute: set on every call
+  cudaFuncSetAttribute(exactVCKernel<kDig>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       Fmt<kDig>::kSmem);
   const int nslab = (2 * m + kSlab - 1) / kSlab;
   const int ntile = (2 * k + kN - 1) / kN;
   const int mtile = (int)((N + kM - 1) / kM);
