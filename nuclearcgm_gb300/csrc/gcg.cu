@@ -220,26 +220,25 @@ int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
   need += ctx->ns * sizeof(float) + 256; // FP32 inverse Jacobi diagonal
   char *base = static_cast<char *>(ctx->buf(10, need + 64 * 4096));
   if (!base) return NCGM_ERR_NOMEM;
-  BlockProducts prod;
-  prod.digits = digits;
-  if (digits == 6 || digitsPayGram(N, vmax, vmax)) {
-    prod.gramScr = static_cast<double *>(ctx->buf(
-        11, sizeof(double) * exactGramScratchDoubles(N, vmax, vmax, digits) +
-                256));
-    prod.vcScr = ctx->buf(31, exactVCScratchBytes(N, vmax, vmax, digits));
-    if (!prod.gramScr || !prod.vcScr) {
-      if (digits == 6) return NCGM_ERR_NOMEM;
-      // no room for the digit images: the plain FP64 kernels
-      prod.gramScr = nullptr;
-      prod.vcScr = nullptr;
-    }
-    prod.err = digitErrWord(ctx);
-    if (!prod.err) return NCGM_ERR_NOMEM;
-  }
   // the projected eigensolver's workspace (Householder methods)
   const size_t heigScrB = heigScratchBytes(mx);
   void *heigScr = ctx->buf(32, heigScrB);
   if (!heigScr) return NCGM_ERR_NOMEM;
+  // the digit images, after all that the call cannot do without; the Gram's
+  // and V C's share them (64 bytes per complex entry of the search space with
+  // 8 digits). Without room for those the plain FP64 kernels run.
+  BlockProducts prod;
+  prod.digits = digits;
+  if (digits == 6 || digitsPayGram(N, vmax, vmax)) {
+    const size_t b = std::max(
+        sizeof(double) * exactGramScratchDoubles(N, vmax, vmax, digits) + 256,
+        exactVCScratchBytes(N, vmax, vmax, digits));
+    prod.vcScr = digits == 6 ? ctx->buf(11, b) : ctx->spare(11, b);
+    if (!prod.vcScr && digits == 6) return NCGM_ERR_NOMEM;
+    prod.gramScr = static_cast<double *>(prod.vcScr);
+    prod.err = digitErrWord(ctx);
+    if (!prod.err) return NCGM_ERR_NOMEM;
+  }
   Carve ar{base};
   double2 *V = ar.take<double2>(N * vmax), *Q = ar.take<double2>(N * vmax),
           *AV = ar.take<double2>(N * vmax), *Q1 = ar.take<double2>(N * vmax);
@@ -725,10 +724,14 @@ extern "C" int ncgm_gram(ncgm_ctx *ctx, const double *A, int p,
   } else {
     BlockProducts prod;
     prod.digits = precision == NCGM_FP32_TC ? 6 : 8;
-    if (prod.digits == 6 || digitsPayGram(N, p, q))
-      prod.gramScr = static_cast<double *>(ctx->buf(
-          29, sizeof(double) * exactGramScratchDoubles(N, p, q, prod.digits) +
-                  256));
+    if (prod.digits == 6 || digitsPayGram(N, p, q)) {
+      const size_t b =
+          sizeof(double) * exactGramScratchDoubles(N, p, q, prod.digits,
+                                                   dA == dB && p == q) +
+          256;
+      prod.gramScr = static_cast<double *>(
+          prod.digits == 6 ? ctx->buf(29, b) : ctx->spare(29, b));
+    }
     if (!prod.gramScr) {
       // FP64 on small blocks, or no room for the digit images
       if (prod.digits == 6) return NCGM_ERR_NOMEM;
@@ -786,7 +789,8 @@ extern "C" int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C,
   BlockProducts prod;
   prod.digits = precision == NCGM_FP32_TC ? 6 : 8;
   if (prod.digits == 6 || digitsPayVC(N, m, k)) {
-    prod.vcScr = ctx->buf(29, exactVCScratchBytes(N, m, k, prod.digits));
+    const size_t b = exactVCScratchBytes(N, m, k, prod.digits);
+    prod.vcScr = prod.digits == 6 ? ctx->buf(29, b) : ctx->spare(29, b);
     if (!prod.vcScr && prod.digits == 6) return NCGM_ERR_NOMEM;
     prod.err = digitErrWord(ctx);
     if (!prod.err) return NCGM_ERR_NOMEM;

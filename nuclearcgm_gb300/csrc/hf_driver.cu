@@ -277,7 +277,8 @@ struct Run {
   }
   BlockProducts products() {
     const int M = std::max(sp[0].orb, sp[1].orb);
-    if (!digitTried && (digits() == 6 || digitsPayGram(N, M, M))) {
+    if (!digitTried && (digits() == 6 || (digitsPayGram(N, M, M) &&
+                                          spareFits(digitBytes(N))))) {
       digitScr = alloc<char>(digitBytes(N));
       if (!digitScr) cudaGetLastError();
     }
@@ -302,15 +303,6 @@ struct Run {
     HfbWork w;
     w.M = M;
     w.gemmParts = alloc<double2>(HfbWork::kChunks * MM);
-    if (digits() == 6 || digitsPayGram(ns, M, M)) {
-      // both bounds hold for every window size nS <= M
-      w.gemmExact = alloc<char>(digitBytes(ns));
-      if (!w.gemmExact || !digitErrWord(ctx)) {
-        w.gemmExact = nullptr;
-        if (digits() == 6) return nullptr;
-        cudaGetLastError();
-      }
-    }
     double *d = alloc<double>(4 * (size_t)M + 4 * MM + 2 * (size_t)M + 16);
     double2 *c = alloc<double2>(2 * MM + 3 * 4 * MM + 3 * MM);
     int *iw = alloc<int>(2 * (size_t)M + 16);
@@ -327,6 +319,18 @@ struct Run {
     w.heigScr = alloc<char>(w.heigScrB);
     if (!w.gemmParts || !d || !c || !iw || !w.gemmW || !w.heigScr)
       return nullptr;
+    // the digit images last: without room for those of 8 digits the plain
+    // FP64 kernels run
+    if (digits() == 6 ||
+        (digitsPayGram(ns, M, M) && spareFits(digitBytes(ns)))) {
+      // both bounds hold for every window size nS <= M
+      w.gemmExact = alloc<char>(digitBytes(ns));
+      if (!w.gemmExact || !digitErrWord(ctx)) {
+        w.gemmExact = nullptr;
+        if (digits() == 6) return nullptr;
+        cudaGetLastError();
+      }
+    }
     w.e = d;
     w.ff = w.e + M;
     w.eig = w.ff + M; // 2M

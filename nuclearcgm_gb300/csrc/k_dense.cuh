@@ -28,7 +28,9 @@ int *tcGramErrWord();
 void gramTCExact(const double2 *A, size_t lda, int p, const double2 *B,
                  size_t ldb, int q, size_t N, double2 *C, int ldc,
                  double *scratch, cudaStream_t s, int digits, int *err);
-size_t exactGramScratchDoubles(size_t N, int p, int q, int digits);
+// self: for Grams of a block with itself alone (half of the images)
+size_t exactGramScratchDoubles(size_t N, int p, int q, int digits,
+                               bool self = false);
 // Y = V C on the tensor cores with the exact digit products of gramTCExact
 // (6 digits: ~1e-12 relative of the column maxima; 8: FP64 accuracy;
 // k_tcgram_exact.cu). scratch: exactVCScratchBytes(N, m, k, digits) bytes,

@@ -1285,7 +1285,7 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
   int *flag = kDig == 8 ? eB + 2 * (size_t)q : nullptr;
   const size_t head = gramHeaderBytes(p, q);
   unsigned char *imgA = reinterpret_cast<unsigned char *>(scratch) + head;
-  unsigned char *imgB = imgA + gramImageBytes(N, p, kDig);
+  unsigned char *imgB = self ? imgA : imgA + gramImageBytes(N, p, kDig);
   long long *partHi =
       reinterpret_cast<long long *>(imgB + gramImageBytes(N, q, kDig));
   const int nslab = (int)((N + kSlab - 1) / kSlab);
@@ -1296,7 +1296,6 @@ void gramDigits(const double2 *A, size_t lda, int p, const double2 *B,
       <<<dim3(nslab, (2 * p + kM - 1) / kM), 256, 0, s>>>(
           A, lda, p, N, eA, nslab, imgA, flag);
   if (self) {
-    imgB = imgA;
     eB = eA;
   } else {
     digitizeGramKernel<kDig>
@@ -1373,7 +1372,8 @@ void vcDigits(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
 // the bound is the largest over every (M tiles, N tiles) count up to those
 // of (p, q), each with its widest p', q' (and, for equal widths, over the
 // tiles on and above the diagonal alone).
-size_t exactGramScratchDoubles(size_t N, int p, int q, int digits) {
+size_t exactGramScratchDoubles(size_t N, int p, int q, int digits,
+                               bool self) {
   const int mtiles = (2 * p + kM - 1) / kM, ntiles = (2 * q + kN - 1) / kN;
   size_t part = 0;
   for (int a = 1; a <= mtiles; ++a)
@@ -1390,7 +1390,7 @@ size_t exactGramScratchDoubles(size_t N, int p, int q, int digits) {
     part = std::max(part, chunks * 4 * (size_t)w * w);
   }
   const size_t bytes = gramHeaderBytes(p, q) + gramImageBytes(N, p, digits) +
-                       gramImageBytes(N, q, digits) +
+                       (self ? 0 : gramImageBytes(N, q, digits)) +
                        (sizeof(long long) + (digits == 8 ? sizeof(int) : 0)) *
                            part +
                        256;

@@ -29,6 +29,15 @@ bool isDevicePtr(const void *p) {
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+bool spareFits(size_t bytes, size_t held) {
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= (free + held) / 2;
+}
+
 int *digitErrWord(ncgm_ctx *ctx) {
   if (!ctx->digitErr) {
     int *d = nullptr;
@@ -79,6 +88,12 @@ void *ncgm_ctx::buf(int slot, size_t bytes) {
     b.second = bytes;
   }
   return b.first;
+}
+
+void *ncgm_ctx::spare(int slot, size_t bytes) {
+  const size_t held = (int)bufs.size() > slot ? bufs[slot].second : 0;
+  return held >= bytes || ncgm::spareFits(bytes, held) ? buf(slot, bytes)
+                                                       : nullptr;
 }
 
 using namespace ncgm;

@@ -65,6 +65,9 @@ struct ncgm_ctx {
   // scratch buffers, grown on demand (device)
   std::vector<std::pair<void *, size_t>> bufs;
   void *buf(int slot, size_t bytes);
+  // the same for scratch that only a faster form needs: null without an error
+  // when growing it would take more than half of the device's free memory
+  void *spare(int slot, size_t bytes);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // set by a digit kernel (k_tcgram_exact.cu) of this context whose bounded
   // wait gave up; allocated on first use
@@ -99,6 +102,9 @@ void applyHInt(const double2 *X, double2 *Y, const double *coef64,
                cudaStream_t s);
 void applyH32(ncgm_ctx *ctx, int species, const float2 *X, float2 *Y,
               int ncols, float shift, cudaStream_t s);
+// At most half of the device's free memory (with `held`, which growing gives
+// back): the other half is left to the caller and to other contexts.
+bool spareFits(size_t bytes, size_t held = 0);
 // The context's error word of the digit kernels (null: no memory).
 int *digitErrWord(ncgm_ctx *ctx);
 // Waits for the context's stream; non-zero when one of its digit kernels gave
