@@ -28,7 +28,7 @@
 
 namespace ncgm {
 
-bool isDevicePtr(const void *p);
+bool isOnDevice(const void *p, int device);
 int gcgRun(ncgm_ctx *ctx, int species, const double2 *Xinit, int xcols,
            const double2 *ConjDir, int pcols, int nev,
            const ncgm_gcg_params &prm, double2 *Xout, double *lamOut,
@@ -1655,10 +1655,10 @@ extern "C" int ncgm_densities(ncgm_ctx *ctx, const double *Phi, int ncols,
     const size_t N = ctx->N, ns = ctx->ns;
     double *d = static_cast<double *>(ctx->buf(24, 12 * ns * sizeof(double)));
     if (!d) return NCGM_ERR_NOMEM;
-    // columns on the device are read where they are, when the 16-byte loads
-    // allow it
+    // columns on the context's device are read where they are, when the
+    // 16-byte loads allow it
     const double2 *dX = reinterpret_cast<const double2 *>(Phi);
-    if (!isDevicePtr(Phi) || reinterpret_cast<uintptr_t>(Phi) % 16) {
+    if (!isOnDevice(Phi, ctx->device) || reinterpret_cast<uintptr_t>(Phi) % 16) {
       double2 *b = static_cast<double2 *>(
           ctx->buf(23, N * ncols * sizeof(double2)));
       if (!b) return NCGM_ERR_NOMEM;

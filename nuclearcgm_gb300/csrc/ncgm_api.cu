@@ -70,6 +70,18 @@ int takeDigitErr(ncgm_ctx *ctx) {
   return flag;
 }
 
+// Memory that a kernel of `device` reads in place: managed, or on that very
+// device (columns on another one are copied).
+bool isOnDevice(const void *p, int device) {
+  cudaPointerAttributes attr;
+  if (!p || cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return attr.type == cudaMemoryTypeManaged ||
+         (attr.type == cudaMemoryTypeDevice && attr.device == device);
+}
+
 } // namespace ncgm
 
 void *ncgm_ctx::buf(int slot, size_t bytes) {
