@@ -256,7 +256,10 @@ __global__ void cgScalarInit(const double *partials, int nblk, double tol2,
   s[1] = bb;
   s[3] = (bb == 0.0) ? 1.0 : 0.0;
   s[7] = first ? 0.0 : s[7] + (s[6] == 0.0 ? 1.0 : 0.0);
-  s[6] = (bb == 0.0 || rr <= tol2 * bb) ? 1.0 : 0.0;
+  // a norm that is not finite also ends the refinements: U stays the guess
+  // that it was, and the host returns the error
+  const bool finite = isfinite(rr) && isfinite(bb);
+  s[6] = (!finite || bb == 0.0 || rr <= tol2 * bb) ? 1.0 : 0.0;
 }
 
 // alpha = rr / pAp; x += alpha p; r -= alpha Ap; partial |r|^2
