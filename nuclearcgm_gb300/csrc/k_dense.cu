@@ -565,9 +565,14 @@ void BlockProducts::vc(const double2 *V, size_t ldv, int m, const double2 *Cm,
 
 // a / b from the correctly rounded r = 1 / b, rounded as the division is
 // (Markstein 1990: one residual step on a r), for three operations of the FP64
-// pipe instead of a division's ten
+// pipe instead of a division's ten. b > 0. Where the residual or the quotient
+// leaves the normal range (an infinite pivot among them) it is the division
+// itself.
 __device__ __forceinline__ double divBy(double a, double b, double r) {
   const double q = a * r;
+  const int e = (__double2hiint(q) >> 20) & 0x7FF;
+  if (__builtin_expect((unsigned)(e - 200) > 1650u, 0))
+    return (__double_as_longlong(a) << 1) == 0 ? a : a / b;
   return fma(fma(-q, b, a), r, q);
 }
 
