@@ -165,10 +165,19 @@ int buildCoefficients(ncgm_ctx *ctx, int species, const double *f,
                       const double *UC) {
   SpeciesFields &F = ctx->sp[species];
   if (!F.coef64) {
-    NCGM_CUDA(cudaMalloc(&F.coef64, ctx->ns * 8 * sizeof(double)));
-    NCGM_CUDA(cudaMalloc(&F.coef32, ctx->ns * 8 * sizeof(float)));
-    NCGM_CUDA(cudaMalloc(&F.coef32s, ctx->ns * 8 * sizeof(float)));
-    NCGM_CUDA(cudaMalloc(&F.coefInt, intCoefBytes(ctx->ns)));
+    // all of them or none: a later call must not find a part
+    if (cudaMalloc(&F.coef64, ctx->ns * 8 * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&F.coef32, ctx->ns * 8 * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&F.coef32s, ctx->ns * 8 * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&F.coefInt, intCoefBytes(ctx->ns)) != cudaSuccess) {
+      cudaGetLastError();
+      for (void *p : {(void *)F.coef64, (void *)F.coef32, (void *)F.coef32s,
+                      F.coefInt})
+        cudaFree(p); // null: no operation
+      F = SpeciesFields{};
+      setError("device allocation of the Hamiltonian's coefficients failed");
+      return NCGM_ERR_CUDA;
+    }
   }
   buildCoefKernel<<<(unsigned)((ctx->ns + 255) / 256), 256, 0, ctx->stream>>>(
       f, gradf, U, W, UC, ctx->ns, ctx->h, F.coef64, F.coef32, F.coef32s);
