@@ -686,23 +686,43 @@ Shape defaultShape(int n) {
 
 } // namespace
 
+namespace {
+// holds a stream for about `cycles` clocks
+__global__ void pauseKernel(long long cycles) {
+  const long long t0 = clock64();
+  for (int i = 0; i < (1 << 16) && clock64() - t0 < cycles; ++i) {
+  }
+}
+} // namespace
+
 // Project autotuner for the FP32 stencil: times candidate (band rows, ring
 // depth, points per thread, CTAs per SM) on the context's own lattice with
-// CUDA events and keeps the fastest. Runs once per context. Launches of a
-// kernel of 5 us one by one time the queue (10 us each), so the first pass's
-// best 16 of each kind are timed again as graphs of several launches, which is
-// also how the correction solver runs them: 30^3 x 12 columns settled on
-// shapes of 5.2 to 6.2 us from run to run before, on the same one of 5.75 us
-// now.
+// CUDA events and keeps the best, once per process and lattice size, with the
+// column count that asks first.
+//  * First pass, every shape: a few launches of one stream. The host takes some
+//    us for each, so for small blocks they queue behind a pause: without it
+//    every shape of 30^3 x 12 columns took 10.4 us and the order was noise.
+//  * Second pass, the shapes within 10 % of the best: graphs of launches one
+//    after the other, as the correction solver runs them, and on two streams
+//    at once, as the two species of a run do. The sum decides, since the best
+//    of one is not the best of the other (36^3 x 20: 11.9 and 9.7 us a launch
+//    for one shape, 14.5 and 8.5 for another).
 static Shape tune(ncgm_ctx *ctx, int species, int ncols) {
   const int n = ctx->n;
   ncols = std::max(1, std::min(ncols, ctx->max_cols));
-  size_t bytes = ctx->N * ncols * sizeof(float2);
-  float2 *X = static_cast<float2 *>(ctx->buf(1, bytes));
-  float2 *Y = static_cast<float2 *>(ctx->buf(2, bytes));
+  const size_t count = ctx->N * ncols;
   Shape best = defaultShape(n);
-  if (!X || !Y) return best;
-  cudaMemsetAsync(X, 0, bytes, ctx->stream);
+  int sets = 2; // one per stream, where there is room
+  float2 *X = nullptr, *Y = nullptr;
+  for (;; --sets) {
+    X = static_cast<float2 *>(ctx->buf(1, sets * count * sizeof(float2)));
+    Y = static_cast<float2 *>(ctx->buf(2, sets * count * sizeof(float2)));
+    if (X && Y) break;
+    if (sets == 1) return best;
+  }
+  cudaMemsetAsync(X, 0, sets * count * sizeof(float2), ctx->stream);
+  // launches that the pause covers, for blocks of less than about 12 us
+  const bool queueBound = 2 * count * sizeof(float2) < ((size_t)64 << 20);
   std::vector<int> rows;
   for (int r = n;; r = (r + 1) / 2) {
     rows.push_back(r);
@@ -712,13 +732,25 @@ static Shape tune(ncgm_ctx *ctx, int species, int ncols) {
   // NCGM_TUNE_LOG=1 prints every candidate's time to stderr
   const char *lg = std::getenv("NCGM_TUNE_LOG");
   const bool log = lg && lg[0] == '1';
+  auto report = [&](const char *how, const Shape &s, float ms) {
+    if (log)
+      std::fprintf(stderr,
+                   "[ncgm tune] %s n=%d cols=%d kind=%d rows=%d ring=%d ppt=%d "
+                   "ctas/SM=%d cpa=%d nc=%d: %.2f us\n",
+                   how, n, ncols, s.kind, s.TY, s.ring, s.ppt, s.ctasPerSM,
+                   s.cpa, s.nc, 1e3f * ms);
+  };
+  auto launch = [&](const Shape &s, int set) {
+    return launchStream(ctx, species, X + set * count, Y + set * count, ncols,
+                        0.f, ctx->stream, s);
+  };
   // ms per launch, negative when the shape cannot run
   auto timeOf = [&](const Shape &s, int launches) -> float {
-    if (!launchStream(ctx, species, X, Y, ncols, 0.f, ctx->stream, s))
-      return -1.f;
+    if (!launch(s, 0)) return -1.f;
+    if (queueBound)
+      pauseKernel<<<1, 1, 0, ctx->stream>>>(25000ll * launches);
     cudaEventRecord(ctx->ev0, ctx->stream);
-    for (int r = 0; r < launches; ++r)
-      launchStream(ctx, species, X, Y, ncols, 0.f, ctx->stream, s);
+    for (int r = 0; r < launches; ++r) launch(s, 0);
     cudaEventRecord(ctx->ev1, ctx->stream);
     if (cudaEventSynchronize(ctx->ev1) != cudaSuccess) {
       cudaGetLastError();
@@ -726,16 +758,22 @@ static Shape tune(ncgm_ctx *ctx, int species, int ncols) {
     }
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    if (log)
-      std::fprintf(stderr,
-                   "[ncgm tune] n=%d cols=%d kind=%d rows=%d ring=%d ppt=%d "
-                   "ctas/SM=%d cpa=%d nc=%d: %.1f us\n",
-                   n, ncols, s.kind, s.TY, s.ring, s.ppt, s.ctasPerSM, s.cpa,
-                   s.nc, 1e3f * ms / launches);
+    report("queue", s, ms / launches);
     return ms / launches;
   };
-  // the same as one graph of `launches` launches, replayed twice
-  auto graphTimeOf = [&](const Shape &s, int launches) -> float {
+  // ms per launch of one graph of `launches` launches, half of them on a
+  // second stream and set of buffers if `two`: the smaller of two replays
+  // after a first one
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  if (sets > 1 &&
+      (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess ||
+       cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess ||
+       cudaEventCreateWithFlags(&join, cudaEventDisableTiming) != cudaSuccess)) {
+    cudaGetLastError();
+    sets = 1;
+  }
+  auto graphTimeOf = [&](const Shape &s, int launches, bool two) -> float {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     float ms = -1.f;
@@ -745,28 +783,43 @@ static Shape tune(ncgm_ctx *ctx, int species, int ncols) {
       return ms;
     }
     bool ok = true;
-    for (int r = 0; r < launches; ++r)
-      ok = launchStream(ctx, species, X, Y, ncols, 0.f, ctx->stream, s) && ok;
+    if (two) {
+      cudaEventRecord(fork, ctx->stream);
+      cudaStreamWaitEvent(side, fork, 0);
+    }
+    for (int r = 0; r < launches; ++r) {
+      const int set = two ? r % 2 : 0;
+      ok = launchStream(ctx, species, X + set * count, Y + set * count, ncols,
+                        0.f, set ? side : ctx->stream, s) &&
+           ok;
+    }
+    if (two) {
+      cudaEventRecord(join, side);
+      cudaStreamWaitEvent(ctx->stream, join, 0);
+    }
     if (cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && ok &&
         cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
+      float t[2] = {-1.f, -1.f};
       cudaGraphLaunch(exec, ctx->stream);
-      cudaEventRecord(ctx->ev0, ctx->stream);
-      cudaGraphLaunch(exec, ctx->stream);
-      cudaEventRecord(ctx->ev1, ctx->stream);
-      if (cudaEventSynchronize(ctx->ev1) == cudaSuccess) {
-        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-        ms /= launches;
+      for (float &x : t) {
+        cudaEventRecord(ctx->ev0, ctx->stream);
+        cudaGraphLaunch(exec, ctx->stream);
+        cudaEventRecord(ctx->ev1, ctx->stream);
+        if (cudaEventSynchronize(ctx->ev1) != cudaSuccess) break;
+        cudaEventElapsedTime(&x, ctx->ev0, ctx->ev1);
       }
+      if (std::min(t[0], t[1]) >= 0.f) ms = std::min(t[0], t[1]) / launches;
       cudaGraphExecDestroy(exec);
     }
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
+    report(two ? "graph, two streams" : "graph", s, ms);
     return ms;
   };
   auto trial = [&](const Shape &s) {
     int th;
     if (!validShape(n, s, th)) return;
-    const float ms = timeOf(s, 3);
+    const float ms = timeOf(s, queueBound ? 5 : 3);
     if (ms >= 0.f) seen.push_back({ms, s});
   };
   // plus, per points-per-thread, the tallest band one block can cover
@@ -798,19 +851,32 @@ static Shape tune(ncgm_ctx *ctx, int species, int ncols) {
           }
   std::sort(seen.begin(), seen.end(),
             [](const auto &a, const auto &b) { return a.first < b.first; });
-  int taken[4] = {0, 0, 0, 0};
   float bestMs = 1e30f;
-  for (size_t i = 0; i < seen.size(); ++i) {
-    if (taken[seen[i].second.kind]++ >= 16) continue;
-    // about 200 us of them
+  for (size_t i = 0; i < std::min<size_t>(seen.size(), 64); ++i) {
+    const auto &c = seen[i];
+    if (i >= 8 && c.first > 1.1f * seen[0].first) break;
+    // about 100 us of them, an even number
     const int launches =
-        std::max(3, std::min(20, (int)(0.2f / std::max(seen[i].first, 1e-4f))));
-    float ms = graphTimeOf(seen[i].second, launches);
-    if (ms < 0.f) ms = seen[i].first;
-    if (ms < bestMs) {
-      bestMs = ms;
-      best = seen[i].second;
+        2 * std::max(2, std::min(6, (int)(0.05f / std::max(c.first, 1e-4f))));
+    float ms = graphTimeOf(c.second, launches, false);
+    if (ms >= 0.f && sets > 1) {
+      const float two = graphTimeOf(c.second, launches, true);
+      ms = two < 0.f ? two : ms + two;
     }
+    if (ms >= 0.f && ms < bestMs) {
+      bestMs = ms;
+      best = c.second;
+    }
+  }
+  if (bestMs == 1e30f && !seen.empty()) best = seen[0].second;
+  report("chosen", best, bestMs);
+  if (fork) cudaEventDestroy(fork);
+  if (join) cudaEventDestroy(join);
+  if (side) cudaStreamDestroy(side);
+  // nothing else uses the buffers
+  for (int slot : {1, 2}) {
+    cudaFree(ctx->bufs[slot].first);
+    ctx->bufs[slot] = {nullptr, 0};
   }
   return best;
 }
