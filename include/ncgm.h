@@ -383,9 +383,13 @@ int ncgm_shell_observables(ncgm_ctx *ctx, const double *Psi, int ncols,
 /* C (p x q) = A^H B for complex column blocks of ctx->N rows (A: N x p,
  * B: N x q, Eigen layout; host or device buffers): the Gram / projection
  * products of the GCG (src/solver/solver.cpp:750-777, V.adjoint() * W).
- * precision NCGM_FP64: FP64 accuracy, deterministic (from N = 6000 rows on
- * the tensor cores with eight exact 7-bit digits per value, FP64 CUDA cores
- * below and for operands with infinities or NaNs);
+ * precision NCGM_FP64: deterministic; from N = 6000 rows on the tensor cores
+ * with eight exact 8-bit digits per value (62 bits below the column's largest
+ * entry: an element is off by at most 2^-52 |a||b| or so, less than FP64 sums
+ * are; entries more than 2^-9 below their column's largest keep fewer than
+ * their 53 bits). FP64 CUDA cores below, for operands with infinities, NaNs or
+ * magnitudes outside 2^-900 .. 2^900, and when the digits' scratch (32 bytes
+ * per complex entry of A and B) would take more than half of the free memory;
  * NCGM_FP32: tensor cores (tcgen05 kind::tf32 with split TF32 operands,
  * FP32 accumulation over row chunks, FP64 chunk sums; ~2e-6 relative);
  * NCGM_FP32_TC: tensor cores (tcgen05 kind::f16, values split into six
@@ -400,10 +404,13 @@ int ncgm_gram(ncgm_ctx *ctx, const double *A, int p, const double *B, int q,
  * and a small matrix C (m x k, column-major): the subspace rotation of the
  * GCG's orthonormalisation and Rayleigh-Ritz steps (the reference forms it
  * with Eigen products, src/solver/solver.cpp:418-463, 669-677). Host or
- * device pointers. precision NCGM_FP64: FP64 accuracy (large products on the tensor
- * cores with eight digits per value, others on FP64 CUDA cores); NCGM_FP32_TC:
- * tensor cores with the exact digit products of ncgm_gram (~1e-12 relative
- * of the column maxima). */
+ * device pointers. precision NCGM_FP64: large products on the tensor cores
+ * with eight digits per value (62 bits below the row's largest entry, columns
+ * scaled to their maxima: row by row closer than FP64 sums are; entries more
+ * than 2^-9 below their row's largest keep fewer than their 53 bits), others,
+ * and the exceptions of ncgm_gram, on FP64 CUDA cores; NCGM_FP32_TC: tensor
+ * cores with the exact digit products of ncgm_gram (~1e-12 relative of the
+ * column maxima). */
 int ncgm_vc(ncgm_ctx *ctx, const double *V, int m, const double *C, int k,
             double *Y, int precision);
 

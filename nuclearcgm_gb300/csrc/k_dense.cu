@@ -3,12 +3,17 @@
 //  * gram:      C = A^H B for N x p, N x q blocks (row chunks, deterministic
 //               two-pass reduction, no atomics);
 //  * gemmVC:    Y = V C for N x m times m x k;
-//  * cholDrop:  one-CTA Cholesky of a Gram matrix with the modified
-//               Gram-Schmidt column-drop rule (|v_j| after projection below
-//               1e-12 -> column dropped, solver.cpp:404-407), returning the
-//               inverse factor so that Q = V R^{-1};
-//  * heig:      one-CTA cyclic Jacobi Hermitian eigensolver reading the lower
-//               triangle (as SelfAdjointEigenSolver does), ascending order.
+//  * BlockProducts: either of the two in this form or with the exact digits of
+//               k_tcgram_exact.cu, by size;
+//  * cholDrop:  Cholesky of a Gram matrix with the modified Gram-Schmidt
+//               column-drop rule (|v_j| after projection below 1e-12 -> column
+//               dropped, solver.cpp:404-407), in one CTA's shared memory up to
+//               80 columns and over the whole GPU above, returning the inverse
+//               factor (one warp per column from 48 on) so that Q = V R^{-1};
+//  * heig:      Hermitian eigensolver reading the lower triangle (as
+//               SelfAdjointEigenSolver does), ascending order: one-CTA cyclic
+//               Jacobi, or by size the methods of k_heig_refine.cu and
+//               k_heig_large.cu.
 #include "k_dense.cuh"
 #include "df64.cuh"
 
@@ -529,14 +534,15 @@ void gemmVC(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
 }
 
 // Measured per call (self-Gram / Y = V C, m = k columns, plain -> digits):
-// n = 36: m = 60 4250 -> 275 us / 3660 -> 454 us; m = 8 370 -> 181 / 81 ->
-// 122. n = 16: m = 24 132 -> 75 / 94 -> 81. The plain Gram never falls below
-// ~130 us (its chunk reduction is a serial chain), so the digits win on every
-// lattice a run uses; on smaller ones (N = 2 n^3 < 6000) both are launches
-// and latency, and the plain kernels keep the small-lattice fixed points on
-// the rounding path they are compared on. The plain V C is FP64-pipe bound
-// from a few million products on (13 us per million) and otherwise one short
-// launch against six.
+// n = 36: m = 60 4250 -> 231 us / 3660 -> 300 us (kernels). The plain Gram never falls
+// below ~130 us (its chunk reduction is a serial chain): n = 8, m = 16 146 ->
+// 81, n = 12 161 -> 82, n = 14 162 -> 83, m = 48 284 -> 97. So the digits are
+// faster from the smallest lattices on, and N = 6000 (n < 15) is not a line of
+// speed: lattices too small for a run in earnest keep the plain kernels and
+// with them their results to the bit, on which fixed points with a nearly free
+// centre of mass have been compared. The plain V C is FP64-pipe bound from a
+// few million products on (13 us per million) and otherwise one short launch
+// against six: n = 14, m = 16 60 -> 76, m = 48 (13 million) 197 -> 91.
 bool digitsPayGram(size_t N, int p, int q) {
   return N >= 6000 && p > 0 && q > 0;
 }
@@ -662,8 +668,9 @@ __device__ __forceinline__ void triangleAt(int e, int &a, int &b) {
 
 // The factorisations in shared memory leave T to cholInvKernel from this size
 // on: measured with T, FP64, m = 60: 427 us inside, 163 us with the second
-// launch. Below, T is small, and the serial order of its sums is the one that
-// the fixed points of the small lattices were compared in.
+// launch. It would pay below, too (a whole call of 12^3 with 8 or 16 states,
+// m = 24 or 48: 4601 -> 4554, 7363 -> 7139 us): there the serial order of the
+// sums stays, and with it the small lattices' results to the bit.
 constexpr int kInvOutside = 48;
 
 // Same factorisation in shared memory, right-looking: at step j the pivot is
@@ -851,9 +858,9 @@ __global__ void cholDropSmemKernel(const double2 *G, int ldg, int m,
 // one launch per column: the rank-1 update of the trailing triangle over the
 // whole GPU, whose last block to finish takes the next pivot and scales its
 // row (m = 192: 5.1 us a column; a pivot launch of its own took 4.4 us beside
-// the update's 2.2 and a gap), then T = R^{-1} (cholInvKernel). G's diagonal (drop floor), the pivots
-// and the arrival counter are kept in T's first 2m + 1 entries until T is
-// computed.
+// the update's 2.2 and a gap), then T = R^{-1} (cholInvKernel). G's diagonal
+// (drop floor), the pivots and the arrival counter are kept in T's first 2m + 1
+// entries until T is computed.
 __global__ void cholCopyKernel(const double2 *G, int ldg, int m, double2 *R,
                                double2 *T) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1045,10 +1052,12 @@ void heig(const double2 *A, int lda, int m, double2 *work, double2 *V,
         heigLarge(A, lda, m, V, w, perm, status, scr, s);
       }))
     return;
-  // The refined double-float method in FP64: m = 60 5100 -> 1250 us, m = 48
-  // 6050 -> 1060 us with the copies of a whole call. Below 48 the Jacobi stays:
-  // it is cheaper there (860 us for m = 8 and 24 together), and the fixed
-  // points of the small lattices were compared in its roundings.
+  // The refined double-float method in FP64, per call (Jacobi -> refined,
+  // twofold levels): m = 8 217 -> 406 us, 16 634 -> 493, 24 1662 -> 587, 32
+  // 2756 -> 698, 40 4585 -> 826, 47 6408 -> 928, 60 5100 -> 1151, residuals
+  // 1e-15 .. 3e-15 -> 2e-16 .. 4e-16. So speed would put the line at 16; from
+  // there to 47 the Jacobi stays for its roundings, in which the fixed points
+  // of small runs have been compared.
   const bool refined =
       !heigFp64Only() && heigRefinedTakes(m) &&
       withScratch(heigRefinedScratchBytes(m), [&](void *scr) {

@@ -7,8 +7,8 @@
 // is also tridiagonalisation based):
 //  1. Householder tridiagonalisation of the full Hermitian matrix, one step
 //     per column: the reflector (one block), the matrix-vector product
-//     p = tau A22 v with a warp per row, w = p - tau/2 (p^H v) v, and the rank-2 update A22 -= v w^H + w v^H over the whole
-//     grid. Reflectors H = I - tau v v^H with real beta (the LAPACK
+//     p = tau A22 v with a warp per row, w = p - tau/2 (p^H v) v, and the
+//     rank-2 update A22 -= v w^H + w v^H over the whole grid. Reflectors H = I - tau v v^H with real beta (the LAPACK
 //     convention), so the tridiagonal matrix is real.
 //  2. Eigenvalues of the real tridiagonal by multisection on Sturm counts,
 //     one warp per eigenvalue.

@@ -596,8 +596,8 @@ __global__ void pcgPKernel(typename C2<T>::type *P,
 
 // Inverse Jacobi diagonal, tabulated once per solve: an FP64 division costs
 // about ten operations of a pipe that retires two a clock per SM, and the step
-// kernels are bound by it (pcgUpdateKernel, 30^3 x 8 columns: 20.8 -> 16.2 us). coef: the species' table, whose first entry of a
-// point is c0.
+// kernels are bound by it (pcgUpdateKernel, 30^3 x 8 columns: 20.8 -> 16.2 us).
+// coef: the species' table, whose first entry of a point is c0.
 __global__ void invDiagKernel(const double *coef, double shift, size_t ns,
                               double *inv, float *inv32) {
   const size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -665,10 +665,10 @@ void pcgRun(const PcgPlan<T> &pl, cudaStream_t s) {
   pcgInitFinish<<<pl.ncols, 32, 0, s>>>(pl.st, pl.partials, nblk, pl.tol,
                                         pl.ndone);
   // Early exit: after the init (a one-thread kernel) and in the last kernel
-  // of every step a thread writes the count of finished columns into the next slot of mapped
-  // pinned host memory (slot 0 after the init, it + 1 after step it); the
-  // host marks a slot unwritten (-1) before it launches the step that
-  // writes it. Before step `it` the host reads the slot of step it - kLag
+  // of every step a thread writes the count of finished columns into the next
+  // slot of mapped pinned host memory (slot 0 after the init, it + 1 after
+  // step it); the host marks a slot unwritten (-1) before it launches the step
+  // that writes it. Before step `it` the host reads the slot of step it - kLag
   // (so the device queue never drains) and stops issuing steps once every
   // column has finished. Later steps would only launch no-op kernels.
   ExitPoll *poll = pl.ndone ? exitPollTake() : nullptr;
