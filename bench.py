@@ -370,9 +370,9 @@ FP64_FLOPS_PER_POINT_COL = 185
 
 
 def _fp64_roofline(lib, ms64):
-    """The FP64 product against its algorithmic bytes: the integer-limb kernel
-    (k_stencil64.cu) is bound by integer issue and takes next to nothing of the
-    FP64 pipe. fp64_pipe_equivalent: the FP64 instructions of the same product
+    """The FP64 product against its algorithmic bytes. What limits the kernel
+    (k_stencil64.cu, integer arithmetic) is instruction issue; it takes next to
+    nothing of the FP64 pipe. fp64_pipe_equivalent: the FP64 instructions of the same product
     in FP64 arithmetic per second over the pipe's measured rate
     (ncgm_measure_fp64_gflops / 2); above 1 no FP64 kernel could follow."""
     import ctypes
@@ -383,7 +383,8 @@ def _fp64_roofline(lib, ms64):
     out = {"ms_per_hx": round(ms64, 4), "gbs": round(gbs, 2),
            "gflops": round(pts * FP64_FLOPS_PER_POINT_COL / (ms64 * 1e-3) /
                            1e9, 1),
-           "roofline": {"bound": "integer issue", "achieved": round(gbs, 1),
+           "limiter": "integer issue",
+           "roofline": {"bound": "hbm", "achieved": round(gbs, 1),
                         "peak": peak, "unit": "GB/s",
                         "frac": round(gbs / peak, 4),
                         "peak_source": peak_kind}}
@@ -581,7 +582,7 @@ def main():
     ap.add_argument("--no-cpu", action="store_true",
                     help="skip the CPU-baseline sample on our arm")
     ap.add_argument("--curve", action="store_true",
-                    help="also time the 16-point 24Mg curve (about 8 minutes)")
+                    help="also time the 16-point 24Mg curve (about 3 minutes)")
     ap.add_argument("--sn120", action="store_true",
                     help="also time the 120Sn HFB run to 1 keV (minutes)")
     ap.add_argument("--no-hf", action="store_true",

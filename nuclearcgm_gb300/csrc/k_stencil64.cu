@@ -6,8 +6,8 @@
 // column took 758 us for 36^3 x 60 columns and 1108 us for 40^3 x 64, where
 // the bytes take 30 us. Here the products run on the integer pipes, with more
 // bits than FP64 keeps, in 243 and 302 us, bound by instruction issue and
-// latency: 43 and 47 % of the slots with 13 and 15 % of the warps (128
-// registers, two blocks of 216 or 256 threads per SM). One scale per tile, 57
+// latency: 43 and 47 % of the slots with 13 and 15 warps per SM (128
+// registers, two blocks of 224 or 256 threads per SM). One scale per tile, 57
 // bits below its largest value, took 210 and 266 us, but an orbital falls by
 // more than the spare bits inside a tile.
 //  * A block owns a tile of lattice points and walks over columns. It copies
