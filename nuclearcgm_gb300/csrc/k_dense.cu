@@ -534,13 +534,13 @@ void gemmVC(const double2 *V, size_t ldv, int m, const double2 *Cm, int ldc,
 }
 
 // Measured per call (self-Gram / Y = V C, m = k columns, plain -> digits):
-// n = 36: m = 60 4250 -> 231 us / 3660 -> 300 us (kernels). The plain Gram never falls
-// below ~130 us (its chunk reduction is a serial chain): n = 8, m = 16 146 ->
-// 81, n = 12 161 -> 82, n = 14 162 -> 83, m = 48 284 -> 97. So the digits are
-// faster from the smallest lattices on, and N = 6000 (n < 15) is not a line of
-// speed: lattices too small for a run in earnest keep the plain kernels and
-// with them their results to the bit, on which fixed points with a nearly free
-// centre of mass have been compared. The plain V C is FP64-pipe bound from a
+// n = 36: m = 60 4250 -> 231 us / 3660 -> 300 us (kernels). The plain Gram never
+// falls below ~130 us (its chunk reduction is a serial chain): n = 8, m = 16
+// 146 -> 81, n = 12 161 -> 82, n = 14 162 -> 83, m = 48 284 -> 97. So the
+// digits are faster from the smallest lattices on, and N = 6000 (n < 15) is not
+// a line of speed: lattices too small for a run in earnest keep the plain
+// kernels and with them their results to the bit, on which fixed points with a
+// nearly free centre of mass have been compared. The plain V C is FP64-pipe bound from a
 // few million products on (13 us per million) and otherwise one short launch
 // against six: n = 14, m = 16 60 -> 76, m = 48 (13 million) 197 -> 91.
 bool digitsPayGram(size_t N, int p, int q) {

@@ -103,13 +103,14 @@ __device__ __forceinline__ double norm2(double2 a, double s) {
 // operations per clock per SM): 172 of its operations per point and column, 96
 // for the six spinor derivatives (differences first) and 76 for the densities,
 // which add one column's contribution at a time to the running sums: rounding
-// those once per column and not once per product halves the error (36^3 x 20
-// columns, tau: 5.3e-16 -> 1.6e-16, 12 operations and 12 % more time). Every point runs the
-// same instructions: rules of lower order next to the faces are zero weights,
-// their neighbours are not read. The form it replaces branched on the rule (a
-// warp spans all of them along x) and divided each derivative by its
-// denominator: 36^3 x 20 columns 1110 -> 339 us, 87 % of the pipe. 64 threads per block: 36^3
-// points are then 4.8 blocks per SM, so the last wave costs little.
+// those once per column and not once per product cuts the error (36^3 x 20
+// columns, tau: 5.3e-16 -> 1.6e-16, 12 operations and 12 % more time). Every
+// point runs the same instructions: rules of lower order next to the faces are
+// zero weights, their neighbours are not read. The form it replaces branched on
+// the rule (a warp spans all of them along x) and divided each derivative by
+// its denominator: 36^3 x 20 columns 1110 -> 339 us, 87 % of the pipe. 64
+// threads per block: 36^3 points are then 4.8 blocks per SM, so the last wave
+// costs little.
 __global__ void __launch_bounds__(64)
     densityKernel(const double2 *__restrict__ Phi, size_t ldphi, int M, int n,
                   DerivScale f, double *rho, double *tau, double *J9,
